@@ -1472,12 +1472,13 @@ cudaError_t fluid_coupled_step(FluidState& s, CoupledField const& f, double dt, 
     // the substeps: every guard accumulates on the device and is checked
     // once, after the step
     if ((e = reset_reductions(s, stream)) != cudaSuccess) return e;
-    if ((e = maxwell_advance_b(f.nr, f.nz, f.dr, f.dz, restagger, f.er, f.ez, f.bt, stream)) != cudaSuccess) return e;
     for (int k = 0; k < substeps; ++k) {
         launch_react(s, 0.5 * dts, false, stream);
         launch_transport(s, dts, f.er, f.amb_er, f.ez, f.amb_ez, f.jr_kin, f.jz_kin, false, stream);
-        if ((e = maxwell_advance_b(f.nr, f.nz, f.dr, f.dz, dts, f.er, f.ez, f.bt, stream)) != cudaSuccess) return e;
-        if ((e = maxwell_silver_mueller(f.nr, f.nz, f.er, f.ez, f.bt, stream)) != cudaSuccess) return e;
+        // the first substep's B carries the restagger (the carriers do not read B)
+        e = k == 0 ? maxwell_advance_b(f.nr, f.nz, f.dr, f.dz, restagger, dts, true, true, f.er, f.ez, f.bt, stream)
+                   : maxwell_advance_b(f.nr, f.nz, f.dr, f.dz, dts, 0.0, false, true, f.er, f.ez, f.bt, stream);
+        if (e != cudaSuccess) return e;
         if ((e = maxwell_advance_e(f.nr, f.nz, f.dr, f.dz, dts, f.bt, s.jr, s.jz, f.er, f.ez, stream)) != cudaSuccess) {
             return e;
         }
@@ -1487,8 +1488,8 @@ cudaError_t fluid_coupled_step(FluidState& s, CoupledField const& f, double dt, 
         if (tables) launch_closure(s, f.cell_er, f.cell_ez, stream);
         launch_react(s, 0.5 * dts, false, stream);
     }
-    if ((e = maxwell_advance_b(f.nr, f.nz, f.dr, f.dz, -restagger, f.er, f.ez, f.bt, stream)) != cudaSuccess) return e;
-    if ((e = maxwell_silver_mueller(f.nr, f.nz, f.er, f.ez, f.bt, stream)) != cudaSuccess) return e;
+    e = maxwell_advance_b(f.nr, f.nz, f.dr, f.dz, -restagger, 0.0, false, true, f.er, f.ez, f.bt, stream);
+    if (e != cudaSuccess) return e;
     launch_conductivity(s, stream);
     if ((e = cudaMemsetAsync(s.se, 0, sizeof(double) * 3 * static_cast<size_t>(s.n), stream)) != cudaSuccess) return e;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -16,25 +16,30 @@
 
 namespace rrea_dev {
 
-__global__ void field_prep_kernel(int nr, int nz, const double* __restrict__ er, const double* __restrict__ ez,
-                                  const double* __restrict__ amb_er, const double* __restrict__ amb_ez,
-                                  double* __restrict__ cell_er, double* __restrict__ cell_ez)
+// A thread owns one column over `rows` rows, so the axial face between two
+// rows is read and summed once.
+__global__ void __launch_bounds__(256) field_prep_kernel(int nr, int nz, int rows, const double* __restrict__ er,
+                                                         const double* __restrict__ ez,
+                                                         const double* __restrict__ amb_er,
+                                                         const double* __restrict__ amb_ez,
+                                                         double* __restrict__ cell_er, double* __restrict__ cell_ez)
 {
-    int64_t const total = static_cast<int64_t>(nr) * nz;
-    for (int64_t c = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; c < total;
-         c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        int const i = static_cast<int>(c % nr);
-        int const j = static_cast<int>(c / nr);
+    int const i = blockIdx.x * 32 + threadIdx.x;
+    int const j0 = (blockIdx.y * 8 + threadIdx.y) * rows;
+    int const j1 = min(j0 + rows, nz);
+    if (i >= nr || j0 >= j1) return;
+    size_t const z0 = static_cast<size_t>(i) + static_cast<size_t>(nr) * j0;
+    double zl = ez[z0] + amb_ez[z0];
+    for (int j = j0; j < j1; ++j) {
         // S/RreaAmrexAdvance.cpp:556-565: 0.5*((m+a)_lo + (m+a)_hi)
+        size_t const c = static_cast<size_t>(i) + static_cast<size_t>(nr) * j;
         size_t const rlo = static_cast<size_t>(i) + static_cast<size_t>(nr + 1) * j;
         double const elo = er[rlo] + amb_er[rlo];
         double const ehi = er[rlo + 1] + amb_er[rlo + 1];
         cell_er[c] = 0.5 * (elo + ehi);
-        size_t const zlo = static_cast<size_t>(i) + static_cast<size_t>(nr) * j;
-        size_t const zhi = static_cast<size_t>(i) + static_cast<size_t>(nr) * (j + 1);
-        double const zl = ez[zlo] + amb_ez[zlo];
-        double const zh = ez[zhi] + amb_ez[zhi];
+        double const zh = ez[c + nr] + amb_ez[c + nr];
         cell_ez[c] = 0.5 * (zl + zh);
+        zl = zh;
     }
 }
 
@@ -159,12 +164,13 @@ cudaError_t set_step_constants(rrea_dev::StepConstants const& c, cudaStream_t st
 cudaError_t field_prep(int nr, int nz, const double* er, const double* ez, const double* amb_er, const double* amb_ez,
                        double* cell_er, double* cell_ez, cudaStream_t stream)
 {
-    int64_t const total = static_cast<int64_t>(nr) * nz;
-    int const threads = 256;
-    int const blocks = static_cast<int>((total + threads - 1) / threads);
+    // up to four rows per thread while every SM keeps its resident threads
+    int64_t const fit = static_cast<int64_t>(nr) * nz / (152 * 1024);
+    int const rows = static_cast<int>(fit < 1 ? 1 : (fit > 4 ? 4 : fit));
+    dim3 const grid(static_cast<unsigned>((nr + 31) / 32), static_cast<unsigned>((nz + 8 * rows - 1) / (8 * rows)));
     note_launch();
-    rrea_dev::field_prep_kernel<<<blocks > 0 ? blocks : 1, threads, 0, stream>>>(nr, nz, er, ez, amb_er, amb_ez,
-                                                                                  cell_er, cell_ez);
+    rrea_dev::field_prep_kernel<<<grid, dim3(32, 8), 0, stream>>>(nr, nz, rows, er, ez, amb_er, amb_ez, cell_er,
+                                                                  cell_ez);
     return cudaGetLastError();
 }
 

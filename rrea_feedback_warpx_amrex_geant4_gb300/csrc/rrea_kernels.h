@@ -190,10 +190,11 @@ cudaError_t population_thin_instances(PopulationInput const& in, PopulationWork*
 cudaError_t population_split(rrea_dev::TileColumns const& t, int64_t n, double min_w, PopulationWork*& work,
                              int64_t first_id, int64_t room, int64_t* added, cudaStream_t stream);
 
-// Maxwell leapfrog pieces (I/RreaMaxwellTMRZ.H:143-214) for the coupled step.
-cudaError_t maxwell_advance_b(int nr, int nz, double dr, double dz, double dt, const double* er, const double* ez,
-                              double* bt, cudaStream_t stream);
-cudaError_t maxwell_silver_mueller(int nr, int nz, const double* er, const double* ez, double* bt, cudaStream_t stream);
+// Maxwell leapfrog pieces (I/RreaMaxwellTMRZ.H:143-214) for the coupled step:
+// B over dt_a (and, when twice, over dt_b after it), with the Silver-Mueller
+// faces when asked, and E.
+cudaError_t maxwell_advance_b(int nr, int nz, double dr, double dz, double dt_a, double dt_b, bool twice,
+                              bool open_faces, const double* er, const double* ez, double* bt, cudaStream_t stream);
 cudaError_t maxwell_advance_e(int nr, int nz, double dr, double dz, double dt, const double* bt, const double* jr,
                               const double* jz, double* er, double* ez, cudaStream_t stream);
 
