@@ -30,15 +30,21 @@ struct Geom {
     bool periodic;
 };
 
+// The wrap into [zlo, zhi) of a periodic domain.  Out of line: the
+// remainder's code would otherwise sit at every point of the transport loop,
+// which no absorbing domain ever reaches.
+static __device__ __noinline__ double periodic_wrap(double z, double zlo, double zhi)
+{
+    double const len = zhi - zlo;
+    if (!(gt0(len))) return z;
+    double w = fmod(z - zlo, len);
+    if (lt0(w)) w += len;
+    return zlo + w;
+}
 // S/RreaTransportPath.cpp:13-27
 __device__ __forceinline__ double wrap_z(Geom const& g, double z)
 {
-    if (!g.periodic) return z;
-    double const len = g.zhi - g.zlo;
-    if (!(gt0(len))) return z;
-    double w = fmod(z - g.zlo, len);
-    if (lt0(w)) w += len;
-    return g.zlo + w;
+    return g.periodic ? periodic_wrap(z, g.zlo, g.zhi) : z;
 }
 // S/RreaTransportPath.cpp:42-52
 template <int NP>
@@ -729,12 +735,17 @@ struct Selection {
     int channel;
     double sampled, total;
 };
+// `draw_u2` gives the channel draw, taken only for an event.  Most hazards
+// end without one, and -log(1 - u) >= u: a draw above the total depth (by
+// more than every rounding: its high word above the total's, and above
+// 2^-30) settles that on the integer pipe, without the logarithm.
+template <class Draw>
 __device__ __forceinline__ Selection select_hazard(const double* __restrict__ arena, double t0, double t1, double t2,
-                                                  int count, double u1, double u2)
+                                                  int count, double u1, Draw&& draw_u2)
 {
     Selection r{false, false, -1, 0.0, 0.0};
     double const taus[3] = {t0, t1, t2};
-    if (count < 1 || count > 3 || !finite_bits(u1) || !finite_bits(u2)) return r;
+    if (count < 1 || count > 3 || !finite_bits(u1)) return r;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         if (i >= count) break;
@@ -743,11 +754,16 @@ __device__ __forceinline__ Selection select_hazard(const double* __restrict__ ar
     }
     r.valid = finite_bits(r.total);
     if (!r.valid) return r;
+    if (__double2hiint(u1) > max(__double2hiint(r.total) + 1, 0x3e100000)) return r;
     u1 = max0(fmin(1.0, u1));
     r.sampled = -flog(arena, fmax(1.0e-30, 1.0 - u1));
     if (!(r.sampled < r.total)) return r;
-    r.event = true;
-    u2 = max0(fmin(1.0, u2));
+    double const u2 = max0(fmin(1.0, draw_u2()));
+    r.event = finite_bits(u2);
+    if (!r.event) {
+        r.valid = false;
+        return r;
+    }
     double const target = u2 * r.total;
     double cum = 0.0;
     int last_open = -1;

@@ -12,6 +12,7 @@
 //   * tallies      -> not kept (diagnostic ledger only).
 #pragma once
 
+#include "rrea_rate_rows.cuh"
 #include "rrea_sinks.cuh"
 
 namespace rrea_dev {
@@ -22,20 +23,19 @@ static __constant__ StepConstants c_step;
 
 
 
-// The electron coefficient tables (collision, soft radiative, hard-Moller
-// and tracked-brems rates) share one bit-identical 2856-row energy grid in
-// the schema-6 bundle (the loader refuses to run the device path otherwise).
-// One bracket per distinct query energy therefore serves every table, and
-// each table value is interpolated on first use only.  The hazard refreeze
-// and the drag segment that follows it query the same frozen energy, so the
-// drag reuses the refreeze's bracket instead of searching again.
-// The positron tables likewise share one grid among themselves; the cache is
-// used with the base table RREA_T_E_COLLISION or RREA_T_P_COLLISION.
+// The coefficient tables of a species (collision, soft radiative, hard
+// Moller or Bhabha, tracked brems, annihilation) share one bit-identical
+// energy grid in the schema-6 bundle (the loader refuses to run the device
+// path otherwise); their values, the inverse elastic mean free path and the
+// angle tables' energy fraction come from one row of interval polynomials
+// (rrea_rate_rows.cuh).  The cache holds the row of the last query energy:
+// the hazard refreeze and the drag segment that follows it query the same
+// frozen energy.  `base` is RREA_T_E_COLLISION or RREA_T_P_COLLISION.
+// Measured, one resident phase of 2^21 scale-up electrons: 34.1 ms with a
+// search, a log and an exp per value, 28.8 ms with rows.
 struct RateCache {
     long long key = -1;  // bit pattern of the bracketed energy; -1 = none
-    Bracket b;
-    double v[6];
-    unsigned have = 0;  // bit i: v[i] valid (0 collision, 1 soft, 2 hard, 3 brems, 5 annihilation)
+    RowHit hit;
 };
 
 __device__ __forceinline__ bool rate_bracket(StepConstants const& C, const double* __restrict__ arena, RateCache& rc,
@@ -44,34 +44,50 @@ __device__ __forceinline__ bool rate_bracket(StepConstants const& C, const doubl
     long long const key = __double_as_longlong(e);
     if (rc.key == key) return true;
     rc.key = -1;
-    rc.have = 0;
-    if (!bracket_hot(arena, C.tix.hot[base], e, rc.b, err)) return false;
+    if (!find_row(arena, C.tix.rate_rows[base == RREA_T_E_COLLISION ? 0 : 1], e, rc.hit)) {
+        err.set(RREA_GPU_ERR_RANGE);
+        return false;
+    }
     rc.key = key;
     return true;
 }
 
+// A value of a flagged row (two nodes within 1e-9 of one another), by the
+// reference's interpolation; NaN where that fails.
+static __device__ __noinline__ double rate_fallback(const double* __restrict__ arena, int table, double e)
+{
+    Err err;
+    double const v = interpolate(arena, c_step.tix.hot[table], e, err);
+    return err.code ? __longlong_as_double(0x7ff8000000000000LL) : v;
+}
+
+// Column `which` (RreaRateColumn, up to annihilation) at energy e.
 __device__ __forceinline__ double rate_value(StepConstants const& C, const double* __restrict__ arena, RateCache& rc,
                                              double e, int which, Err& err, int base = RREA_T_E_COLLISION)
 {
     if (!rate_bracket(C, arena, rc, e, err, base)) return 0.0;
-    unsigned const bit = 1u << which;
-    if (!(rc.have & bit)) {
-        rc.v[which] = eval_hot(arena, C.tix.hot[base + which], rc.b, err);
-        rc.have |= bit;
+    // a linear piece that starts at a zero node may round below it
+    double v = max0(row_value(rc.hit, which));
+    if (row_flags(rc.hit) >> which & 1u) {
+        v = rate_fallback(arena, which == RREA_RATE_ANNIHILATION ? RREA_T_P_ANNIHILATION : base + which, e);
+        if (nan_bits(v)) {
+            err.set(RREA_GPU_ERR_INVALID_STATE);
+            return 0.0;
+        }
     }
-    return rc.v[which];
+    return v;
 }
 
 __device__ __forceinline__ bool rate_positive(StepConstants const& C, const double* __restrict__ arena, RateCache& rc,
                                               double e, int which, Err& err, int base = RREA_T_E_COLLISION)
 {
-    if (!rate_bracket(C, arena, rc, e, err, base)) return false;
-    unsigned const bit = 1u << which;
-    if (rc.have & bit) return gt0(rc.v[which]);
-    return positive_hot(arena, C.tix.hot[base + which], rc.b, err);
+    return gt0(rate_value(C, arena, rc, e, which, err, base));
 }
 
-enum { kRateCollision = 0, kRateSoft = 1, kRateMoller = 2, kRateBhabha = 2, kRateBrems = 3, kRateAnnihilation = 5 };
+enum {
+    kRateCollision = RREA_RATE_COLLISION, kRateSoft = RREA_RATE_SOFT, kRateMoller = RREA_RATE_HARD,
+    kRateBhabha = RREA_RATE_HARD, kRateBrems = RREA_RATE_BREMS, kRateAnnihilation = RREA_RATE_ANNIHILATION
+};
 
 // Competing STP rates, O/RreaChargedFinalStates.H:107-152 with the accessors
 // ElectronHardMollerMeanFreePath / ElectronBremsstrahlungMeanFreePath
@@ -225,19 +241,90 @@ __device__ __noinline__ int plane_crossings(StepConstants const& C, ElectronArgs
     return 0;
 }
 
+// S/RreaInteractionTables.cpp:2477-2493, interpolated
+static __device__ __noinline__ double elastic_inverse_fallback(const double* __restrict__ arena, double e, int species)
+{
+    Err err;
+    RreaElasticIndex const& el = c_step.tix.elastic[species];
+    double const mfp = semilogx(arena + el.x, arena + el.lx, arena + el.ilx, arena + el.mfp, el.n, e, err);
+    return err.code ? __longlong_as_double(0x7ff8000000000000LL) : gt0(mfp) ? 1.0 / mfp : 0.0;
+}
+
 // S/RreaInteractionTables.cpp:2477-2493
 __device__ __forceinline__ double elastic_inverse_stp(StepConstants const& C, const double* __restrict__ arena,
-                                                      double e, Err& err,
-                                                      double le = __builtin_nan(""), int species = 0)
+                                                      RateCache& rc, double e, Err& err, int species = 0)
 {
-    RreaElasticIndex const& el = C.tix.elastic[species];
-    double const mfp = semilogx(arena + el.x, arena + el.lx, arena + el.ilx, arena + el.mfp, el.n, e, err, le) / 1.0;
-    return frozen_rate(gt0(mfp) ? 1.0 / mfp : 0.0, err);
+    if (!rate_bracket(C, arena, rc, e, err, species ? RREA_T_P_COLLISION : RREA_T_E_COLLISION)) return 0.0;
+    double v = row_value(rc.hit, RREA_RATE_ELASTIC);
+    if (row_flags(rc.hit) >> RREA_RATE_ELASTIC & 1u) v = elastic_inverse_fallback(arena, e, species);
+    return frozen_rate(v, err);
+}
+
+// The angle where a row or a node pair is outside what the fast form below
+// covers: the reference's steps.  NaN where a query fails.
+static __device__ __noinline__ double gs_angle_fallback(const double* __restrict__ arena, int species, int wentzel,
+                                                        double e, double n, double u)
+{
+    Err err;
+    RreaAngleIndex const& a = wentzel ? c_step.tix.wentzel[species] : c_step.tix.gs[species];
+    double const c = sample_gs_angle(arena, a, e, n, u, err);
+    return err.code ? __longlong_as_double(0x7ff8000000000000LL) : c;
+}
+
+// S/RreaInteractionTables.cpp:831-891: the bilinear log interpolation of
+// 1 - cos at the two CDF nodes around u and the log-log interpolation
+// between them.  The energy, path and CDF fractions come from rows.  The
+// node values are rounded as the reference rounds them (1 - (1 - x) on the
+// grid of 2^-53: cos near 1 keeps that rounding), and the logarithm of their
+// ratio is the difference of the interpolated logs plus the relative
+// roundings e - e^2/2 + e^3/3, e = (rounded - x) / x; e times the node is at
+// most 2^-53, so FP32 carries it.
+__device__ __forceinline__ double sample_gs_angle_rows(StepConstants const& C, const double* __restrict__ arena,
+                                                       RateCache& rc, RreaAngleIndex const& a, int species, int wentzel,
+                                                       double e, double n, double u, Err& err)
+{
+    RowHit hp, hu;
+    bool ok = rate_bracket(C, arena, rc, e, err, species ? RREA_T_P_COLLISION : RREA_T_E_COLLISION);
+    ok = ok && !(row_flags(rc.hit) >> RREA_RATE_ANGLE_ENERGY & 1u);
+    ok = ok && find_row(arena, a.p_rows, n, hp) && !row_flags(hp);
+    ok = ok && find_row(arena, a.u_rows, u, hu) && !row_flags(hu);
+    if (ok) {
+        int const ie = row_index(rc.hit), ip = row_index(hp), iu = row_index(hu) + 1;
+        double const te = row_value(rc.hit, RREA_RATE_ANGLE_ENERGY);
+        double const tn = row_value(hp, 0);
+        const double* l = arena + a.lomc + (static_cast<size_t>(ie) * a.np + ip) * a.nu + iu;
+        size_t const de = static_cast<size_t>(a.np) * a.nu, dp = a.nu;
+        auto at = [&](int k) {
+            double const p0 = __ldg(l + k), p1 = __ldg(l + dp + k);
+            double const lo = p0 + te * (__ldg(l + de + k) - p0);
+            double const hi = p1 + te * (__ldg(l + de + dp + k) - p1);
+            return lo + tn * (hi - lo);
+        };
+        double const l0 = at(0), l1 = at(1);
+        double const x0 = fexp(arena, l0), x1 = fexp(arena, l1);
+        double const d0 = 1.0 - (1.0 - x0), d1 = 1.0 - (1.0 - x1);
+        float const e0 = __fdividef(narrow_f32(d0 - x0), narrow_f32(x0));
+        float const e1 = __fdividef(narrow_f32(d1 - x1), narrow_f32(x1));
+        if (fabsf(e0) < 0.015625f && fabsf(e1) < 0.015625f) {
+            float const corr = (e1 - e0) - 0.5f * (e1 * e1 - e0 * e0) + (1.0f / 3.0f) * (e1 * e1 * e1 - e0 * e0 * e0);
+            double const fu = row_value(hu, 0);
+            double const omc = d0 * fexp(arena, fu * ((l1 - l0) + widen_f32(corr)));
+            double const c = 1.0 - fmin(2.0, omc);
+            return fmin(1.0, fmax(-1.0, c));
+        }
+    }
+    if (err.code) return 1.0;
+    double const c = gs_angle_fallback(arena, species, wentzel, e, n, u);
+    if (nan_bits(c)) {
+        err.set(RREA_GPU_ERR_RANGE);
+        return 1.0;
+    }
+    return c;
 }
 
 // S/RreaInteractionTables.cpp:2504-2560
-__device__ __forceinline__ double sample_gs_cos(StepConstants const& C, const double* __restrict__ arena, double e,
-                                                double n, double u, Err& err, double le, int species = 0)
+__device__ __forceinline__ double sample_gs_cos(StepConstants const& C, const double* __restrict__ arena, RateCache& rc,
+                                                double e, double n, double u, Err& err, int species = 0)
 {
     RreaArenaIndex const& ix = C.tix;
     if (!charged_in_range(ix, e)) {
@@ -259,7 +346,7 @@ __device__ __forceinline__ double sample_gs_cos(StepConstants const& C, const do
         return 1.0;
     }
     if (n >= ix.gs_isotropic_above_n) return 2.0 * u - 1.0;
-    return sample_gs_angle(arena, a, e, n, u, err, le);
+    return sample_gs_angle_rows(C, arena, rc, a, species, use_gs ? 0 : 1, e, n, u, err);
 }
 __device__ __forceinline__ double sample_single_elastic_cos(StepConstants const& C, const double* __restrict__ arena,
                                                             double e, double cdf_u, Err& err, double le,
@@ -295,6 +382,7 @@ __device__ __forceinline__ double sample_brems_cos(StepConstants const& C, doubl
     double const umax = 2.0 * (1.0 + e / kMeC2);
     double const target = cdf_u * (0.25 * tsai_g2(a * umax) + 0.75 * tsai_g2(3.0 * a * umax));
     double lo = 0.0, hi = umax;
+#pragma unroll 1
     for (int it = 0; it < 60; ++it) {
         double const mid = 0.5 * (lo + hi);
         double const m = 0.25 * tsai_g2(a * mid) + 0.75 * tsai_g2(3.0 * a * mid);
@@ -442,6 +530,7 @@ __device__ __forceinline__ double annihilation_fraction(double gamma, double dra
     if (!(gt0(span))) return 0.5;
     double const target = flo + u * span;
     double lo = emin, hi = emax;
+#pragma unroll 1
     for (int it = 0; it < 64; ++it) {
         double const mid = 0.5 * (lo + hi);
         if (a * log(mid) - mid + 1.0 / (c * mid) < target) lo = mid; else hi = mid;
@@ -543,9 +632,9 @@ static __device__ __noinline__ uint32_t spawn_annihilation(ElectronArgs A, RngSt
 // tracked electrons (n >= 10 elastic collisions per substep at MeV energies),
 // so it is kept out of line.
 static __device__ __noinline__ Dir3 gs_few_collisions(const double* __restrict__ arena, RngStream rng, uint64_t sub,
-                                               double gs_n, double k, double lk, double dx, double dy, double dz,
-                                               int species)
+                                               double gs_n, double k, double dx, double dy, double dz, int species)
 {
+    double const lk = flog(arena, k);
     uint64_t const ch_count = species ? kChPositronGsFewCount : kChElectronGsFewCount;
     uint64_t const ch_scatter = species ? kChPositronGsFewScatter : kChElectronGsFewScatter;
     uint64_t const ch_azimuth = species ? kChPositronGsFewAzimuth : kChElectronGsFewAzimuth;
@@ -574,6 +663,7 @@ __device__ __noinline__ double cutoff_bisection(Intervals<NP> iv, Path<NP> path,
                                                 double to_cut)
 {
     double lo = b, hi = e;
+#pragma unroll 1
     for (int it = 0; it < 56; ++it) {
         double const mid = 0.5 * (lo + hi);
         double const l = total * density_path(iv, path, b, mid);
@@ -769,6 +859,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
         bool viol = req > cap;
         uint64_t sub = req < cap ? req : cap;
         // selected_material_subcycles, O/RreaTransportStep.H:148-184
+#pragma unroll 1
         for (int guard = 0; guard < 64; ++guard) {
             double const maximum = total_stp * max_uniform_slice(iv, path, sub);
             double const tol = 64.0 * kEps * fmax(1.0, target);
@@ -783,7 +874,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
             else if (est > static_cast<double>(next)) next = static_cast<uint64_t>(est);
             sub = next < cap ? next : cap;
         }
-        double const gs_n = elastic_inverse_stp(C, arena, k, err, __builtin_nan(""), species) * driver_dpath;
+        double const gs_n = elastic_inverse_stp(C, arena, rc, k, err, species) * driver_dpath;
         double const ke = fmax(k, cutoff);
         double drag_est = 0.0;
         if constexpr (POS) {
@@ -1009,9 +1100,8 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
                                                                 : kChPositronContinuationChannel)
                                                 : (ordinal == 0 ? kChElectronCompetingChannel
                                                                 : kChElectronContinuationChannel);
-                double const u1 = rng.uniform(rng_index, ch_depth);
-                double const u2 = rng.uniform(rng_index, ch_channel);
-                Selection const selv = select_hazard(arena, t0, t1, t2, POS ? 3 : 2, u1, u2);
+                Selection const selv = select_hazard(arena, t0, t1, t2, POS ? 3 : 2, rng.uniform(rng_index, ch_depth),
+                                                     [&]() { return rng.uniform(rng_index, ch_channel); });
                 if (!selv.valid) {
                     err.set(RREA_GPU_ERR_INVALID_STATE);
                     break;
@@ -1086,20 +1176,18 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
         // ---- finish_interleaved_substep, O/RreaElectronTransport.cpp:502-524
         if (k >= cutoff) {
             // apply_gs_elastic_scatter, O/RreaTransportStep.H:371-423
-            // log(k) is shared by the elastic-MFP and angle-table brackets.
-            double const lk = (gt0(k)) ? flog(arena, k) : __longlong_as_double(0x7ff8000000000000LL);
-            double const gs_n = elastic_inverse_stp(C, arena, k, err, lk, species) * density_path(iv, path, sb, se);
+            double const gs_n = elastic_inverse_stp(C, arena, rc, k, err, species) * density_path(iv, path, sb, se);
             if (gt0(gs_n)) {
                 double const few = C.tix.gs_few_collision_threshold;
                 if (gs_n < few) {
-                    Dir3 const d3 = gs_few_collisions(arena, rng, sub, gs_n, k, lk, dx, dy, dz, species);
+                    Dir3 const d3 = gs_few_collisions(arena, rng, sub, gs_n, k, dx, dy, dz, species);
                     dx = d3.x; dy = d3.y; dz = d3.z;
                     if (d3.err) err.set(d3.err);
                     if (err.code) break;
                 } else {
-                    double const ct = sample_gs_cos(C, arena, k, gs_n,
+                    double const ct = sample_gs_cos(C, arena, rc, k, gs_n,
                                                     rng.uniform(sub << 8, POS ? kChPositronGsAngle : kChElectronGsAngle),
-                                                    err, lk, species);
+                                                    err, species);
                     double nx, ny, nz;
                     cone_direction(dx, dy, dz, ct, rng.uniform(sub << 8, POS ? kChPositronGsAzimuth : kChElectronGsAzimuth),
                                    nx, ny, nz);

@@ -108,21 +108,26 @@ template <class F>
 __device__ __forceinline__ void for_each_particle(int64_t n, unsigned long long* work, F&& f,
                                                   const uint32_t* __restrict__ order = nullptr)
 {
-    if (work) {
-        int const lane = threadIdx.x & 31;
-        for (;;) {
+    // one call site: the body is the whole transport loop, and a second
+    // inlined copy would double the kernel's instruction footprint
+    int const lane = threadIdx.x & 31;
+    int64_t next = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    for (;;) {
+        int64_t ip;
+        if (work) {
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(work, 32ULL);
             base = __shfl_sync(0xffffffffu, base, 0);
             if (base >= static_cast<unsigned long long>(n)) break;
             int64_t const k = static_cast<int64_t>(base) + lane;
-            if (k < n) f(order ? static_cast<int64_t>(__ldg(order + k)) : n - 1 - k);
+            if (k >= n) continue;
+            ip = order ? static_cast<int64_t>(__ldg(order + k)) : n - 1 - k;
+        } else {
+            if (next >= n) break;
+            ip = next;
+            next += static_cast<int64_t>(gridDim.x) * blockDim.x;
         }
-    } else {
-        for (int64_t ip = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; ip < n;
-             ip += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-            f(ip);
-        }
+        f(ip);
     }
 }
 

@@ -201,7 +201,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
         return -1;
     }
     double const driver_dpath = density_path(iv, path, path.in_begin, path.in_end);
-    double const gs_total = elastic_inverse_stp(C, arena, k, err, __builtin_nan(""), species) * driver_dpath;
+    double const gs_total = elastic_inverse_stp(C, arena, rc, k, err, species) * driver_dpath;
     double drag_est;
     if constexpr (POS) {
         drag_est = rate_value(C, arena, rc, k, kRateCollision, err, rate_base) * 1.0 * driver_dpath;
@@ -388,9 +388,9 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
                 double const seg_dp = density_path(iv, path, rem, se);
                 uint64_t const idx = pack(sub, ordinal, 0);
                 if (err.code) break;
-                double const u1 = rng.uniform(idx, kChNewbornCompetingOpticalDepth);
-                double const u2 = rng.uniform(idx, kChNewbornCompetingChannel);
-                Selection const selv = select_hazard(arena, s0 * seg_dp, s1 * seg_dp, s2 * seg_dp, POS ? 3 : 2, u1, u2);
+                Selection const selv = select_hazard(arena, s0 * seg_dp, s1 * seg_dp, s2 * seg_dp, POS ? 3 : 2,
+                                                     rng.uniform(idx, kChNewbornCompetingOpticalDepth),
+                                                     [&]() { return rng.uniform(idx, kChNewbornCompetingChannel); });
                 if (!selv.valid) {
                     err.set(RREA_GPU_ERR_INVALID_STATE);
                     break;
@@ -463,8 +463,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
         }
         if (err.code || terminal_interaction || terminal_at_point) break;
         if (k >= cut) {
-            double const lk = (gt0(k)) ? flog(arena, k) : __longlong_as_double(0x7ff8000000000000LL);
-            double const gs_n = elastic_inverse_stp(C, arena, k, err, lk, species) * density_path(iv, path, sb, se);
+            double const gs_n = elastic_inverse_stp(C, arena, rc, k, err, species) * density_path(iv, path, sb, se);
             if (gt0(gs_n)) {
                 double const few = C.tix.gs_few_collision_threshold;
                 if (gs_n < few) {
@@ -474,6 +473,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
                         break;
                     }
                     uint64_t const i0 = pack(sub, 0, 0);
+                    double const lk = flog(arena, k);
                     int const cnt = poisson_capped(
                         gs_n, rng.uniform(i0, POS ? kChNewbornPositronGsFewCount : kChNewbornElectronGsFewCount), cap);
                     for (int qq = 0; qq < cnt; ++qq) {
@@ -492,8 +492,8 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
                 } else {
                     uint64_t const i0 = pack(sub, 0, 0);
                     double const ct = sample_gs_cos(
-                        C, arena, k, gs_n, rng.uniform(i0, POS ? kChNewbornPositronGsAngle : kChNewbornElectronGsAngle),
-                        err, lk, species);
+                        C, arena, rc, k, gs_n,
+                        rng.uniform(i0, POS ? kChNewbornPositronGsAngle : kChNewbornElectronGsAngle), err, species);
                     double nx, ny, nz;
                     cone_direction(dx, dy, dz, ct,
                                    rng.uniform(i0, POS ? kChNewbornPositronGsAzimuth : kChNewbornElectronGsAzimuth), nx,
@@ -624,7 +624,8 @@ __device__ int advance_photon_newborn(StepConstants const& C, ElectronArgs const
         double const mfp = mfp_from_inverse(rates.total(), err);
         double const tau = density_path(iv, path, path.in_begin, path.in_end) / mfp;
         Selection const sel =
-            select_hazard(arena, tau, 0.0, 0.0, 1, rng.uniform(idx, kChNewbornCompetingOpticalDepth), 0.0);
+            select_hazard(arena, tau, 0.0, 0.0, 1, rng.uniform(idx, kChNewbornCompetingOpticalDepth),
+                          []() { return 0.0; });
         if (!sel.valid) {
             err.set(RREA_GPU_ERR_INVALID_STATE);
             return -1;

@@ -220,6 +220,7 @@ static __device__ __noinline__ double sample_photoelectron_cos(double k, double 
     if (beta.hi < 1.0e-4) {
         // non-relativistic limit: CDF (2 + m(3 - m^2))/4 in m = cos(theta)
         double lo = -1.0, hi = 1.0;
+#pragma unroll 1
         for (int it = 0; it < 96; ++it) {
             double const mid = 0.5 * (lo + hi);
             if (mid == lo || mid == hi) break;
@@ -243,6 +244,7 @@ static __device__ __noinline__ double sample_photoelectron_cos(double k, double 
     dd const target = dd_add(dd_mul(two_sum(1.0, -u), f_hi), dd_mul_d(f_lo, u));
     double const bd = b.hi, cd = c.hi, pbd = twopbc.hi, bm1d = twobm1.hi, tgt = target.hi;
     double lo = t_lo.hi, hi = t_hi.hi;
+#pragma unroll 1
     for (int it = 0; it < 128; ++it) {
         double const mid = 0.5 * (lo + hi);
         if (mid == lo || mid == hi) break;
@@ -620,7 +622,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
         ++events_out;
         double const u_int =
             rng.uniform(idx, ordinal == 0 ? kChPhotonOpticalDepth : kChPhotonContinuationOpticalDepth);
-        Selection const sel = select_hazard(arena, tau, 0.0, 0.0, 1, u_int, 0.0);
+        Selection const sel = select_hazard(arena, tau, 0.0, 0.0, 1, u_int, []() { return 0.0; });
         if (!sel.valid) {
             err.set(RREA_GPU_ERR_INVALID_STATE);
             return -1;

@@ -52,12 +52,7 @@ __device__ __forceinline__ CellStencil make_stencil(StepConstants const& C, doub
     rrea_gpu_config const& cfg = C.cfg;
     int const nr = cfg.nr, nz = cfg.nz;
     double zz = z;
-    if (cfg.periodic_z) {
-        double const len = cfg.z_hi - cfg.z_lo;
-        double s = fmod(zz - cfg.z_lo, len);
-        if (lt0(s)) s += len;
-        zz = cfg.z_lo + s;
-    }
+    if (cfg.periodic_z) zz = periodic_wrap(zz, cfg.z_lo, cfg.z_hi);
     double const fr = quot(r - cfg.r_lo, C.div_dr);
     double const fz = quot(zz - cfg.z_lo, C.div_dz);
     int const ic = static_cast<int>(floor(fr));

@@ -91,6 +91,40 @@ typedef struct {
     int64_t lmean;     // ng logs of the group means (0 where the mean is not positive)
 } RreaCondCdfIndex;
 
+// Interval-polynomial rows over one axis (device/rrea_rate_rows.cuh): cells
+// of 1/256 octave, each with its first row; a row's upper bound; and its
+// record {xc, 1/xc, meta, 0} followed by RREA_ROW_COLUMN doubles per column
+// {c0, c1, c2, c3, (float c4, c5), (float c6, 0)}.  meta: bit c of the low
+// word flags column c (interpolate instead), the high word is the lower node
+// index of the axis' own grid where the rows carry one.
+#define RREA_ROW_CELL_SHIFT 44
+#define RREA_ROW_HEADER 4
+#define RREA_ROW_COLUMN 6
+typedef struct {
+    int32_t rows;
+    int32_t stride;      // doubles per record
+    int64_t first_cell;  // bits(lowest argument) >> RREA_ROW_CELL_SHIFT
+    int64_t lo_key;      // bits of the lowest argument
+    int64_t span_key;    // bits of the highest argument - lo_key; negative: no rows
+    int64_t start;       // int32 first row per cell
+    int64_t hi;          // upper bound per row
+    int64_t rec;         // records
+} RreaRowIndex;
+
+// Columns of a species' rate rows: its coefficient tables in the order of
+// the hot tables (the column of the transport inverse length unused), the
+// inverse elastic mean free path, and the angle tables' energy fraction.
+enum RreaRateColumn {
+    RREA_RATE_COLLISION = 0,
+    RREA_RATE_SOFT = 1,
+    RREA_RATE_HARD = 2,
+    RREA_RATE_BREMS = 3,
+    RREA_RATE_ANNIHILATION = 4,
+    RREA_RATE_ELASTIC = 5,
+    RREA_RATE_ANGLE_ENERGY = 6,
+    RREA_RATE_COLUMNS = 7,
+};
+
 typedef struct {
     int32_t n;
     int32_t pad;
@@ -112,6 +146,8 @@ typedef struct {
     int64_t ile, ilp;   // 1 / (le[i] - le[i-1]), 1 / (lp[i] - lp[i-1]) at i >= 1
     int64_t ilur;       // 1 / lur[i] (0 where lur[i] = 0)
     int64_t iu;         // 1 / u[i] (0 where u[i] = 0)
+    RreaRowIndex p_rows;  // path fraction and lower node
+    RreaRowIndex u_rows;  // CDF log fraction and lower node between u[1] and u[nu - 2]
 } RreaAngleIndex;
 
 // Photoelectric subshell CDF (S/RreaInteractionTables.cpp:893-987): groups
@@ -148,6 +184,7 @@ typedef struct {
     RreaAngleIndex gs[2];              // option4 GS, E <= transition
     RreaAngleIndex wentzel[2];         // WentzelVI, E > transition
     int64_t hard_moller_mean_secondary;  // on the hard-Moller rate grid
+    RreaRowIndex rate_rows[2];         // 0 electron, 1 positron
     RreaPhotoelectricIndex pe;
     RreaPairBankIndex pair[2];         // 0 nuclear, 1 triplet
     int64_t total_doubles;
