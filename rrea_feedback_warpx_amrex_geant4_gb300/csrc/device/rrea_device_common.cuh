@@ -11,6 +11,7 @@
 #include "../rrea_arena.h"
 #include "../../../include/rrea_gpu.h"
 #include "rrea_fastmath.cuh"
+#include "rrea_rate_rows.cuh"
 
 #include <stdint.h>
 
@@ -80,6 +81,8 @@ struct StepConstants {
     double hm_threshold_eV;
     double photon_cutoff_eV;
     double density_ratio;
+    // bounds a billionth of the domain inside its faces: squared radius and z
+    double r2_inner, z_inner_lo, z_inner_hi;
     uint64_t step_key;
     double dt_s;
     int32_t hm_enabled;
@@ -121,9 +124,12 @@ struct RngStream {
         s ^= splitmix64(ch + 0x94d049bb133111ebULL);
         return splitmix64(s);
     }
+    // (n + 1/2) 2^-52 of the counter's top 52 bits n: 1 + n 2^-52 by its bits,
+    // less 1 - 2^-53, which is exact
     __device__ __forceinline__ double uniform(uint64_t idx, uint64_t ch) const
     {
-        return (__ull2double_rn(counter(idx, ch) >> 12) + 0.5) * 0x1.0p-52;
+        uint64_t const one = 0x3ff0000000000000ULL | (counter(idx, ch) >> 12);
+        return __longlong_as_double(static_cast<long long>(one)) - 0x1.fffffffffffffp-1;
     }
 };
 

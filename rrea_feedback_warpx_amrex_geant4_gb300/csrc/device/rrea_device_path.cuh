@@ -19,7 +19,9 @@ struct Piece {
 template <int NP>
 struct Path {
     double sx, sy, sz, ex, ey, ez;
+    double dx, dy, dz;  // end - start
     double full, in_begin, in_end, in_length;
+    double inv_full;    // 1 / full
     bool exits;
     int npieces;
     Piece pieces[NP];
@@ -28,7 +30,13 @@ struct Path {
 struct Geom {
     double rlo, rhi, zlo, zhi;
     bool periodic;
+    double r2_in, z_in_lo, z_in_hi;  // a billionth of the domain inside its faces
 };
+__device__ __forceinline__ Geom make_geom(StepConstants const& C)
+{
+    rrea_gpu_config const& c = C.cfg;
+    return Geom{c.r_lo, c.r_hi, c.z_lo, c.z_hi, c.periodic_z != 0, C.r2_inner, C.z_inner_lo, C.z_inner_hi};
+}
 
 // The wrap into [zlo, zhi) of a periodic domain.  Out of line: the
 // remainder's code would otherwise sit at every point of the transport loop,
@@ -51,19 +59,27 @@ template <int NP>
 __device__ __forceinline__ void point_at_full(Path<NP> const& p, Geom const& g, double f, double& x, double& y, double& z)
 {
     f = max0(fmin(1.0, f));
-    x = p.sx + f * (p.ex - p.sx);
-    y = p.sy + f * (p.ey - p.sy);
-    z = wrap_z(g, p.sz + f * (p.ez - p.sz));
+    x = p.sx + f * p.dx;
+    y = p.sy + f * p.dy;
+    z = wrap_z(g, p.sz + f * p.dz);
 }
 // S/RreaTransportPath.cpp:54-71
 template <int NP>
 __device__ __forceinline__ void point_at_piece(Path<NP> const& p, Geom const& g, Piece const& pc, double f, double& x,
                                                double& y, double& z)
 {
+    if constexpr (NP == 1) {
+        // an absorbing domain's one piece: its callers pass fractions inside
+        // it, its shift is zero, and a z an ulp past a face reads the edge cell
+        x = p.sx + f * p.dx;
+        y = p.sy + f * p.dy;
+        z = p.sz + f * p.dz;
+        return;
+    }
     f = fmax(pc.begin, fmin(pc.end, f));
-    x = p.sx + f * (p.ex - p.sx);
-    y = p.sy + f * (p.ey - p.sy);
-    z = p.sz + f * (p.ez - p.sz) + pc.shift;
+    x = p.sx + f * p.dx;
+    y = p.sy + f * p.dy;
+    z = p.sz + f * p.dz + pc.shift;
     z = fmax(g.zlo, fmin(g.zhi, z));
 }
 // S/RreaTransportPath.cpp:29-40
@@ -74,17 +90,59 @@ __device__ __forceinline__ bool outside_certified(Geom const& g, double r, doubl
     return !g.periodic && (z < g.zlo || z >= g.zhi);
 }
 
+// A chord with both ends strictly inside an absorbing domain, a convex body:
+// nothing is clipped, its one piece is [0, 1].  Almost every microchord of
+// the transport loops is one, and skips two radii, three divisions and a
+// square root.  False (p unset) when an end is within a billionth of a face,
+// outside, or not finite: clip_chord decides those.
+__device__ __forceinline__ bool strictly_inside(Geom const& g, double r2, double z)
+{
+    // a NaN or negative-zero-free non-negative r2 orders as its bits
+    return dbits(r2) < dbits(g.r2_in) && z > g.z_in_lo && z < g.z_in_hi;
+}
+template <int NP>
+__device__ __forceinline__ bool clip_inside(double x0, double y0, double z0, double r02, double x1, double y1, double z1,
+                                            double r12, Geom const& g, Path<NP>& p)
+{
+    if constexpr (NP != 1) return false;
+    if (!strictly_inside(g, r02, z0) || !strictly_inside(g, r12, z1)) return false;
+    double const dx = x1 - x0, dy = y1 - y0, dz = z1 - z0;
+    double const n2 = dx * dx + dy * dy + dz * dz;
+    if (!gt0(n2)) return false;
+    double const inv = frsqrt(n2);
+    p.sx = x0;
+    p.sy = y0;
+    p.sz = z0;
+    p.ex = x1;
+    p.ey = y1;
+    p.ez = z1;
+    p.dx = dx;
+    p.dy = dy;
+    p.dz = dz;
+    p.full = n2 * inv;
+    p.inv_full = inv;
+    p.in_begin = 0.0;
+    p.in_end = 1.0;
+    p.in_length = p.full;
+    p.exits = false;
+    p.npieces = 1;
+    p.pieces[0] = Piece{0.0, 1.0, p.full, 0.0};
+    return true;
+}
+
 // S/RreaTransportPath.cpp:73-295 on Cartesian chord ends (x0, y0, z0) ->
 // (x1, y1, z1) with their radii r0, r1.  Periodic seams use double
 // arithmetic where the host reference uses long double.
+// Out of line: the chords that reach it are at a face (clip_inside).
 template <int NP>
-__device__ __forceinline__ void clip_chord(double x0, double y0, double z0, double r0, double x1, double y1, double z1,
+__device__ __noinline__ void clip_chord(double x0, double y0, double z0, double r0, double x1, double y1, double z1,
                                            double r1, bool ends_finite, Geom const& g, Path<NP>& p, Err& err)
 {
     if (!ends_finite || !finite_bits(r0) || !finite_bits(z0) || !finite_bits(r1) || !finite_bits(z1) || lt0(r0) || lt0(r1)) {
         err.set(RREA_GPU_ERR_GEOMETRY);
         p.npieces = 0;
         p.full = 0.0;
+        p.inv_full = 0.0;
         p.in_begin = p.in_end = p.in_length = 0.0;
         p.exits = false;
         return;
@@ -96,7 +154,11 @@ __device__ __forceinline__ void clip_chord(double x0, double y0, double z0, doub
     p.ey = y1;
     p.ez = z1;
     double const dx = p.ex - p.sx, dy = p.ey - p.sy, dz = p.ez - p.sz;
+    p.dx = dx;
+    p.dy = dy;
+    p.dz = dz;
     p.full = sqrt(dx * dx + dy * dy + dz * dz);
+    p.inv_full = 1.0 / p.full;
     p.in_begin = 0.0;
     double const scale = fmax(1.0, fmax(g.rhi, fmax(fabs(g.zlo), fabs(g.zhi))));
     double const tol = 64.0 * kEps * scale;
@@ -222,7 +284,13 @@ __device__ __forceinline__ void clip_rz(double r0, double th0, double z0, double
         sincos(th0, &s0, &c0);
         sincos(th1, &s1, &c1);
     }
-    clip_chord(r0 * c0, r0 * s0, z0, r0, r1 * c1, r1 * s1, z1, r1, finite, g, p, err);
+    double const x0 = r0 * c0, y0 = r0 * s0, x1 = r1 * c1, y1 = r1 * s1;
+    if (finite && !lt0(r0) && !lt0(r1) && clip_inside(x0, y0, z0, r0 * r0, x1, y1, z1, r1 * r1, g, p)) return;
+    Path<NP> out;   // the out-of-line call's, so that p stays in registers
+    Err e;
+    clip_chord(x0, y0, z0, r0, x1, y1, z1, r1, finite, g, out, e);
+    p = out;
+    if (e.code) err.set(e.code);
 }
 
 // The chords the transport loops build run between Cartesian points, which
@@ -234,8 +302,13 @@ template <int NP>
 __device__ __forceinline__ void clip_xyz(double x0, double y0, double z0, double x1, double y1, double z1, Geom const& g,
                                          Path<NP>& p, Err& err)
 {
+    if (clip_inside(x0, y0, z0, fma(x0, x0, y0 * y0), x1, y1, z1, fma(x1, x1, y1 * y1), g, p)) return;
     bool const finite = finite_bits(x0) && finite_bits(y0) && finite_bits(x1) && finite_bits(y1);
-    clip_chord(x0, y0, z0, rz_radius(x0, y0), x1, y1, z1, rz_radius(x1, y1), finite, g, p, err);
+    Path<NP> out;   // the out-of-line call's, so that p stays in registers
+    Err e;
+    clip_chord(x0, y0, z0, rz_radius(x0, y0), x1, y1, z1, rz_radius(x1, y1), finite, g, out, e);
+    p = out;
+    if (e.code) err.set(e.code);
 }
 
 // ------------------------------------------------------------ kinematics
@@ -253,13 +326,25 @@ __device__ __forceinline__ double kinetic_from_proper_velocity(double ux, double
     double const gm = sqrt(1.0 + u2 / (kC * kC));
     return u2 * kMeC2 / ((kC * kC) * (gm + 1.0));
 }
-// O/RreaParticleInteraction.H:92-105
-__device__ __forceinline__ double charged_speed(double k)
+// gamma beta = sqrt(gamma^2 - 1) of kinetic energy k, from gamma^2 - 1 =
+// (k/mc^2)(k/mc^2 + 2) (no cancellation); 0 for k <= 0.
+__device__ __forceinline__ double gamma_beta(double k)
 {
-    if (!finite_bits(k) || lt0(k)) return __longlong_as_double(0x7ff8000000000000LL);
-    double const gm = 1.0 + k * kInvMeC2;
-    double const b2 = max0(1.0 - 1.0 / (gm * gm));
-    return kC * sqrt(b2);
+    double const t = k * kInvMeC2;
+    return le0(k) ? 0.0 : fsqrt(t * (t + 2.0));
+}
+// Speed c beta (O/RreaParticleInteraction.H:92-105: c sqrt(1 - 1/gamma^2)) as
+// c (gamma beta) / gamma, with gamma beta handed on; NaN for k < 0 or not
+// finite, as there.
+__device__ __forceinline__ double charged_speed(double k, double& gb)
+{
+    if (!finite_bits(k) || lt0(k)) {
+        gb = 0.0;
+        return __longlong_as_double(0x7ff8000000000000LL);
+    }
+    gb = gamma_beta(k);
+    double const t = k * kInvMeC2;
+    return (kC * gb) * frsqrt(fma(t, t + 2.0, 1.0));
 }
 // O/RreaChargedInterleave.H:294-307.  The reference divides by sqrt(n2);
 // scaling by rsqrt(n2) (within an ulp of 1/sqrt(n2)) gives the same unit
@@ -272,38 +357,48 @@ __device__ __forceinline__ void normalize(double& x, double& y, double& z)
         x = 0.0; y = 0.0; z = 1.0;
         return;
     }
-    double const inv = rsqrt(n2);
+    double const inv = frsqrt(n2);
     x *= inv; y *= inv; z *= inv;
 }
-// O/RreaChargedInterleave.H:309-364.  The reference normalises five times:
-// the axis, a copy of it, the first and second basis vectors and the
-// result.  The copy of a unit axis, the cross product of two orthonormal
-// vectors and the rotated unit vector are already unit to within a few ulps,
-// so only the axis and the first basis vector are normalised here; the
-// direction differs from the reference's by ulps (and is renormalised by the
-// next half kick).
-__device__ __forceinline__ void cone_direction(double ax, double ay, double az, double cos_t, double u_phi,
-                                               double& ox, double& oy, double& oz)
+// O/RreaChargedInterleave.H:309-364 about a unit axis d, for cos_t in [-1, 1].
+// The reference normalises the axis, a copy of it, both basis vectors and
+// the result.  With b1 = e x d / rho (e the z axis, or x where |d_z| > 0.9;
+// rho = |e x d|) and b2 = d x b1 the rotated vector is, component by
+// component,
+//   along e:      d_e cos + B rho^2
+//   across, a, b: a (cos - B d_e) - A b,  b (cos - B d_e) + A a
+// with A, B = (sin / rho) (cos phi, sin phi) and sin / rho = sin^2 / sqrt(sin^2
+// rho^2), one inverse root; the direction differs from the reference's by
+// ulps (and is renormalised by the next half kick).
+__device__ __forceinline__ void cone_unit(const double* __restrict__ arena, double dx, double dy, double dz, double cos_t,
+                                          double u_phi, double& ox, double& oy, double& oz)
 {
-    normalize(ax, ay, az);
-    double const dx = ax, dy = ay, dz = az;
-    double rx = 0.0, ry = 0.0, rz = 1.0;
-    if (fabs(dz) > 0.9) { rx = 1.0; rz = 0.0; }
-    double b1x = ry * dz - rz * dy, b1y = rz * dx - rx * dz, b1z = rx * dy - ry * dx;
-    normalize(b1x, b1y, b1z);
-    double const b2x = dy * b1z - dz * b1y, b2y = dz * b1x - dx * b1z, b2z = dx * b1y - dy * b1x;
-    cos_t = fmin(1.0, fmax(-1.0, cos_t));
+    bool const about_x = (dbits(dz) & 0x7fffffffffffffffull) > 0x3feccccccccccccdull;  // |d_z| > 0.9
+    double const pole = about_x ? dx : dz, a = about_x ? dy : dx, b = about_x ? dz : dy;
     // cos^2 is rounded on its own before the subtraction, as the reference's
     // x86-64 build rounds it: a fused 1 - cos^2 differs by up to an ulp of 1,
     // which a small-angle deflection (cos near 1, the Wentzel-VI energies)
     // amplifies by 1/sin^2 in sin and then in every later direction.
-    double const sin_t = sqrt(max0(1.0 - __dmul_rn(cos_t, cos_t)));
-    double const phi = kTwoPi * u_phi;
+    double const s2 = 1.0 - __dmul_rn(cos_t, cos_t);
+    double const rho2 = fma(a, a, b * b);
+    double const q = gt0(s2) ? s2 * frsqrt(s2 * rho2) : 0.0;
     double sp, cp;
-    sincos(phi, &sp, &cp);
-    ox = ax * cos_t + sin_t * (cp * b1x + sp * b2x);
-    oy = ay * cos_t + sin_t * (cp * b1y + sp * b2y);
-    oz = az * cos_t + sin_t * (cp * b1z + sp * b2z);
+    sincos_turn(arena, u_phi, sp, cp);
+    double const A = q * cp, B = q * sp;
+    double const h = fma(-B, pole, cos_t);
+    double const op = fma(pole, cos_t, B * rho2);
+    double const oa = fma(a, h, -(A * b));
+    double const ob = fma(b, h, A * a);
+    ox = about_x ? op : oa;
+    oy = about_x ? oa : ob;
+    oz = about_x ? ob : op;
+}
+// The same about any axis and for any cos_t (clamped), u_phi in [0, 1).
+__device__ __forceinline__ void cone_direction(const double* __restrict__ arena, double ax, double ay, double az,
+                                               double cos_t, double u_phi, double& ox, double& oy, double& oz)
+{
+    normalize(ax, ay, az);
+    cone_unit(arena, ax, ay, az, fmin(1.0, fmax(-1.0, cos_t)), u_phi, ox, oy, oz);
 }
 // O/RreaChargedInterleave.H:371-389
 __device__ __forceinline__ int poisson_capped(double mean, double u, int kmax)
@@ -330,7 +425,7 @@ __device__ __forceinline__ double moller_cos(double kp, double ks_or_scat)
     double const v = ks_or_scat * (kp + 2.0 * kMeC2) / (kp * (ks_or_scat + 2.0 * kMeC2));
     return sqrt(fmin(1.0, max0(v)));
 }
-__device__ __forceinline__ void moller_lab_directions(double px, double py, double pz, double kp, double ks,
+__device__ __forceinline__ void moller_lab_directions(const double* __restrict__ arena, double px, double py, double pz, double kp, double ks,
                                                       double u_az, double& opx, double& opy, double& opz,
                                                       double& osx, double& osy, double& osz)
 {
@@ -346,8 +441,8 @@ __device__ __forceinline__ void moller_lab_directions(double px, double py, doub
         double const scat = max0(kp - ks);
         cpm = (le0(kp) || le0(scat)) ? 1.0 : moller_cos(kp, scat);
     }
-    cone_direction(px, py, pz, cs, u_az, osx, osy, osz);
-    cone_direction(px, py, pz, cpm, unit_cycle(u_az + 0.5), opx, opy, opz);
+    cone_unit(arena, px, py, pz, cs, u_az, osx, osy, osz);
+    cone_unit(arena, px, py, pz, cpm, unit_cycle(u_az + 0.5), opx, opy, opz);
 }
 // O/RreaChargedInterleave.H:465-496
 __device__ __forceinline__ void photon_recoil(double k0, double eg, double gx, double gy, double gz, double& cx,
@@ -368,35 +463,41 @@ __device__ __forceinline__ void photon_recoil(double k0, double eg, double gx, d
 }
 
 struct FieldRange {
-    double work, ex, ey, ez, bx, by, bz, length;
+    double work, ex, ey, ez, bx, by, length;  // B is azimuthal: no z component
 };
 
 // O/RreaChargedInterleave.H:100-138 with the Boris rotation of
-// I/RreaLorentzPush.H:21-46
-__device__ __forceinline__ void half_kick(FieldRange const& f, double half_dt, double q, double& k, double& dx,
+// I/RreaLorentzPush.H:21-46, in units of c: v = u/c with |v| = gb at energy k.
+// The rotation keeps |v|, so the norm of the kicked vector (needed for its
+// gamma) normalises the result; without B nothing rotates.
+__device__ __forceinline__ void half_kick(FieldRange const& f, double half_dt, double q, double gb, double& k, double& dx,
                                           double& dy, double& dz)
 {
-    double const umag = proper_velocity_from_kinetic(k);
-    double const s = q * (kC * kC / kMeC2) * half_dt;
-    double const uxm = umag * dx + s * f.ex;
-    double const uym = umag * dy + s * f.ey;
-    double const uzm = umag * dz + s * f.ez;
-    double const gamma = sqrt(1.0 + (uxm * uxm + uym * uym + uzm * uzm) / (kC * kC));
-    Divisor const d2g = make_divisor(2.0 * gamma);
-    double const tx = quot(s * f.bx, d2g), ty = quot(s * f.by, d2g), tz = quot(s * f.bz, d2g);
-    double const t2 = tx * tx + ty * ty + tz * tz;
-    Divisor const d1t = make_divisor(1.0 + t2);
-    double const sx = quot(2.0 * tx, d1t), sy = quot(2.0 * ty, d1t), sz = quot(2.0 * tz, d1t);
-    double const ppx = uxm + uym * tz - uzm * ty;
-    double const ppy = uym + uzm * tx - uxm * tz;
-    double const ppz = uzm + uxm * ty - uym * tx;
-    double const ux = uxm + ppy * sz - ppz * sy;
-    double const uy = uym + ppz * sx - ppx * sz;
-    double const uz = uzm + ppx * sy - ppy * sx;
-    double const norm = sqrt(ux * ux + uy * uy + uz * uz);
-    if (gt0(norm) && finite_bits(norm)) {
-        Divisor const dn = make_divisor(norm);
-        dx = quot(ux, dn); dy = quot(uy, dn); dz = quot(uz, dn);
+    double const s = q * (kC / kMeC2) * half_dt;
+    double vx = fma(gb, dx, s * f.ex);
+    double vy = fma(gb, dy, s * f.ey);
+    double vz = fma(gb, dz, s * f.ez);
+    double const v2 = vx * vx + vy * vy + vz * vz;
+    if (ne0(f.bx) || ne0(f.by)) {
+        // t = q B dt / (2 m gamma), w = 2 t / (1 + t^2)
+        double const h = (0.5 * kC) * s * frsqrt(1.0 + v2);
+        double const tx = h * f.bx, ty = h * f.by;
+        double const t2 = tx * tx + ty * ty;
+        // 1 / (1 + t^2): below t^2 = 2^-18 the series' next term is below 2^-54
+        double const d = 2.0 * (__double2hiint(t2) < 0x3ed00000 ? fma(t2, t2 - 1.0, 1.0) : 1.0 / (1.0 + t2));
+        double const wx = tx * d, wy = ty * d;
+        double const px = vx - vz * ty;
+        double const py = vy + vz * tx;
+        double const pz = vz + vx * ty - vy * tx;
+        vx -= pz * wy;
+        vy += pz * wx;
+        vz += px * wy - py * wx;
+    }
+    if (gt0(v2) && finite_bits(v2)) {
+        double const inv = frsqrt(v2);
+        dx = vx * inv;
+        dy = vy * inv;
+        dz = vz * inv;
     }
     k = max0(k + 0.5 * f.work);
 }
@@ -431,17 +532,39 @@ struct FieldView {
     }
 };
 
+// x / d - offset (0 or 1/2) split into a whole cell and the fraction in it:
+// the whole part is read from the low word of a sum (a floor and two
+// conversions otherwise, 3 to 4 FP64 slots).  Within an ulp of a cell's edge
+// the split may name either neighbour with a fraction of 1 or 0 (to an ulp):
+// the weights on either are the same.
+template <bool Centred>
+__device__ __forceinline__ void split_cell(double x, Divisor const& d, int& cell, double& fraction)
+{
+    constexpr double magic = 6755399441055744.0;   // 1.5 2^52: the sum's low word is the nearest integer
+    if constexpr (Centred) {
+        double const t = fma(x, d.y, magic - 1.0);   // nearest of (x/d - 1/2) - 1/2
+        cell = __double2loint(t);
+        fraction = fma(x, d.y, -0.5) - (t - magic);
+    } else {
+        double const t = fma(x, d.y, magic);
+        cell = __double2loint(t);
+        fraction = fma(x, d.y, magic - t);
+        if (lt0(fraction)) {
+            cell -= 1;
+            fraction += 1.0;
+        }
+    }
+}
+
 // S/RreaAmrexAdvance.cpp:532-579 with I/RreaFieldGatherStencil.H:49-133 and
 // MaxwellBthetaAt :511-530
 __device__ __forceinline__ void gather(FieldView const& fv, double r, double z, double& er, double& ez, double& bth)
 {
-    double const fx = quot(r - fv.r_lo, fv.div_dr) + 0.0 - 0.5;
-    double const fz = quot(z - fv.z_lo, fv.div_dz) + 0.0 - 0.5;
-    double const flx = floor(fx), flz = floor(fz);
-    int const ir0 = static_cast<int>(flx);
-    int const iz0 = static_cast<int>(flz);
-    double const tx = fx - static_cast<double>(ir0);
-    double const tz = fz - static_cast<double>(iz0);
+    int ir0, iz0;
+    double tx, tz;
+    double const zr = z - fv.z_lo;
+    split_cell<true>(r - fv.r_lo, fv.div_dr, ir0, tx);
+    split_cell<true>(zr, fv.div_dz, iz0, tz);
     int const i0 = max(0, min(fv.nr - 1, ir0));
     int const i1 = max(0, min(fv.nr - 1, ir0 + 1));
     int j0, j1;
@@ -453,27 +576,32 @@ __device__ __forceinline__ void gather(FieldView const& fv, double r, double z, 
         j1 = max(0, min(fv.nz - 1, iz0 + 1));
     }
     size_t const r0 = static_cast<size_t>(fv.nr) * j0, r1 = static_cast<size_t>(fv.nr) * j1;
-    double const e00 = __ldg(fv.cell_er + i0 + r0), e01 = __ldg(fv.cell_er + i0 + r1);
-    double const e10 = __ldg(fv.cell_er + i1 + r0), e11 = __ldg(fv.cell_er + i1 + r1);
-    double const z00 = __ldg(fv.cell_ez + i0 + r0), z01 = __ldg(fv.cell_ez + i0 + r1);
-    double const z10 = __ldg(fv.cell_ez + i1 + r0), z11 = __ldg(fv.cell_ez + i1 + r1);
-    double const first_center = fv.r_lo + 0.5 * fv.dr;
-    double const axis = r >= first_center ? 1.0 : max0((r - fv.r_lo) / (0.5 * fv.dr));
-    er = ((1.0 - tx) * ((1.0 - tz) * e00 + tz * e01) + tx * ((1.0 - tz) * e10 + tz * e11)) * axis;
-    ez = (1.0 - tx) * ((1.0 - tz) * z00 + tz * z01) + tx * ((1.0 - tz) * z10 + tz * z11);
+    auto bilinear = [](double v00, double v01, double v10, double v11, double a, double b) {
+        double const lo = fma(b, v01 - v00, v00), hi = fma(b, v11 - v10, v10);
+        return fma(a, hi - lo, lo);
+    };
+    er = bilinear(__ldg(fv.cell_er + i0 + r0), __ldg(fv.cell_er + i0 + r1), __ldg(fv.cell_er + i1 + r0),
+                  __ldg(fv.cell_er + i1 + r1), tx, tz);
+    ez = bilinear(__ldg(fv.cell_ez + i0 + r0), __ldg(fv.cell_ez + i0 + r1), __ldg(fv.cell_ez + i1 + r0),
+                  __ldg(fv.cell_ez + i1 + r1), tx, tz);
+    // inside the first cell centre Er falls linearly to the axis
+    if (ir0 < 0) er *= max0(2.0 * quot(r - fv.r_lo, fv.div_dr));
     if (!fv.has_b || le0(r)) {
         bth = 0.0;
-        if (!fv.has_b && gt0(r)) bth = 0.0;
         return;
     }
-    double const fr = fmin(max0(quot(r, fv.div_dr)), static_cast<double>(fv.nr));
-    double const fzz = fmin(max0(quot(z - fv.z_lo, fv.div_dz)), static_cast<double>(fv.nz));
-    int const a0 = min(static_cast<int>(floor(fr)), fv.nr - 1);
-    int const b0 = min(static_cast<int>(floor(fzz)), fv.nz - 1);
-    double const tr = fr - a0, tzz = fzz - b0;
+    int a0, b0;
+    double tr, tzz;
+    split_cell<false>(r, fv.div_dr, a0, tr);
+    split_cell<false>(zr, fv.div_dz, b0, tzz);
+    // the corners' range, clamped as r <= nr dr and 0 <= z - z_lo <= nz dz are
+    if (a0 < 0) { a0 = 0; tr = 0.0; }
+    if (a0 > fv.nr - 1) { a0 = fv.nr - 1; tr = 1.0; }
+    if (b0 < 0) { b0 = 0; tzz = 0.0; }
+    if (b0 > fv.nz - 1) { b0 = fv.nz - 1; tzz = 1.0; }
     size_t const w = static_cast<size_t>(fv.nr + 1);
-    bth = (1.0 - tr) * ((1.0 - tzz) * __ldg(fv.bt + a0 + w * b0) + tzz * __ldg(fv.bt + a0 + w * (b0 + 1)))
-        + tr * ((1.0 - tzz) * __ldg(fv.bt + a0 + 1 + w * b0) + tzz * __ldg(fv.bt + a0 + 1 + w * (b0 + 1)));
+    const double* const corner = fv.bt + a0 + w * b0;
+    bth = bilinear(__ldg(corner), __ldg(corner + w), __ldg(corner + 1), __ldg(corner + w + 1), tr, tzz);
 }
 
 // O/RreaPathFieldWork.H:57-150 with the two-node rule of
@@ -482,26 +610,23 @@ template <int NP>
 __device__ __forceinline__ FieldRange path_field_work(FieldView const& fv, Geom const& g, Path<NP> const& p, double q,
                                                       double begin, double end, Err& err)
 {
-    FieldRange res{0, 0, 0, 0, 0, 0, 0, 0};
+    FieldRange res{0, 0, 0, 0, 0, 0, 0};
     if (!(gt0(p.full))) return res;
     begin = fmax(p.in_begin, begin);
     end = fmin(p.in_end, end);
     if (!(end > begin)) return res;
-    Divisor const dfull = make_divisor(p.full);
-    double const pdx = quot(p.ex - p.sx, dfull);
-    double const pdy = quot(p.ey - p.sy, dfull);
-    double const pdz = quot(p.ez - p.sz, dfull);
+    double const pdx = p.dx * p.inv_full, pdy = p.dy * p.inv_full, pdz = p.dz * p.inv_full;
 #pragma unroll
     for (int ip = 0; ip < NP; ++ip) {
         if (ip >= p.npieces) break;
         Piece const& pc = p.pieces[ip];
-        double const pb = fmax(begin, pc.begin);
-        double const pe = fmin(end, pc.end);
-        if (!(pe > pb)) continue;
+        double const pb = NP == 1 ? begin : fmax(begin, pc.begin);
+        double const pe = NP == 1 ? end : fmin(end, pc.end);
+        if (NP != 1 && !(pe > pb)) continue;
         double const mid = 0.5 * (pb + pe);
         double const half = 0.5 * (pe - pb);
         double const off = half * kGl2Node;
-        double acc[7];
+        double acc[6];
 #pragma unroll
         for (int node = 0; node < 2; ++node) {
             double const f = node == 0 ? mid - off : mid + off;
@@ -512,40 +637,44 @@ __device__ __forceinline__ FieldRange path_field_work(FieldView const& fv, Geom 
             double const r2 = fma(x, x, y * y);
             double r = 0.0, rad = 0.0, rc = 1.0, rs = 0.0;
             if (gt0(r2)) {
-                double const inv = rsqrt(r2);
+                double const inv = frsqrt(r2);
                 r = r2 * inv;
-                rad = (pdx * x + pdy * y) * inv;
                 rc = x * inv;
                 rs = y * inv;
+                rad = pdx * rc + pdy * rs;
             }
             double er, ez, bth;
             gather(fv, r, z, er, ez, bth);
-            double const work = q * (er * rad + ez * pdz) * 1.0;
+            double const work = er * rad + ez * pdz;
             if (!finite_bits(work) || !finite_bits(er) || !finite_bits(ez) || !finite_bits(bth)) {
                 err.set(RREA_GPU_ERR_INVALID_STATE);
             }
-            double const v[7] = {work, er * rc, er * rs, ez, -bth * rs, bth * rc, 0.0};
-            if (node == 0) {
+            double const v[6] = {work, er * rc, er * rs, ez, -bth * rs, bth * rc};
 #pragma unroll
-                for (int c = 0; c < 7; ++c) acc[c] = v[c];
-            } else {
-#pragma unroll
-                for (int c = 0; c < 7; ++c) acc[c] = half * (acc[c] + v[c]);
-            }
+            for (int c = 0; c < 6; ++c) acc[c] = node == 0 ? v[c] : acc[c] + v[c];
         }
-        res.work += p.full * acc[0];
-        res.ex += p.full * acc[1];
-        res.ey += p.full * acc[2];
-        res.ez += p.full * acc[3];
-        res.bx += p.full * acc[4];
-        res.by += p.full * acc[5];
-        res.bz += p.full * acc[6];
+        double const w = p.full * half;
+        res.work += (q * w) * acc[0];
+        if constexpr (NP == 1) {
+            // one piece: the mean over the path is the mean of its two nodes
+            res.ex = 0.5 * acc[1];
+            res.ey = 0.5 * acc[2];
+            res.ez = 0.5 * acc[3];
+            res.bx = 0.5 * acc[4];
+            res.by = 0.5 * acc[5];
+        } else {
+            res.ex += w * acc[1];
+            res.ey += w * acc[2];
+            res.ez += w * acc[3];
+            res.bx += w * acc[4];
+            res.by += w * acc[5];
+        }
         res.length += p.full * (pe - pb);
     }
-    if (gt0(res.length)) {
+    if (NP != 1 && gt0(res.length)) {
         Divisor const dl = make_divisor(res.length);
         res.ex = quot(res.ex, dl); res.ey = quot(res.ey, dl); res.ez = quot(res.ez, dl);
-        res.bx = quot(res.bx, dl); res.by = quot(res.by, dl); res.bz = quot(res.bz, dl);
+        res.bx = quot(res.bx, dl); res.by = quot(res.by, dl);
     }
     return res;
 }
@@ -620,12 +749,11 @@ __device__ __forceinline__ void build_intervals(Path<NP> const& p, double rho, I
     if constexpr (NP == 1) {
         Piece const& pc = p.pieces[0];
         if (p.npieces < 1 || !(gt0(pc.length))) return;
-        double dl = 0.0;
-        if (pc.end > pc.begin && gt0(p.full)) dl = p.full * (pc.end - pc.begin) * positive_or(rho, rho);
         iv.begin[0] = pc.begin;
         iv.end[0] = pc.end;
         iv.length[0] = pc.length;
-        iv.density[0] = positive_or(dl / pc.length, rho);
+        // the reference's (length * rho) / length, to within an ulp
+        iv.density[0] = rho;
         iv.n = 1;
     } else {
         for (int i = 0; i < p.npieces; ++i) {
@@ -679,6 +807,10 @@ __device__ __forceinline__ void build_intervals(Path<NP> const& p, Geom const& g
 template <int NP>
 __device__ __forceinline__ double density_path(Intervals<NP> const& iv, Path<NP> const& p, double b, double e)
 {
+    if constexpr (NP == 1) {
+        // the one interval is the path's inside, and every caller's [b, e] lies in it
+        return iv.n > 0 && e > b ? p.full * (e - b) * iv.density[0] : 0.0;
+    }
     b = fmax(p.in_begin, b);
     e = fmin(p.in_end, e);
     if (!(e > b)) return 0.0;

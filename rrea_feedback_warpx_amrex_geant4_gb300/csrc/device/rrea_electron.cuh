@@ -362,12 +362,70 @@ __device__ __forceinline__ double sample_single_elastic_cos(StepConstants const&
     return 1.0 - 2.0 * eta * u / (1.0 + eta - u);
 }
 // S/RreaInteractionTables.cpp:2714-2760
-__device__ __forceinline__ double tsai_g2(double x)
+static __device__ __noinline__ double tsai_g2(double x)
 {
     if (x < 1.0e-3) {
         return x * x * (0.5 + x * (-1.0 / 3.0 + x * (1.0 / 8.0 + x * (-1.0 / 30.0 + x * (1.0 / 144.0)))));
     }
     return -expm1(-x) - x * exp(-x);
+}
+// The root x in [0, umax] of m(x) = target, m(x) = (G(a x) + 3 G(3 a x)) / 4
+// with G = tsai_g2 (increasing), which the reference finds by 60 bisections.
+// One photon in a warp made the whole warp pay 240 exponentials for it, a
+// third of the electron kernel's FP64 slots.  Here 20 bisections in FP32 over
+// the bit patterns (so over the logarithm of x) bracket it to 2^-14, and
+// Halley steps on m, m' and m'' in FP64 (G' = y exp(-y), G'' = (1 - y)
+// exp(-y); exp(-y) = 1 + expm1(-y)) square that three times over: two or
+// three steps until one is below 2^-40 of x.  The bisection stays for a root
+// the steps do not settle (the flat end, where m is 1 to rounding).
+// Measured, one resident phase of 2^21 scale-up electrons: 28.8 -> 26.9 ms.
+static __device__ __noinline__ double brems_angle_root(double target, double umax)
+{
+    double constexpr a = 0.625;
+    auto g32 = [](float y) {
+        return y < 0.25f ? y * y * (0.5f + y * (-1.0f / 3.0f + y * (0.125f - y * (1.0f / 30.0f))))
+                         : 1.0f - (1.0f + y) * __expf(-y);
+    };
+    float const t32 = static_cast<float>(target);
+    int lo32 = __float_as_int(1.0e-9f), hi32 = __float_as_int(fminf(static_cast<float>(umax), 128.0f));
+#pragma unroll 1
+    for (int it = 0; it < 20 && hi32 - lo32 > 1; ++it) {
+        int const mid = lo32 + ((hi32 - lo32) >> 1);
+        float const y = 0.625f * __int_as_float(mid);
+        if (0.25f * g32(y) + 0.75f * g32(3.0f * y) < t32) lo32 = mid; else hi32 = mid;
+    }
+    double x = static_cast<double>(__int_as_float(hi32));
+#pragma unroll 1
+    for (int it = 0; it < 8; ++it) {
+        double const y = a * x;
+        double m = 0.0, d1 = 0.0, d2 = 0.0;
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+            double const k = c == 0 ? 1.0 : 3.0, w = c == 0 ? 0.25 : 0.75;
+            double const v = k * y;
+            double const em = expm1(-v), e = 1.0 + em;
+            double const series =
+                v * v * (0.5 + v * (-1.0 / 3.0 + v * (1.0 / 8.0 + v * (-1.0 / 30.0 + v * (1.0 / 144.0)))));
+            m += w * (v < 1.0e-3 ? series : -em - v * e);
+            d1 += w * k * (v * e);
+            d2 += w * k * k * ((1.0 - v) * e);
+        }
+        if (!(gt0(d1))) break;
+        double const step = (target - m) / (a * d1);
+        double const next = x + step / (1.0 + 0.5 * step * (a * d2 / d1));
+        if (!(gt0(next)) || !(next <= umax)) break;
+        bool const done = fabs(next - x) <= 9.1e-13 * next;
+        x = next;
+        if (done) return x;
+    }
+    double lo = 0.0, hi = umax;
+#pragma unroll 1
+    for (int it = 0; it < 60; ++it) {
+        double const mid = 0.5 * (lo + hi);
+        double const m = 0.25 * tsai_g2(a * mid) + 0.75 * tsai_g2(3.0 * a * mid);
+        if (m < target) lo = mid; else hi = mid;
+    }
+    return 0.5 * (lo + hi);
 }
 __device__ __forceinline__ double sample_brems_cos(StepConstants const& C, double e, double cdf_u, Err& err)
 {
@@ -381,14 +439,7 @@ __device__ __forceinline__ double sample_brems_cos(StepConstants const& C, doubl
     double constexpr a = 0.625;
     double const umax = 2.0 * (1.0 + e / kMeC2);
     double const target = cdf_u * (0.25 * tsai_g2(a * umax) + 0.75 * tsai_g2(3.0 * a * umax));
-    double lo = 0.0, hi = umax;
-#pragma unroll 1
-    for (int it = 0; it < 60; ++it) {
-        double const mid = 0.5 * (lo + hi);
-        double const m = 0.25 * tsai_g2(a * mid) + 0.75 * tsai_g2(3.0 * a * mid);
-        if (m < target) lo = mid; else hi = mid;
-    }
-    double const f = 0.5 * (lo + hi) / umax;
+    double const f = brems_angle_root(target, umax) / umax;
     return 1.0 - 2.0 * f * f;
 }
 
@@ -413,7 +464,7 @@ __device__ __forceinline__ void moller_final_state(StepConstants const& C, Elect
                                     rng.uniform(rng_index, kChHardMollerEnergy), true, err);
     sec = fmax(C.hm_threshold_eV, fmin(sec, 0.5 * kb));
     double pdx, pdy, pdz, sdx, sdy, sdz;
-    moller_lab_directions(dx, dy, dz, kb, sec, rng.uniform(rng_index, kChHardMollerAzimuth), pdx, pdy, pdz, sdx, sdy,
+    moller_lab_directions(A.arena, dx, dy, dz, kb, sec, rng.uniform(rng_index, kChHardMollerAzimuth), pdx, pdy, pdz, sdx, sdy,
                           sdz);
     k = max0(kb - sec);
     dx = pdx; dy = pdy; dz = pdz;
@@ -449,7 +500,7 @@ __device__ __forceinline__ void brems_final_state(StepConstants const& C, Electr
     bool const tracked = finite_bits(C.photon_cutoff_eV) && ge0(C.photon_cutoff_eV) && eg >= C.photon_cutoff_eV;
     double const ct = sample_brems_cos(C, kb, rng.uniform(rng_index, POS ? kChPositronBremsAngle : kChBremsAngle), err);
     double gx, gy, gz;
-    cone_direction(dx, dy, dz, ct, rng.uniform(rng_index, POS ? kChPositronBremsAzimuth : kChBremsAzimuth), gx, gy,
+    cone_direction(A.arena, dx, dy, dz, ct, rng.uniform(rng_index, POS ? kChPositronBremsAzimuth : kChBremsAzimuth), gx, gy,
                    gz);
     photon_recoil(kb, eg, gx, gy, gz, dx, dy, dz);
     k = after;
@@ -498,7 +549,7 @@ __device__ __forceinline__ void bhabha_final_state(StepConstants const& C, Elect
     double const thr = C.hm_threshold_eV;
     if (!(gt0(sec)) || (gt0(thr) && sec < thr)) return;
     double pdx, pdy, pdz, sdx, sdy, sdz;
-    moller_lab_directions(dx, dy, dz, kb, sec, rng.uniform(rng_index, kChPositronBhabhaAzimuth), pdx, pdy, pdz, sdx,
+    moller_lab_directions(A.arena, dx, dy, dz, kb, sec, rng.uniform(rng_index, kChPositronBhabhaAzimuth), pdx, pdy, pdz, sdx,
                           sdy, sdz);
     k = max0(kb - sec);
     dx = pdx; dy = pdy; dz = pdz;
@@ -584,7 +635,7 @@ static __device__ __noinline__ uint32_t spawn_annihilation(ElectronArgs A, RngSt
         }
     }
     double g1x, g1y, g1z;
-    cone_direction(ax, ay, az, cos1, azim, g1x, g1y, g1z);
+    cone_direction(A.arena, ax, ay, az, cos1, azim, g1x, g1y, g1z);
     e1 = max0(e1);
     e2 = max0(e2);
     double g2x = -g1x, g2y = -g1y, g2z = -g1z;
@@ -649,7 +700,7 @@ static __device__ __noinline__ Dir3 gs_few_collisions(const double* __restrict__
         double const ct =
             sample_single_elastic_cos(C, arena, k, rng.uniform((sub << 8) | inner, ch_scatter), err, lk, species);
         double nx, ny, nz;
-        cone_direction(dx, dy, dz, ct, rng.uniform((sub << 8) | inner, ch_azimuth), nx, ny, nz);
+        cone_direction(arena, dx, dy, dz, ct, rng.uniform((sub << 8) | inner, ch_azimuth), nx, ny, nz);
         dx = nx; dy = ny; dz = nz;
     }
     return Dir3{dx, dy, dz, err.code};
@@ -690,7 +741,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
     constexpr int rate_base = POS ? RREA_T_P_COLLISION : RREA_T_E_COLLISION;
     const double* __restrict__ arena = A.arena;
     rrea_gpu_config const& cfg = C.cfg;
-    Geom const g{cfg.r_lo, cfg.r_hi, cfg.z_lo, cfg.z_hi, cfg.periodic_z != 0};
+    Geom const g = make_geom(C);
     double const cutoff = cfg.low_energy_cutoff_eV;
     double const rho = C.density_ratio;
     double const w_air = C.tix.w_air_eV_per_pair;
@@ -727,13 +778,15 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
     double const r_particle = prev_r, z_particle = run_z;
     double const x_particle = run_x, y_particle = run_y;
 
+    double gb = 0.0;  // gamma beta at the energy of the last chord
     auto build_chord = [&](double req_dt, Path<NP>& path) -> bool {
-        // O/RreaParticleInteraction.H:110-161
+        // O/RreaParticleInteraction.H:110-161; the direction is a unit vector
+        // (normalised by the half kick or the prologue, a cone apart), so the
+        // reference's division by its norm changes nothing beyond an ulp
         if (!finite_bits(req_dt) || !(ge0(req_dt))) return false;
-        double const speed = charged_speed(k);
-        double const dn = sqrt(dx * dx + dy * dy + dz * dz);
-        if (!finite_bits(speed) || !finite_bits(dn) || !(gt0(dn))) return false;
-        double const sc = speed * req_dt / dn;
+        double const speed = charged_speed(k, gb);
+        if (!finite_bits(speed) || !finite_bits(dx) || !finite_bits(dy) || !finite_bits(dz)) return false;
+        double const sc = speed * req_dt;
         double const exx = run_x + sc * dx, eyy = run_y + sc * dy, ezz = run_z + sc * dz;
         clip_xyz(run_x, run_y, run_z, exx, eyy, ezz, g, path, err);
         return finite_bits(path.full) && eq0(path.in_begin);
@@ -905,7 +958,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
     double mid_r = r_particle, mid_z = z_particle;
     double mid_x = x_particle, mid_y = y_particle, mid_elapsed = 1.0;
     double const sub_dt = dt_s / static_cast<double>(subcycles);
-    FieldRange sub_field{0, 0, 0, 0, 0, 0, 0, 0};
+    FieldRange sub_field{0, 0, 0, 0, 0, 0, 0};
     double sub_dt_eff = 0.0;
     uint64_t events = 0;
 
@@ -947,11 +1000,13 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
         double const total = sc + ss;
         // limiter
         double eff = b;
+        double path_m = 0.0;
         bool reaches = false;
         bool valid = false;
         if (finite_bits(b) && finite_bits(e) && finite_bits(k) && finite_bits(cutoff) && e >= b && k >= cutoff && ge0(cutoff)) {
             double const to_cut = k - cutoff;
-            double const req = total * density_path(iv, path, b, e);
+            path_m = density_path(iv, path, b, e);
+            double const req = total * path_m;
             if (finite_bits(req) && ge0(req)) {
                 valid = true;
                 if (req < to_cut) {
@@ -966,6 +1021,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
                             reaches = false;
                         }
                     }
+                    path_m = density_path(iv, path, b, eff);
                 }
             }
         }
@@ -973,7 +1029,6 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
             err.set(RREA_GPU_ERR_INVALID_STATE);
             return false;
         }
-        double const path_m = density_path(iv, path, b, eff);
         double const raw_col = sc * path_m;
         double const raw_soft = ss * path_m;
         double const avail = max0(k - cutoff);
@@ -984,7 +1039,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
 #pragma unroll
             for (int i = 0; i < NP; ++i) {
                 if (i >= iv.n) break;
-                double const bb = fmax(b, iv.begin[i]), ee = fmin(eff, iv.end[i]);
+                double const bb = NP == 1 ? b : fmax(b, iv.begin[i]), ee = NP == 1 ? eff : fmin(eff, iv.end[i]);
                 if (!(ee > bb)) continue;
                 double const raw = path.full * (ee - bb) * iv.density[i] * sc;
                 // with one interval raw is raw_col (the same products), and
@@ -995,7 +1050,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
                 double x, y, z;
                 point_at_full(path, g, 0.5 * (bb + ee), x, y, z);
                 // deposit_source(kind 0, sec POS ? 0 : cutoff/2, loss w_air) through the cache
-                ion_pairs.add(C, A.cells, rz_radius(x, y), z, pw);
+                ion_pairs.add(C, A.cells, fsqrt(fma(x, x, y * y)), z, pw);
             }
         }
         if constexpr (!POS) {
@@ -1064,7 +1119,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
             se = path.in_end;
             sub_field = path_field_work(fv, g, path, q, sb, se, err);
             sub_dt_eff = sub_dt * (se - sb);
-            half_kick(sub_field, 0.5 * sub_dt_eff, q, k, dx, dy, dz);
+            half_kick(sub_field, 0.5 * sub_dt_eff, q, gb, k, dx, dy, dz);
             if (k < cutoff) {
                 mark_stopped(sb);
                 break;
@@ -1189,13 +1244,13 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
                                                     rng.uniform(sub << 8, POS ? kChPositronGsAngle : kChElectronGsAngle),
                                                     err, species);
                     double nx, ny, nz;
-                    cone_direction(dx, dy, dz, ct, rng.uniform(sub << 8, POS ? kChPositronGsAzimuth : kChElectronGsAzimuth),
-                                   nx, ny, nz);
+                    cone_unit(arena, dx, dy, dz, ct,
+                              rng.uniform(sub << 8, POS ? kChPositronGsAzimuth : kChElectronGsAzimuth), nx, ny, nz);
                     dx = nx; dy = ny; dz = nz;
                 }
             }
         }
-        half_kick(sub_field, 0.5 * sub_dt_eff, q, k, dx, dy, dz);
+        half_kick(sub_field, 0.5 * sub_dt_eff, q, gamma_beta(k), k, dx, dy, dz);
         if (k < cutoff) {
             mark_stopped(se);
             break;
@@ -1205,7 +1260,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
             double x, y, z;
             point_at_full(path, g, se, x, y, z);
             double const wz = wrap_z(g, z);
-            if (!cartesian_half_open(g, x, y, wz)) {
+            if (!(NP == 1 && strictly_inside(g, fma(x, x, y * y), wz)) && !cartesian_half_open(g, x, y, wz)) {
                 exited = true;
                 break;
             }

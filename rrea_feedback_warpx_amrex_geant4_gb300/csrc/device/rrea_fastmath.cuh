@@ -19,6 +19,7 @@
 #pragma once
 
 #include "../rrea_arena.h"
+#include "rrea_rate_rows.cuh"
 
 #include <stdint.h>
 
@@ -26,6 +27,8 @@ namespace rrea_dev {
 
 constexpr double kLn2Hi = 6.93147180559945286227e-01;   // RN(ln 2)
 constexpr double kLn2Lo = 2.31904681384629955842e-17;   // RN(ln 2 - kLn2Hi)
+
+static __device__ __noinline__ double log_any(double x) { return log(x); }
 
 __device__ __forceinline__ double flog(const double* __restrict__ arena, double x)
 {
@@ -36,17 +39,18 @@ __device__ __forceinline__ double flog(const double* __restrict__ arena, double 
 #endif
     long long const bits = __double_as_longlong(x);
     // normal, positive and finite: sign clear, biased exponent in [1, 2046]
-    if (bits < 0x0010000000000000LL || bits >= 0x7ff0000000000000LL) return log(x);
-    int const e = static_cast<int>(bits >> 52) - 1023;
+    if (bits < 0x0010000000000000LL || bits >= 0x7ff0000000000000LL) return log_any(x);
     long long const mant = bits & 0x000fffffffffffffLL;
     int const j = static_cast<int>((mant + (1LL << 43)) >> 44);  // nearest of the 257 points, 0..256
     double const m = __longlong_as_double(mant | 0x3ff0000000000000LL);
-    double const f = m - (1.0 + static_cast<double>(j) * 0.00390625);
+    // F = 1 + j/256 by its bits (j = 256 carries into the exponent: 2)
+    double const f = m - __longlong_as_double(0x3ff0000000000000LL + (static_cast<long long>(j) << 44));
     const double* t = arena + RREA_ARENA_LOG_TABLE + 3 * j;
     double const r = f * __ldg(t);
     double const q = fma(r, fma(r, fma(r, fma(r, -1.0 / 6.0, 1.0 / 5.0), -0.25), 1.0 / 3.0), -0.5);
     double const p = fma(r * r, q, r);
-    double const de = static_cast<double>(e);
+    // e = biased exponent - 1023 as a double, by the low word of 2^52 + it
+    double const de = __longlong_as_double(0x4330000000000000LL | (bits >> 52)) - (4503599627370496.0 + 1023.0);
     double const hi = fma(de, kLn2Hi, __ldg(t + 1));
     double const lo = fma(de, kLn2Lo, __ldg(t + 2)) + p;
     return hi + lo;
@@ -57,12 +61,16 @@ __device__ __forceinline__ double flog(const double* __restrict__ arena, double 
 // 15(2), 1989: k = rint(x 128/ln2), x = k ln2/128 + r with |r| <= ln2/256
 // (r from the split of ln2/128, two FMAs), exp x = 2^(k div 128) *
 // 2^((k mod 128)/128) * exp(r), expm1(r) by its Taylor series through r^5
-// (first omitted term below 2^-62).  2^(j/128) comes from the table as two
-// doubles.  Within two ulps of the correctly rounded exponential for
-// |x| < 700; larger, infinite and NaN arguments go to the CUDA exp.
+// (first omitted term below 2^-62; the r^4 and r^5 terms, below 2^-38, in
+// FP32).  2^(j/128) comes from the table as two doubles.  k is read from the
+// low word of a sum and 2^(k div 128) added to the exponent, so neither takes
+// a conversion or a product.  Within two ulps of the correctly rounded
+// exponential for |x| < 512; the rest goes to the CUDA exp.
 constexpr double kInvLn2x128 = 1.84664965233787316142e+02;  // RN(128 / ln 2)
 constexpr double kLn2by128Hi = 5.41521234812457272982e-03;  // RN(ln 2 / 128)
 constexpr double kLn2by128Lo = 1.81175532331742157843e-19;  // RN(ln 2 / 128 - kLn2by128Hi)
+
+static __device__ __noinline__ double exp_any(double x) { return exp(x); }
 
 __device__ __forceinline__ double fexp(const double* __restrict__ arena, double x)
 {
@@ -71,18 +79,67 @@ __device__ __forceinline__ double fexp(const double* __restrict__ arena, double 
     (void)arena;
     return exp(x);
 #endif
-    if (!(fabs(x) < 700.0)) return exp(x);
-    double const kf = rint(x * kInvLn2x128);
-    int const k = static_cast<int>(kf);
+    // |x| >= 512, infinite or NaN
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x40800000) return exp_any(x);
+    constexpr double magic = 6755399441055744.0;   // 1.5 2^52: the sum's low word is the nearest integer
+    double const t = fma(x, kInvLn2x128, magic);
+    int const k = __double2loint(t);
+    double const kf = t - magic;
     double r = fma(-kf, kLn2by128Hi, x);
     r = fma(-kf, kLn2by128Lo, r);
-    double const q = fma(r, fma(r, fma(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5);
+    float const r32 = narrow_f32(r);
+    double const q = fma(r, widen_f32(r32 * (1.0f / 24.0f + r32 * (1.0f / 120.0f))) + 1.0 / 6.0, 0.5);
     double const p = fma(r * r, q, r);  // expm1(r)
-    const double* t = arena + RREA_ARENA_EXP_TABLE + 2 * (k & 127);
-    double const th = __ldg(t);
-    double const v = th + fma(th, p, __ldg(t + 1));
-    // 2^(k >> 7): |k| < 129,300, so the exponent stays in the normal range
-    return v * __longlong_as_double(static_cast<long long>((k >> 7) + 1023) << 52);
+    double2 const tab = __ldg(reinterpret_cast<const double2*>(arena + RREA_ARENA_EXP_TABLE) + (k & 127));
+    double const v = tab.x + fma(tab.x, p, tab.y);
+    // 2^(k >> 7) into the exponent: |k| < 94,600, so v stays normal
+    return __longlong_as_double(__double_as_longlong(v) + (static_cast<long long>(k >> 7) << 52));
+}
+
+// 1/sqrt(x) for the normalisations of the loop: an FP32 seed (relative error
+// below 2^-21) and one third-order Householder step, y (1 + e/2 + 3 e^2/8)
+// with e = 1 - x y^2 (the remainder 5 e^3/16 is below 2^-62), five FP64
+// slots; within an ulp.  Arguments outside [2^-100, 2^100] go to CUDA's.
+static __device__ __noinline__ double rsqrt_any(double x) { return rsqrt(x); }
+
+__device__ __forceinline__ double frsqrt(double x)
+{
+    uint32_t const hi = static_cast<uint32_t>(__double2hiint(x));
+    if (hi - 0x39b00000u > 0x0c800000u) return rsqrt_any(x);
+    uint32_t const lo = static_cast<uint32_t>(__double2loint(x));
+    float const x32 = __uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29));
+    float y32;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y32) : "f"(x32));
+    uint32_t const u = __float_as_uint(y32);
+    double const y = __hiloint2double(static_cast<int>((u >> 3) + 0x38000000u), static_cast<int>(u << 29));
+    double const e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+// sqrt(x) = x / sqrt(x), within two ulps; 0 for 0 (and for anything not positive)
+__device__ __forceinline__ double fsqrt(double x)
+{
+    return __double2hiint(x) > 0 ? x * frsqrt(x) : 0.0;
+}
+
+// sin and cos of 2 pi u for u in [0, 1): the nearest of 256 table angles and
+// the remainder r (|r| <= pi/256, exact up to the product by 2 pi/256), whose
+// sin and cos - 1 are r - r^3/6 + r^5/120 and -r^2/2 + r^4/24 - r^6/720, the
+// terms from r^4 on in FP32; within 2^-52 absolutely, for 14 FP64 slots
+// against 31 of a reduction of 2 pi u.  It takes the angle itself, where the
+// reference rounds 2 pi u (to 4e-16) first.
+__device__ __forceinline__ void sincos_turn(const double* __restrict__ arena, double u, double& s, double& c)
+{
+    constexpr double magic = 6755399441055744.0;   // 1.5 2^52: the sum's low word is the nearest integer
+    double const t = fma(u, 256.0, magic);
+    int const j = __double2loint(t) & 255;
+    double const r = fma(u, 256.0, magic - t) * 2.45436926061702596755e-02;   // 2 pi / 256
+    double2 const tab = __ldg(reinterpret_cast<const double2*>(arena + RREA_ARENA_TURN_TABLE) + j);
+    double const r2 = r * r;
+    float const q = narrow_f32(r2);
+    double const cm = r2 * (widen_f32(q * (1.0f / 24.0f - q * (1.0f / 720.0f))) - 0.5);
+    double const sr = fma(r * r2, widen_f32(q * (1.0f / 120.0f)) - 1.0 / 6.0, r);
+    s = fma(tab.y, sr, fma(tab.x, cm, tab.x));
+    c = fma(-tab.x, sr, fma(tab.y, cm, tab.y));
 }
 
 }  // namespace rrea_dev

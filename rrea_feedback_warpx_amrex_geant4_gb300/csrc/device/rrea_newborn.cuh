@@ -100,7 +100,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
 {
     const double* __restrict__ arena = A.arena;
     rrea_gpu_config const& cfg = C.cfg;
-    Geom const g{cfg.r_lo, cfg.r_hi, cfg.z_lo, cfg.z_hi, cfg.periodic_z != 0};
+    Geom const g = make_geom(C);
     constexpr double q = POS ? 1.0 : -1.0;
     constexpr int species = POS ? 1 : 0;
     constexpr int rate_base = POS ? RREA_T_P_COLLISION : RREA_T_E_COLLISION;
@@ -227,7 +227,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
     double final_fraction = 0.0;
     bool terminal_interaction = false, terminal_at_point = false, exited = false;
     uint64_t completed = 0;
-    FieldRange sub_field{0, 0, 0, 0, 0, 0, 0, 0};
+    FieldRange sub_field{0, 0, 0, 0, 0, 0, 0};
     double sub_dt_eff = 0.0;
     auto elapsed_at = [&](double f) {
         double const within = fmin(1.0, max0(f));
@@ -337,10 +337,14 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
         double sb, se;
         {
             // RreaBuildRunningChargedChord with the residual dt as the step bound
-            double const speed = charged_speed(k);
-            double const dn = sqrt(dx * dx + dy * dy + dz * dz);
-            if (!finite_bits(sub_dt) || !(ge0(sub_dt)) || !finite_bits(speed) || !finite_bits(dn) || !(gt0(dn))) break;
-            double const sc = speed * sub_dt / dn;
+            // (the direction is a unit vector, as in the live loop)
+            double gb;
+            double const speed = charged_speed(k, gb);
+            if (!finite_bits(sub_dt) || !(ge0(sub_dt)) || !finite_bits(speed) || !finite_bits(dx) || !finite_bits(dy)
+                || !finite_bits(dz)) {
+                break;
+            }
+            double const sc = speed * sub_dt;
             double const exx = run_x + sc * dx, eyy = run_y + sc * dy, ezz = run_z + sc * dz;
             Path<NP> np;
             clip_xyz(run_x, run_y, run_z, exx, eyy, ezz, g, np, err);
@@ -362,7 +366,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
             final_fraction = se;
             sub_field = path_field_work(fv, g, path, q, sb, se, err);
             sub_dt_eff = sub_dt * (se - sb);
-            half_kick(sub_field, 0.5 * sub_dt_eff, q, k, dx, dy, dz);
+            half_kick(sub_field, 0.5 * sub_dt_eff, q, gb, k, dx, dy, dz);
             if (k < cut) {
                 final_fraction = sb;
                 terminal_at_point = true;
@@ -483,7 +487,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
                             rng.uniform(ii, POS ? kChNewbornPositronGsFewScatter : kChNewbornElectronGsFewScatter), err,
                             lk, species);
                         double nx, ny, nz;
-                        cone_direction(dx, dy, dz, ct,
+                        cone_direction(arena, dx, dy, dz, ct,
                                        rng.uniform(ii, POS ? kChNewbornPositronGsFewAzimuth
                                                            : kChNewbornElectronGsFewAzimuth),
                                        nx, ny, nz);
@@ -495,7 +499,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
                         C, arena, rc, k, gs_n,
                         rng.uniform(i0, POS ? kChNewbornPositronGsAngle : kChNewbornElectronGsAngle), err, species);
                     double nx, ny, nz;
-                    cone_direction(dx, dy, dz, ct,
+                    cone_direction(arena, dx, dy, dz, ct,
                                    rng.uniform(i0, POS ? kChNewbornPositronGsAzimuth : kChNewbornElectronGsAzimuth), nx,
                                    ny, nz);
                     dx = nx; dy = ny; dz = nz;
@@ -503,7 +507,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
             }
         }
         if (err.code) break;
-        half_kick(sub_field, 0.5 * sub_dt_eff, q, k, dx, dy, dz);
+        half_kick(sub_field, 0.5 * sub_dt_eff, q, gamma_beta(k), k, dx, dy, dz);
         if (k < cut) {
             final_fraction = se;
             terminal_at_point = true;
@@ -572,7 +576,7 @@ __device__ int advance_photon_newborn(StepConstants const& C, ElectronArgs const
 {
     const double* __restrict__ arena = A.arena;
     rrea_gpu_config const& cfg = C.cfg;
-    Geom const g{cfg.r_lo, cfg.r_hi, cfg.z_lo, cfg.z_hi, cfg.periodic_z != 0};
+    Geom const g = make_geom(C);
     double const cut = cfg.low_energy_cutoff_eV;
     double const photon_cut = C.photon_cutoff_eV;
     double const rho = C.density_ratio;
@@ -661,7 +665,7 @@ __device__ int advance_photon_newborn(StepConstants const& C, ElectronArgs const
             ComptonState const cs =
                 sample_klein_nishina(inc, rng.uniform(idx, kChComptonMu), rng.uniform(idx, kChComptonAccept));
             double sx, sy, sz;
-            cone_direction(dx, dy, dz, cs.cos_theta, rng.uniform(idx, kChComptonAzimuth), sx, sy, sz);
+            cone_direction(arena, dx, dy, dz, cs.cos_theta, rng.uniform(idx, kChComptonAzimuth), sx, sy, sz);
             double rx = inc * dx - cs.scattered * sx, ry = inc * dy - cs.scattered * sy, rz = inc * dz - cs.scattered * sz;
             normalize(rx, ry, rz);
             if (cs.recoil >= cut) {
@@ -720,7 +724,7 @@ __device__ int advance_photon_newborn(StepConstants const& C, ElectronArgs const
                 }
                 double const cth = sample_photoelectron_cos(ee, rng.uniform(idx, kChPhotoelectronCos));
                 double sx, sy, sz;
-                cone_direction(dx, dy, dz, cth, rng.uniform(idx, kChPhotoelectronAzimuth), sx, sy, sz);
+                cone_direction(arena, dx, dy, dz, cth, rng.uniform(idx, kChPhotoelectronAzimuth), sx, sy, sz);
                 child(0, 6, px, py, pz, sx, sy, sz, ee, b);
                 deposit_source(C, A.cells, 0, pr, pz, w, ee, ee);
             } else {

@@ -524,7 +524,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
 {
     const double* __restrict__ arena = A.arena;
     rrea_gpu_config const& cfg = C.cfg;
-    Geom const g{cfg.r_lo, cfg.r_hi, cfg.z_lo, cfg.z_hi, cfg.periodic_z != 0};
+    Geom const g = make_geom(C);
     double const cutoff = cfg.low_energy_cutoff_eV;
     double const photon_cut = C.photon_cutoff_eV;
     double const rho = C.density_ratio;
@@ -649,7 +649,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
             ComptonState const cs =
                 sample_klein_nishina(inc, rng.uniform(idx, kChComptonMu), rng.uniform(idx, kChComptonAccept));
             double sx, sy, sz;
-            cone_direction(dx, dy, dz, cs.cos_theta, rng.uniform(idx, kChComptonAzimuth), sx, sy, sz);
+            cone_direction(arena, dx, dy, dz, cs.cos_theta, rng.uniform(idx, kChComptonAzimuth), sx, sy, sz);
             double rx = inc * dx - cs.scattered * sx, ry = inc * dy - cs.scattered * sy,
                    rz = inc * dz - cs.scattered * sz;
             normalize(rx, ry, rz);
@@ -721,7 +721,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
                     return -1;
                 }
                 double ex, ey, ez;
-                cone_direction(dx, dy, dz, cth, rng.uniform(idx, kChPhotoelectronAzimuth), ex, ey, ez);
+                cone_direction(arena, dx, dy, dz, cth, rng.uniform(idx, kChPhotoelectronAzimuth), ex, ey, ez);
                 add_secondary(0, px, py, pz, ex, ey, ez, ee, birth);
                 deposit_source(C, A.cells, 0, pr, pz, weight, ee, ee);
             } else {
@@ -781,7 +781,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
             double const cos1 = 2.0 * clamp_unit(d_e) - 1.0;
             double const azim = wrap_unit(d_a);
             double g1x, g1y, g1z;
-            cone_direction(ax, ay, az, cos1, azim, g1x, g1y, g1z);
+            cone_direction(arena, ax, ay, az, cos1, azim, g1x, g1y, g1z);
             double const e1 = kMeC2, e2 = kMeC2;
             double local = 0.0;
             if (e1 >= photon_cut) add_secondary(2, px, py, pz, g1x, g1y, g1z, e1, birth);

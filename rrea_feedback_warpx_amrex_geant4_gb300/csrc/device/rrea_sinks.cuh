@@ -177,26 +177,30 @@ struct IonPairCache {
     __device__ __forceinline__ void add(StepConstants const& C, double* __restrict__ cells, double r, double z, double w)
     {
         if (!cells) return;
-        CellStencil const st = make_stencil(C, r, z);
-        if (!st.valid) return;
-        long long const key = (static_cast<long long>(st.j0) << 32) | static_cast<unsigned int>(st.i0);
+        rrea_gpu_config const& cfg = C.cfg;
+        double const zz = (cfg.periodic_z ? periodic_wrap(z, cfg.z_lo, cfg.z_hi) : z) - cfg.z_lo;
+        int i0, j0;
+        double wr1, wz1;
+        split_cell<true>(r - cfg.r_lo, C.div_dr, i0, wr1);
+        split_cell<true>(zz, C.div_dz, j0, wz1);
+        // the containing cell (the source counts only inside the grid): the
+        // upper one from a fraction of 1/2 on
+        int const ic = i0 + (__double2hiint(wr1) >= 0x3fe00000 ? 1 : 0);
+        int const jc = j0 + (__double2hiint(wz1) >= 0x3fe00000 ? 1 : 0);
+        if (ic < 0 || ic >= cfg.nr || jc < 0 || jc >= cfg.nz) return;
+        long long const key = (static_cast<long long>(j0) << 32) | static_cast<unsigned int>(i0);
         if (slot->key != key) {
             flush(C, cells);
             slot->key = key;
 #pragma unroll
             for (int q = 0; q < 4; ++q) slot->acc[q] = 0.0;
         }
-        double const wv = max0(w);
+        // rows and columns outside the grid are dropped at the flush
+        double const hi = max0(w) * wr1, lo = max0(w) - hi;
+        double const v[4] = {lo - lo * wz1, hi - hi * wz1, lo * wz1, hi * wz1};
 #pragma unroll
-        for (int a = 0; a < 2; ++a) {
-            double const wz = st.wz[a];
-            if (eq0(wz) || !st.use_j[a]) continue;
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                double const v = wv * st.wr[b] * wz;
-                if (eq0(v) || !st.use_i[b] || !finite_bits(v)) continue;
-                slot->acc[2 * a + b] += v;
-            }
+        for (int c = 0; c < 4; ++c) {
+            if (finite_bits(v[c])) slot->acc[c] += v[c];
         }
     }
 };

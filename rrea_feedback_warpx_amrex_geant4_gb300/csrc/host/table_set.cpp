@@ -204,6 +204,18 @@ void TableSet::Load(std::string const& config_path)
             x[2 * j + 1] = static_cast<double>(T - static_cast<long double>(hi));
         }
         if (push(x) != RREA_ARENA_EXP_TABLE) throw std::logic_error("exp table must follow the log table");
+        std::vector<double> turn(2 * RREA_ARENA_TURN_TABLE_ROWS);
+        for (int j = 0; j < RREA_ARENA_TURN_TABLE_ROWS; ++j) {
+            // the angle in the first octant, so that exact values come out exact
+            int const q = j / 64, i = j % 64;
+            long double const pi = 3.14159265358979323846264338327950288L;
+            int const o = i <= 32 ? i : 64 - i;
+            long double const a = std::sin(o * pi / 128.0L), b = std::cos(o * pi / 128.0L);
+            double const sn = static_cast<double>(i <= 32 ? a : b), cs = static_cast<double>(i <= 32 ? b : a);
+            turn[2 * j] = q == 0 ? sn : q == 1 ? cs : q == 2 ? -sn : -cs;
+            turn[2 * j + 1] = q == 0 ? cs : q == 1 ? -sn : q == 2 ? -cs : sn;
+        }
+        if (push(turn) != RREA_ARENA_TURN_TABLE) throw std::logic_error("turn table must follow the exp table");
     }
     std::string const dir = dir_of(config_path);
     JsonValue const cfg = ParseJson(read_text(config_path));

@@ -31,6 +31,9 @@
 // 32-byte boundary.
 #define RREA_ARENA_EXP_TABLE 772
 #define RREA_ARENA_EXP_TABLE_ROWS 128
+// Then {sin, cos} of j/256 turns, j = 0..255.
+#define RREA_ARENA_TURN_TABLE 1028
+#define RREA_ARENA_TURN_TABLE_ROWS 256
 
 enum RreaInterpMode {
     RREA_INTERP_LOGLOG = 0,

@@ -770,6 +770,10 @@ rrea_dev::StepConstants step_constants(rrea_gpu_ctx const* ctx, int32_t step, do
     double const configured = c.density_ratio > 0.0 ? c.density_ratio : 1.0;
     sc.density_ratio = ctx->profile_n > 0 ? (ctx->profile_step_ratio > 0.0 ? ctx->profile_step_ratio : configured)
                                           : configured;
+    double const r_in = c.r_hi * (1.0 - 1.0e-9), z_margin = 1.0e-9 * (c.z_hi - c.z_lo);
+    sc.r2_inner = r_in * r_in;
+    sc.z_inner_lo = c.z_lo + z_margin;
+    sc.z_inner_hi = c.z_hi - z_margin;
     sc.step_key = static_cast<uint64_t>(step > 0 ? step : 0);
     sc.dt_s = dt_s;
     sc.hm_enabled = c.debug_disable_hard_moller ? 0 : 1;
