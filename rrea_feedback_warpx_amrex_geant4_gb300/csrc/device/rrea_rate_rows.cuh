@@ -20,6 +20,7 @@
 
 #include "../rrea_arena.h"
 
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -131,7 +132,19 @@ RREA_HD double row_value(RowHit const& h, int c)
     float const tail = h.df * (t[0] + h.df * (t[1] + h.df * t[2]));
     double const c3 = p[3] + widen_f32(tail);
     double const c0 = p[0], c1 = p[1], c2 = p[2];
-    return c0 + h.d * (c1 + h.d * (c2 + h.d * c3));
+    return fma(h.d, fma(h.d, fma(h.d, c3, c2), c1), c0);
+}
+
+// d (column c) / d d = c1 + d (2 c2 + d (3 c3 + d (4 c4 + d (5 c5 + 6 d c6)))); divided by xc it is the
+// derivative by the argument.
+RREA_HD double row_slope(RowHit const& h, int c)
+{
+    const double* p = h.rec + RREA_ROW_HEADER + RREA_ROW_COLUMN * c;
+    const float* t = reinterpret_cast<const float*>(p + 4);
+    float const tail = h.df * (4.0f * t[0] + h.df * (5.0f * t[1] + h.df * 6.0f * t[2]));
+    double const c3 = 3.0 * p[3] + widen_f32(tail);
+    double const c1 = p[1], c2 = p[2];
+    return fma(h.d, fma(h.d, c3, 2.0 * c2), c1);
 }
 
 }  // namespace rrea_dev

@@ -266,6 +266,7 @@ struct AdjointSetup {
     double k_th, tau_k, z_p, tau_z, lambda;
     uint64_t seed;
     RreaTable1DIndex col, soft;
+    RreaRowIndex rows;
 };
 struct AdjointState;
 void adjoint_free(AdjointState* s);
