@@ -23,7 +23,12 @@ __device__ __forceinline__ void charged_step_body(ElectronArgs const& A)
     __shared__ IonPairSlot ion_slots[128];
     IonPairSlot* const my_slot = ion_slots + threadIdx.x;
     unsigned int moved = 0;
-    for_each_particle(A.n, A.work, [&](int64_t ip) {
+    // the electrons' common-history loop has handled (and counted) the rest
+    bool const resumed = !POS && A.resumed != 0;
+    int64_t const n = resumed ? static_cast<int64_t>(*A.resume_count) : A.n;
+    for_each_particle(n, A.work, [&](int64_t i) {
+        ResumeRec const* const from = resumed ? A.resume + i : nullptr;
+        int64_t const ip = from ? from->ip : i;
         if (!(A.id[ip] > 0)) {
             if (A.segments) A.segments[ip].kind = 0;
             if (A.sec_per_parent) A.sec_per_parent[ip] = 0;
@@ -35,11 +40,11 @@ __device__ __forceinline__ void charged_step_body(ElectronArgs const& A)
         Err err;
         uint64_t sub = 0, ev = 0;
         uint32_t lineage = 0;
-        ++moved;
+        if (!resumed) ++moved;
         if (A.segments) A.segments[ip].kind = 0;
         IonPairCache ion_pairs;
         ion_pairs.init(my_slot, POS ? 0.0 : 0.5 * C.cfg.low_energy_cutoff_eV, C.tix.w_air_eV_per_pair);
-        int const disp = transport_charged<NP, POS>(C, A, ip, sub, ev, lineage, ion_pairs, err);
+        int const disp = transport_charged<NP, POS>(C, A, ip, sub, ev, lineage, ion_pairs, err, from);
         ion_pairs.flush(C, A.cells);
         // Every record this particle appended carries a lineage below this
         // count, so the ordering scan/scatter stays in bounds on every path.

@@ -100,12 +100,14 @@ __device__ __forceinline__ bool strictly_inside(Geom const& g, double r2, double
     // a NaN or negative-zero-free non-negative r2 orders as its bits
     return dbits(r2) < dbits(g.r2_in) && z > g.z_in_lo && z < g.z_in_hi;
 }
-template <int NP>
+// StartInside: the caller knows it of the start (r02 is not read).
+template <int NP, bool StartInside = false>
 __device__ __forceinline__ bool clip_inside(double x0, double y0, double z0, double r02, double x1, double y1, double z1,
                                             double r12, Geom const& g, Path<NP>& p)
 {
     if constexpr (NP != 1) return false;
-    if (!strictly_inside(g, r02, z0) || !strictly_inside(g, r12, z1)) return false;
+    if (!StartInside && !strictly_inside(g, r02, z0)) return false;
+    if (!strictly_inside(g, r12, z1)) return false;
     double const dx = x1 - x0, dy = y1 - y0, dz = z1 - z0;
     double const n2 = dx * dx + dy * dy + dz * dz;
     if (!gt0(n2)) return false;
@@ -649,10 +651,15 @@ __device__ __forceinline__ FieldRange path_field_work(FieldView const& fv, Geom 
             if (!finite_bits(work) || !finite_bits(er) || !finite_bits(ez) || !finite_bits(bth)) {
                 err.set(RREA_GPU_ERR_INVALID_STATE);
             }
-            double const v[6] = {work, er * rc, er * rs, ez, -bth * rs, bth * rc};
+            double const v[4] = {work, er * rc, er * rs, ez};
 #pragma unroll
-            for (int c = 0; c < 6; ++c) acc[c] = node == 0 ? v[c] : acc[c] + v[c];
+            for (int c = 0; c < 4; ++c) acc[c] = node == 0 ? v[c] : acc[c] + v[c];
+            if (fv.has_b) {
+                acc[4] = node == 0 ? -bth * rs : acc[4] - bth * rs;
+                acc[5] = node == 0 ? bth * rc : acc[5] + bth * rc;
+            }
         }
+        if (!fv.has_b) acc[4] = acc[5] = 0.0;
         double const w = p.full * half;
         res.work += (q * w) * acc[0];
         if constexpr (NP == 1) {

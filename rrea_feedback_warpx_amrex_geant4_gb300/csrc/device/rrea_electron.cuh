@@ -286,10 +286,28 @@ __device__ __forceinline__ double sample_gs_angle_rows(StepConstants const& C, c
     RowHit hp, hu;
     bool ok = rate_bracket(C, arena, rc, e, err, species ? RREA_T_P_COLLISION : RREA_T_E_COLLISION);
     ok = ok && !(row_flags(rc.hit) >> RREA_RATE_ANGLE_ENERGY & 1u);
-    ok = ok && find_row(arena, a.p_rows, n, hp) && !row_flags(hp);
-    ok = ok && find_row(arena, a.u_rows, u, hu) && !row_flags(hu);
+    ok = ok && find_row(arena, a.p_rows, n, hp) && !row_flags(hp) && a.u_rows.span_key >= 0;
+    // below the second node the first log-log slope extends to 1e-6 of it,
+    // from the last but one on the angle is that node's: lower node and
+    // fraction of the logarithm
+    int iu = 1;
+    double fu = 0.0;
     if (ok) {
-        int const ie = row_index(rc.hit), ip = row_index(hp), iu = row_index(hu) + 1;
+        double const u1 = __ldg(arena + a.u + 1);
+        if (u <= u1) {
+            fu = flog(arena, fmax(u, u1 * 1.0e-6) * __ldg(arena + a.iu + 1)) * __ldg(arena + a.ilur + 1);
+        } else if (u >= __ldg(arena + a.u + a.nu - 2)) {
+            iu = a.nu - 2;
+        } else {
+            ok = find_row(arena, a.u_rows, u, hu) && !row_flags(hu);
+            if (ok) {
+                iu = row_index(hu) + 1;
+                fu = row_value(hu, 0);
+            }
+        }
+    }
+    if (ok) {
+        int const ie = row_index(rc.hit), ip = row_index(hp);
         double const te = row_value(rc.hit, RREA_RATE_ANGLE_ENERGY);
         double const tn = row_value(hp, 0);
         const double* l = arena + a.lomc + (static_cast<size_t>(ie) * a.np + ip) * a.nu + iu;
@@ -307,7 +325,6 @@ __device__ __forceinline__ double sample_gs_angle_rows(StepConstants const& C, c
         float const e1 = __fdividef(narrow_f32(d1 - x1), narrow_f32(x1));
         if (fabsf(e0) < 0.015625f && fabsf(e1) < 0.015625f) {
             float const corr = (e1 - e0) - 0.5f * (e1 * e1 - e0 * e0) + (1.0f / 3.0f) * (e1 * e1 * e1 - e0 * e0 * e0);
-            double const fu = row_value(hu, 0);
             double const omc = d0 * fexp(arena, fu * ((l1 - l0) + widen_f32(corr)));
             double const c = 1.0 - fmin(2.0, omc);
             return fmin(1.0, fmax(-1.0, c));
@@ -734,7 +751,8 @@ __device__ __noinline__ double cutoff_bisection(Intervals<NP> iv, Path<NP> path,
 template <int NP, bool POS = false>
 __device__ __forceinline__ int transport_charged(StepConstants const& C, ElectronArgs const& A, int64_t ip,
                                                  uint64_t& subcycles_out, uint64_t& events_out,
-                                                 uint32_t& lineage, IonPairCache& ion_pairs, Err& err)
+                                                 uint32_t& lineage, IonPairCache& ion_pairs, Err& err,
+                                                 ResumeRec const* from = nullptr)
 {
     constexpr double q = POS ? 1.0 : -1.0;
     constexpr int species = POS ? 1 : 0;
@@ -892,7 +910,10 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
     // ---- substep count, O/RreaElectronTransport.cpp:187-279
     uint64_t subcycles;
     RateCache rc;
-    {
+    bool const resume = !POS && from && from->sub != kResumeFromStart;
+    if (resume) {
+        subcycles = from->subcycles;
+    } else {
         double s0, s1, s2 = 0.0;
         if constexpr (POS) competing_rates_positron(C, arena, rc, k, s0, s1, s2, err);
         else competing_rates(C, arena, rc, k, s0, s1, err);
@@ -1092,8 +1113,24 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
         return false;
     };
 
+    uint64_t first = 0;
+    if (resume) {
+        // the state the common-history loop reached, one hazard draw per substep
+        first = from->sub;
+        completed = first;
+        events = first;
+        run_x = from->x;
+        run_y = from->y;
+        run_z = from->z;
+        dx = from->dx;
+        dy = from->dy;
+        dz = from->dz;
+        k = from->k;
+        transported_dpath = from->dpath;
+        transported_len = from->length;
+    }
     // ---- substep interleave, O/RreaChargedInterleave.H:693-732
-    for (uint64_t sub = 0; sub < subcycles; ++sub) {
+    for (uint64_t sub = first; sub < subcycles; ++sub) {
         if (k < cutoff) break;
         double sb, se;
         {

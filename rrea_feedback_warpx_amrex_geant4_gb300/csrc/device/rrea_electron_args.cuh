@@ -30,6 +30,17 @@ struct NetGrid {
     double* jz;
 };
 
+// An electron the common-history loop (rrea_charged_lean.cuh) left to the
+// full one: its state at the start of substep `sub` of `subcycles`, and the
+// transported path so far.  sub = kResumeFromStart: nothing was done.
+constexpr uint32_t kResumeFromStart = 0xffffffffu;
+struct ResumeRec {
+    double x, y, z, dx, dy, dz, k;
+    double dpath, length;
+    int64_t ip;
+    uint32_t sub, subcycles;
+};
+
 struct ElectronArgs {
     int64_t n;
     // The current and prev_* arrays may alias (resident engine mode, where
@@ -84,6 +95,11 @@ struct ElectronArgs {
     // optional scheduling order of the tile indices (null: the end of the
     // tile first); it changes which thread visits a particle, never a result
     const uint32_t* __restrict__ order;
+    // records of the common-history loop (capacity n) and their count; the
+    // full kernel with resumed != 0 runs over the records instead of the tile
+    ResumeRec* __restrict__ resume;
+    unsigned long long* __restrict__ resume_count;
+    int32_t resumed;
     // plane-crossing diagnostic of the electrons' continuous segments:
     // n_planes strictly increasing plane z and kPlaneValues accumulators per
     // plane (n_planes = 0: off)

@@ -33,6 +33,16 @@ constexpr int kSpecies = 3;
 // Chunks of a drop-in phase call whose upload overlaps the compute of the
 // chunks before it, and the tile size from which that pays.
 constexpr int kPhaseChunks = 4;
+// Electron tiles from here on run the common-history loop first.  Its
+// records' launch adds the latency of a full loop at low occupancy, which a
+// small tile does not earn back.  Measured (full loop alone / with the common
+// loop): scale-up electrons 3e4 0.43 / 0.54 ms, 6e4 0.74 / 0.71, 1e5 1.09 /
+// 0.96, 3e5 2.64 / 1.88; the plain case's slower ones 6e4 1.06 / 1.16, 1e5
+// 1.27 / 1.30, 1.5e5 1.63 / 1.58, 3e5 2.78 / 2.33.
+#ifndef RREA_LEAN_MIN_PARTICLES
+#define RREA_LEAN_MIN_PARTICLES (3 << 15)
+#endif
+constexpr int64_t kLeanMinParticles = RREA_LEAN_MIN_PARTICLES;
 #ifndef RREA_PIPELINE_MIN_PARTICLES
 #define RREA_PIPELINE_MIN_PARTICLES (1LL << 18)
 #endif
@@ -179,7 +189,10 @@ struct rrea_gpu_ctx {
     int* d_status = nullptr;
     long long* d_fail_index = nullptr;
     unsigned long long* d_transported = nullptr;
-    unsigned long long* d_work = nullptr;  // dynamic scheduling counters of the phase kernels, one per chunk
+    // per chunk: dynamic scheduling counters of the phase kernel, of the full
+    // kernel over the common-history loop's records, and the records' count
+    unsigned long long* d_work = nullptr;
+    rrea_dev::ResumeRec* d_resume = nullptr;  // those records, one slot per tile slot
     // a drop-in phase call uploads its host tile in chunks on side[0] while
     // the kernels of earlier chunks run on `stream` and side[1]
     cudaEvent_t chunk_up[kPhaseChunks] = {};
@@ -418,7 +431,8 @@ rrea_gpu_status rrea_gpu_create(const rrea_gpu_config* cfg, int64_t capacity, rr
         && dalloc(&ctx->d_alive, n) == cudaSuccess && dalloc(&ctx->d_child_lineage, nsec) == cudaSuccess
         && dalloc(&ctx->d_cost_scratch,
                   static_cast<size_t>(kPhaseChunks) * rrea_launch::cost_order_scratch_elems()) == cudaSuccess
-        && dalloc(&ctx->d_invalid, 1) == cudaSuccess && dalloc(&ctx->d_work, kPhaseChunks) == cudaSuccess
+        && dalloc(&ctx->d_invalid, 1) == cudaSuccess && dalloc(&ctx->d_work, 3 * kPhaseChunks) == cudaSuccess
+        && dalloc(&ctx->d_resume, n) == cudaSuccess
         && cudaEventCreate(&ctx->ev_start) == cudaSuccess && cudaEventCreate(&ctx->ev_stop) == cudaSuccess;
     if (!ok) return bail(RREA_GPU_ERR_CUDA);
     if (cudaMemsetAsync(ctx->d_cells, 0, 5 * ncell * sizeof(double), ctx->stream) != cudaSuccess) {
@@ -493,6 +507,7 @@ rrea_gpu_status rrea_gpu_destroy(rrea_gpu_ctx* ctx)
     dfree(ctx->d_roots);
     if (ctx->h_roots) cudaFreeHost(ctx->h_roots);
     dfree(ctx->d_work);
+    dfree(ctx->d_resume);
     if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
     if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -913,8 +928,9 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         int const fit = warps_per_sm <= 8 ? 2 : warps_per_sm <= 16 ? 4 : warps_per_sm <= 32 ? 8 : 16;
         if (fit < min_blocks) min_blocks = fit;
     }
+    bool const lean = species == RREA_SPECIES_ELECTRON && c.periodic_z == 0 && a.n_planes == 0 && a.n >= kLeanMinParticles;
 #ifndef RREA_STATIC_SCHEDULE
-    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long) * chunks, ctx->stream));
+    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long) * 3 * kPhaseChunks, ctx->stream));
 #endif
     RREA_CUDA(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
     if (host && chunks == 1) {
@@ -983,6 +999,16 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         } else if (species == RREA_SPECIES_POSITRON) {
             RREA_CUDA(ctx, rrea_launch::positron_step(b, blocks > 0 ? blocks : 1, ctx->launch_threads, min_blocks,
                                                       c.periodic_z != 0, cs));
+        } else if (lean) {
+            b.resume = ctx->d_resume + off;
+            b.resume_count = ctx->d_work + 2 * kPhaseChunks + k;
+            RREA_CUDA(ctx, rrea_launch::electron_lean(b, blocks > 0 ? blocks : 1, ctx->launch_threads, ctx->launch_min_blocks, cs));
+            // the rest: about one electron in twenty, so the variant with
+            // registers for a quarter of the SM's threads
+            b.resumed = 1;
+            b.order = nullptr;
+            b.work = ctx->d_work + kPhaseChunks + k;
+            RREA_CUDA(ctx, rrea_launch::electron_step(b, ctx->num_sms * 8, 128, 8, false, cs));
         } else {
             RREA_CUDA(ctx, rrea_launch::electron_step(b, blocks > 0 ? blocks : 1, ctx->launch_threads, min_blocks,
                                                       c.periodic_z != 0, cs));

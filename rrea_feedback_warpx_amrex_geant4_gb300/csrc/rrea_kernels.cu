@@ -4,6 +4,8 @@
 //                         averages), once per step
 //   electron_step_kernel  one thread per electron, full outer step (the
 //                         positron kernel lives in rrea_positron_kernels.cu)
+//   electron_lean_kernel  the same for the electrons of common history; the
+//                         rest is recorded for electron_step_kernel
 //   scan / scatter        orders the appended secondaries into the reference's
 //                         deterministic order (parent index, then lineage)
 #include "rrea_kernels.h"
@@ -11,6 +13,7 @@
 #include <atomic>
 
 #include "device/rrea_charged_kernel.cuh"
+#include "device/rrea_charged_lean.cuh"
 
 #include <cuda_runtime.h>
 
@@ -188,6 +191,18 @@ cudaError_t electron_step(rrea_dev::ElectronArgs const& args, int blocks, int th
     case 12: rrea_dev::electron_step_kernel<12, 1><<<blocks, threads, 0, stream>>>(args); break;
     case 16: rrea_dev::electron_step_kernel<16, 1><<<blocks, threads, 0, stream>>>(args); break;
     default: rrea_dev::electron_step_kernel<2, 1><<<blocks, threads, 0, stream>>>(args); break;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t electron_lean(rrea_dev::ElectronArgs const& args, int blocks, int threads, int min_blocks,
+                          cudaStream_t stream)
+{
+    note_launch();
+    switch (min_blocks) {
+    case 8: rrea_dev::electron_lean_kernel<8><<<blocks, threads, 0, stream>>>(args); break;
+    case 12: rrea_dev::electron_lean_kernel<12><<<blocks, threads, 0, stream>>>(args); break;
+    default: rrea_dev::electron_lean_kernel<16><<<blocks, threads, 0, stream>>>(args); break;
     }
     return cudaGetLastError();
 }

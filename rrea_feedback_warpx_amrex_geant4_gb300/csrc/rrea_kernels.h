@@ -35,6 +35,12 @@ cudaError_t field_prep(int nr, int nz, const double* er, const double* ez, const
                        double* cell_er, double* cell_ez, cudaStream_t stream);
 cudaError_t electron_step(rrea_dev::ElectronArgs const& args, int blocks, int threads, int min_blocks, bool periodic,
                           cudaStream_t stream);
+// The electrons' common-history loop over an absorbing domain without planes
+// (device/rrea_charged_lean.cuh): finishes most of the tile and records the
+// rest in args.resume / resume_count (zeroed by the caller); electron_step
+// with args.resumed then runs over the records.
+cudaError_t electron_lean(rrea_dev::ElectronArgs const& args, int blocks, int threads, int min_blocks,
+                          cudaStream_t stream);
 // Positron phase (rrea_positron_kernels.cu): its own constant bank, set
 // once per phase before its launches; min_blocks picks the register variant
 // as for electrons (2, 4, 8 or 16 resident 128-thread blocks per SM).
