@@ -34,19 +34,6 @@ public:
     double const* at(int64_t offset) const { return m_arena.data() + offset; }
 
 private:
-    // One column of interval-polynomial rows: a table on nodes x (n of them).
-    struct RowColumn {
-        enum Kind { Table, InverseSemilog, LogFraction } kind = Table;
-        int mode = 0;                // RreaInterpMode of a Table
-        const double* x = nullptr;
-        const double* y = nullptr;   // values (LogFraction: none)
-        int n = 0;
-        bool index = false;          // its lower node index goes into the rows' meta
-    };
-    // Taylor coefficients of the column about xc on a row (lo, hi]; false
-    // when the truncated polynomial is not the interpolant to within an ulp.
-    static bool row_polynomial(RowColumn const& col, double lo, double hi, double xc, double c[7], int& lower);
-    void push_rows(RreaRowIndex& ix, double x_min, double x_max, std::vector<std::vector<RowColumn>> const& columns);
     void LoadRows();
     void LoadPairBank(std::string const& bin_path, std::string const& index_path);
     int64_t push(std::vector<double> const& values);

@@ -16,6 +16,7 @@
 // Measured on 512 x 4096: ten updates of two substeps with the upload and
 // download of the vectors and the particle diagnostics 16.0 -> 6.6 ms.
 #include "rrea_kernels.h"
+#include "device/rrea_exact_quot.cuh"
 
 #include <cuda_runtime.h>
 
@@ -33,22 +34,6 @@ __device__ __forceinline__ size_t er_at(int nr, int i, int j)
 __device__ __forceinline__ size_t ez_at(int nr, int i, int j)
 {
     return static_cast<size_t>(i) + static_cast<size_t>(nr) * j;
-}
-
-// Divisor of a quotient that must round as a / b does: y = RN(1 / b).
-struct ExactDivisor {
-    double b, y;
-};
-
-// RN(a / b) from y = RN(1 / b): the quotient estimate RN(a y) is within two
-// ulps, its residual a - q b is exact in one fused multiply-add, and adding
-// residual * y rounds to the nearest (Markstein, IBM J. Res. Dev. 34, 1990).
-// An overflowed or NaN estimate has no residual and is returned as it is.
-__device__ __forceinline__ double exact_quot(double a, ExactDivisor const& d)
-{
-    double const q = a * d.y;
-    double const r = fma(-q, d.b, a);
-    return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : fma(r, d.y, q);
 }
 
 // dBtheta/dt = dEz/dr - dEr/dz at the interior corners, over dt_a and (when
@@ -102,7 +87,7 @@ __global__ void __launch_bounds__(256) advance_e_kernel(int nr, int nz, double d
     if (j0 >= j1) return;
     double const fi = i, fi1 = i + 1;
     double const radius = (fi + 0.5) * dr;
-    ExactDivisor const rad{radius, 1.0 / radius};
+    ExactDivisor const rad = exact_divisor(radius);
     double here = bt[er_at(nr, i, j0)];
     for (int j = j0; j < j1; ++j) {
         double const above = j < nz ? bt[er_at(nr, i, j + 1)] : 0.0;
@@ -149,8 +134,8 @@ cudaError_t maxwell_advance_b(int nr, int nz, double dr, double dz, double dt_a,
     using namespace rrea_dev;
     note_launch();
     int const rows = rows_for(nr, nz, kFieldThreads);
-    advance_b_kernel<<<grid_for(nr, nz, rows), dim3(32, 8), 0, stream>>>(nr, nz, ExactDivisor{dr, 1.0 / dr},
-                                                                         ExactDivisor{dz, 1.0 / dz}, dt_a, dt_b, twice,
+    advance_b_kernel<<<grid_for(nr, nz, rows), dim3(32, 8), 0, stream>>>(nr, nz, exact_divisor(dr),
+                                                                         exact_divisor(dz), dt_a, dt_b, twice,
                                                                          open_faces, rows, er, ez, bt);
     return cudaGetLastError();
 }
@@ -161,7 +146,7 @@ cudaError_t maxwell_advance_e(int nr, int nz, double dr, double dz, double dt, c
     using namespace rrea_dev;
     note_launch();
     int const rows = rows_for(nr, nz, kFieldThreads);
-    advance_e_kernel<<<grid_for(nr, nz, rows), dim3(32, 8), 0, stream>>>(nr, nz, dr, ExactDivisor{dz, 1.0 / dz},
+    advance_e_kernel<<<grid_for(nr, nz, rows), dim3(32, 8), 0, stream>>>(nr, nz, dr, exact_divisor(dz),
                                                                          dt / (kEps0 * kMu0), dt / kEps0, rows, bt, jr,
                                                                          jz, er, ez);
     return cudaGetLastError();

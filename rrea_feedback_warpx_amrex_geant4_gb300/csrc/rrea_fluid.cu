@@ -12,6 +12,9 @@
 // that sizes the substeps).  This file is compiled without FMA contraction
 // so that every product and sum rounds as in the reference's host build.
 #include "rrea_kernels.h"
+#include "device/rrea_exact_quot.cuh"
+#include "device/rrea_fastmath.cuh"
+#include "host/interval_rows.hpp"
 
 #include <cuda_runtime.h>
 
@@ -73,6 +76,9 @@ __device__ __forceinline__ double warp_sum(double v)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
+// 1 - 2^-50: a quotient a / b exceeds w only if a >= w b (1 - 2^-50), whatever
+// the roundings of either side, so maxima of quotients divide only then
+constexpr double kBelowOne = 1.0 - 8.8817841970012523e-16;
 __device__ __forceinline__ bool lane0() { return (threadIdx.x & 31) == 0; }
 // One atomic per warp; every lane of the warp must call these (the kernels
 // below run whole warps through their grid-stride loops and reduce after).
@@ -147,6 +153,18 @@ struct Grid {
     }
 };
 
+// Column launches: 32 x 8 threads, a thread owns one column i over rows
+// strided by the grid, so what depends on r alone (volumes, areas, their
+// reciprocals) is formed once per thread; a block's warps are its rows.
+// The kernels are bound by the FP64 pipe (an operation holds it 64 cycles a
+// warp, a division or a root ten operations), so the divisions count: on
+// 256 x 2048 cells, with exact_quot and the closure's rows, closure 235 to
+// 96 us, face flux 240 to 126, react 137 to 112, update 197 to 128; the
+// coupled step 2.78 to 1.94 ms.
+__device__ __forceinline__ int column() { return blockIdx.x * 32 + threadIdx.x; }
+__device__ __forceinline__ int first_row() { return blockIdx.y * 8 + threadIdx.y; }
+__device__ __forceinline__ int row_stride() { return gridDim.y * 8; }
+
 struct ReactParams {
     int64_t n;
     double dt;
@@ -173,8 +191,26 @@ __global__ void react_kernel(ReactParams p, double* __restrict__ ne, double* __r
         if (p.table) {
             nu = nu_cell[k];
             double const x = nu * p.dt;
-            decay = exp(-x);
-            factor = nu > 0.0 ? -expm1(-x) / nu : p.dt;
+            if (x >= 0.0 && x < 0.0625) {
+                // factor = dt (1 - e^-x) / x by its series (the next term is
+                // below 2^-57) and e^-x = 1 - x (1 - e^-x) / x: 13 FP64 slots
+                // for an exponential, an expm1 and a division (58)
+                double f = 1.0 / 3628800.0;
+                f = fma(-x, f, 1.0 / 362880.0);
+                f = fma(-x, f, 1.0 / 40320.0);
+                f = fma(-x, f, 1.0 / 5040.0);
+                f = fma(-x, f, 1.0 / 720.0);
+                f = fma(-x, f, 1.0 / 120.0);
+                f = fma(-x, f, 1.0 / 24.0);
+                f = fma(-x, f, 1.0 / 6.0);
+                f = fma(-x, f, 0.5);
+                f = fma(-x, f, 1.0);
+                decay = fma(-x, f, 1.0);
+                factor = nu > 0.0 ? f * p.dt : p.dt;
+            } else {
+                decay = exp(-x);
+                factor = nu > 0.0 ? -expm1(-x) / nu : p.dt;
+            }
         }
         double const e0 = dmax(ne[k], 0.0);
         double const p0 = dmax(np[k], 0.0);
@@ -217,9 +253,13 @@ __global__ void react_kernel(ReactParams p, double* __restrict__ ne, double* __r
         }
         double const actual = kQe * (q - m - e);
         double const scale = dmax(fabs(expected) + kQe * (fabs(q) + fabs(m) + fabs(e)), kDblMin);
-        double const r = fabs(actual - expected) / scale;
-        if (isnan(r)) nan = 1;
-        else if (bits(r) > worst) worst = bits(r);
+        // only a residual that can exceed the worst so far is divided out
+        double const diff = fabs(actual - expected);
+        if (!(diff < __longlong_as_double(static_cast<long long>(worst)) * scale * kBelowOne)) {
+            double const r = diff / scale;
+            if (isnan(r)) nan = 1;
+            else if (bits(r) > worst) worst = bits(r);
+        }
     }
     post_max(words + w_residual, worst);
     if (w_rate >= 0) post_max(words + w_rate, rate_max);
@@ -280,14 +320,15 @@ __global__ void normalize_sources_kernel(Grid g, double dt, const double* __rest
                                          double* __restrict__ se, double* __restrict__ sp, double* __restrict__ sn)
 {
     int64_t const n = static_cast<int64_t>(g.nr) * g.nz;
-    int64_t const stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n; k += stride) {
-        int const i = static_cast<int>(k % g.nr);
-        double const r_in = g.r_lo + static_cast<double>(i) * g.dr;
-        double const denom = shell_volume(r_in, r_in + g.dr, g.dz) * dt;
-        se[k] = denom > 0.0 ? cells[k] / denom : 0.0;
-        sp[k] = denom > 0.0 ? cells[n + k] / denom : 0.0;
-        sn[k] = denom > 0.0 ? cells[2 * n + k] / denom : 0.0;
+    int const i = column();
+    double const r_in = g.r_lo + static_cast<double>(i) * g.dr;
+    double const denom = shell_volume(r_in, r_in + g.dr, g.dz) * dt;
+    ExactDivisor const d = exact_divisor(denom);
+    for (int j = first_row(); j < g.nz && i < g.nr; j += row_stride()) {
+        int64_t const k = i + static_cast<int64_t>(g.nr) * j;
+        se[k] = denom > 0.0 ? exact_quot(cells[k], d) : 0.0;
+        sp[k] = denom > 0.0 ? exact_quot(cells[n + k], d) : 0.0;
+        sn[k] = denom > 0.0 ? exact_quot(cells[2 * n + k], d) : 0.0;
     }
 }
 
@@ -295,34 +336,16 @@ __global__ void normalize_sources_kernel(Grid g, double dt, const double* __rest
 struct Closure {
     int n;
     const double *en, *log_en, *k0, *log_k0, *nu2, *nu3, *log_nu3, *dl, *log_dl, *dt, *log_dt;
+    // the five coefficients between the nodes as interval polynomials
+    // (device/rrea_rate_rows.cuh), offsets into `arena`
+    const double* arena;
+    RreaRowIndex rows;
 };
 
-// LowEnergyElectronClosure::Evaluate (S/RreaInteractionTables.cpp:3406-3478);
-// status 0 in range, 1 held below, 2 above range, 3 invalid.
-__device__ void closure_eval(Closure const& t, double en, int& status, double out[5])
+// The interpolation between two nodes as the reference forms it, where a row
+// is flagged.
+__device__ __noinline__ void closure_between(Closure const& t, double en, double out[5])
 {
-    out[0] = out[1] = out[2] = out[3] = out[4] = 0.0;
-    if (t.n == 0 || !isfinite(en) || en < 0.0) {
-        status = 3;
-        return;
-    }
-    int node = t.n;
-    if (en <= t.en[0]) {
-        status = en < t.en[0] ? 1 : 0;
-        node = 0;
-    } else if (en >= t.en[t.n - 1]) {
-        status = en > t.en[t.n - 1] ? 2 : 0;
-        node = t.n - 1;
-    }
-    if (node < t.n) {
-        out[0] = t.k0[node];
-        out[1] = t.nu2[node];
-        out[2] = t.nu3[node];
-        out[3] = t.dl[node];
-        out[4] = t.dt[node];
-        return;
-    }
-    status = 0;
     int lo = 0, hi = t.n;   // first node above en (upper_bound)
     while (lo < hi) {
         int const mid = (lo + hi) >> 1;
@@ -348,6 +371,44 @@ __device__ void closure_eval(Closure const& t, double en, int& status, double ou
     out[4] = exp(t.log_dt[lo] + f * (t.log_dt[hi] - t.log_dt[lo]));
 }
 
+// LowEnergyElectronClosure::Evaluate (S/RreaInteractionTables.cpp:3406-3478);
+// status 0 in range, 1 held below, 2 above range, 3 invalid.  Between nodes
+// the values are interval polynomials: 22 FP64 slots for two logarithms and
+// five exponentials (about 200).
+__device__ __forceinline__ void closure_eval(Closure const& t, double en, int& status, double out[5])
+{
+    out[0] = out[1] = out[2] = out[3] = out[4] = 0.0;
+    if (t.n == 0 || !isfinite(en) || en < 0.0) {
+        status = 3;
+        return;
+    }
+    int node = t.n;
+    if (en <= t.en[0]) {
+        status = en < t.en[0] ? 1 : 0;
+        node = 0;
+    } else if (en >= t.en[t.n - 1]) {
+        status = en > t.en[t.n - 1] ? 2 : 0;
+        node = t.n - 1;
+    }
+    if (node < t.n) {
+        out[0] = t.k0[node];
+        out[1] = t.nu2[node];
+        out[2] = t.nu3[node];
+        out[3] = t.dl[node];
+        out[4] = t.dt[node];
+        return;
+    }
+    status = 0;
+    RowHit h;
+    if (find_row(t.arena, t.rows, en, h) && !row_flags(h)) {
+#pragma unroll
+        for (int c = 0; c < 5; ++c) out[c] = row_value(h, c);
+        out[1] = dmax(out[1], 0.0);   // nu2 may be linear from a zero node
+        return;
+    }
+    closure_between(t, en, out);
+}
+
 // BuildElectronClosureCellFields (S/LowEnergyFluidFaceTransport.cpp:1034-1243)
 __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const double* __restrict__ chi,
                                const double* __restrict__ er, const double* __restrict__ ez,
@@ -359,8 +420,12 @@ __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const doubl
     int64_t const n = static_cast<int64_t>(g.nr) * g.nz;
     u64 held = 0, above = 0, invalid = 0, min_en = ~0ULL, max_en = 0;
     double count = 0.0, held_count = 0.0, source = 0.0;
-    int64_t const stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n; k += stride) {
+    int const i = column();
+    double const r_in = g.r_lo + static_cast<double>(i) * g.dr;
+    double const volume = shell_volume(r_in, r_in + g.dr, g.dz);
+    ExactDivisor by_x = exact_divisor(scalar_chi), by_xn = exact_divisor(scalar_chi * kNL);
+    for (int j = first_row(); j < g.nz && i < g.nr; j += row_stride()) {
+        int64_t const k = i + static_cast<int64_t>(g.nr) * j;
         if (mu) mu[k] = 0.0;
         if (nu) nu[k] = 0.0;
         if (d3) {
@@ -369,14 +434,24 @@ __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const doubl
             d3[2 * n + k] = 0.0;
         }
         double const x = chi ? chi[k] : scalar_chi;
-        double const e_mag = hypot(er[k], ez[k]);
+        if (chi) {
+            by_x = exact_divisor(x);
+            by_xn = exact_divisor(x * kNL);
+        }
+        // |E| and 1/|E| from one inverse root, |E| corrected by its residual
+        // (to half an ulp as hypot is; |E|^2 is far from overflow)
+        double const e_r = er[k], e_z = ez[k];
+        double const e2 = fma(e_r, e_r, e_z * e_z);
+        double const inv_e = e2 > 0.0 ? frsqrt(e2) : 0.0;
+        double e_mag = e2 * inv_e;
+        e_mag = fma(0.5 * inv_e, fma(-e_mag, e_mag, e2), e_mag);
         double const ev = ne ? ne[k] : 0.0;
         double const sv = src ? src[k] : 0.0;
         if (!isfinite(x) || !(x > 0.0) || !isfinite(e_mag) || !isfinite(ev) || !isfinite(sv)) {
             ++invalid;
             continue;
         }
-        double const en = e_mag * 1.0e21 / (x * kNL);
+        double const en = exact_quot(e_mag * 1.0e21, by_xn);
         int status = 3;
         double co[5];
         closure_eval(t, en, status, co);
@@ -388,22 +463,15 @@ __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const doubl
         }
         min_en = bits(en) < min_en ? bits(en) : min_en;
         max_en = bits(en) > max_en ? bits(en) : max_en;
-        int const i = static_cast<int>(k % g.nr);
-        double const r_in = g.r_lo + static_cast<double>(i) * g.dr;
-        double const volume = shell_volume(r_in, r_in + g.dr, g.dz);
         double const c = dmax(ev, 0.0) * volume;
         count += c;
         source += dmax(sv, 0.0) * volume;
         if (status == 1) held_count += c;
-        if (mu) mu[k] = co[0] / x;
+        if (mu) mu[k] = exact_quot(co[0], by_x);
         if (nu) nu[k] = co[1] * x + co[2] * x * x;
         if (d3) {
-            double const dl = co[3] / x, dt = co[4] / x;
-            double br = 0.0, bz = 0.0;
-            if (e_mag > 0.0) {
-                br = er[k] / e_mag;
-                bz = ez[k] / e_mag;
-            }
+            double const dl = exact_quot(co[3], by_x), dt = exact_quot(co[4], by_x);
+            double const br = e_r * inv_e, bz = e_z * inv_e;
             double const an = dl - dt;
             d3[k] = dt + an * br * br;
             d3[n + k] = an * br * bz;
@@ -443,11 +511,26 @@ __global__ void tensor_check_kernel(int64_t n, const double* __restrict__ d3, u6
             bad = 1;
             continue;
         }
-        double const e = 0.5 * (rr + zz + hypot(rr - zz, 2.0 * rz));
+        double const a = rr - zz, b = 2.0 * rz;
+        double const e = 0.5 * (rr + zz + fsqrt(fma(a, a, b * b)));
         eig = bits(e) > eig ? bits(e) : eig;
     }
     post_max(words + w_eig, eig);
     if (__any_sync(0xffffffffu, bad) && lane0()) atomicOr(words + w_bad, 1ULL);
+}
+
+// t = i + width j, with a 32-bit division while the index fits one (the
+// 64-bit one costs four times the instructions)
+__device__ __forceinline__ void split_index(int64_t t, int width, int& i, int& j)
+{
+    if (t < (int64_t{1} << 32)) {
+        uint32_t const q = static_cast<uint32_t>(t) / static_cast<uint32_t>(width);
+        j = static_cast<int>(q);
+        i = static_cast<int>(static_cast<uint32_t>(t) - q * static_cast<uint32_t>(width));
+    } else {
+        j = static_cast<int>(t / width);
+        i = static_cast<int>(t % width);
+    }
 }
 
 struct TransportParams {
@@ -458,6 +541,7 @@ struct TransportParams {
     double scalar_chi;
     double dt;
     double limiter_cfl;
+    ExactDivisor dr, dz, dr2, dz2;   // cell sizes and their doubles
 };
 
 // The frozen carrier density of one cell as the flux law reads it: vacuum
@@ -499,13 +583,11 @@ __global__ void face_flux_kernel(TransportParams p, const double* __restrict__ o
         double e_face;
         if (dir == 0) {
             f = t;
-            i = static_cast<int>(t % (nr + 1));
-            j = static_cast<int>(t / (nr + 1));
+            split_index(t, nr + 1, i, j);
             e_face = efr_add ? efr[f] + efr_add[f] : efr[f];
         } else {
             f = t - nfr;
-            i = static_cast<int>(f % nr);
-            j = static_cast<int>(f / nr);
+            split_index(f, nr, i, j);
             int64_t const fe = (per && j == nz) ? static_cast<int64_t>(i) : f;
             e_face = efz_add ? efz[fe] + efz_add[fe] : efz[fe];
             if (per && j == nz) j = 0;
@@ -562,11 +644,11 @@ __global__ void face_flux_kernel(TransportParams p, const double* __restrict__ o
                     if (i > 0 && i <= nr - 1) {
                         double const d_rr = 0.5 * (tensor(i - 1, j, 0) + tensor(i, j, 0));
                         double const d_rz = 0.5 * (tensor(i - 1, j, 1) + tensor(i, j, 1));
-                        double const grad_r = (n_hi - n_lo) / g.dr;
+                        double const grad_r = exact_quot(n_hi - n_lo, p.dr);
                         auto axial = [&](int ii, int jj) {
-                            if (!per && jj <= 0) return (cd(ii, jj + 1) - cd(ii, jj)) / g.dz;
-                            if (!per && jj >= nz - 1) return (cd(ii, jj) - cd(ii, jj - 1)) / g.dz;
-                            return (cd(ii, jj + 1) - cd(ii, jj - 1)) / (2.0 * g.dz);
+                            if (!per && jj <= 0) return exact_quot(cd(ii, jj + 1) - cd(ii, jj), p.dz);
+                            if (!per && jj >= nz - 1) return exact_quot(cd(ii, jj) - cd(ii, jj - 1), p.dz);
+                            return exact_quot(cd(ii, jj + 1) - cd(ii, jj - 1), p.dz2);
                         };
                         double const grad_z = 0.5 * (axial(i - 1, j) + axial(i, j));
                         diffusive = -(d_rr * grad_r + d_rz * grad_z);
@@ -579,12 +661,12 @@ __global__ void face_flux_kernel(TransportParams p, const double* __restrict__ o
                         double const d_zz = 0.5 * (tensor(i, j - 1, 2) + tensor(i, j, 2));
                         auto radial = [&](int ii, int jj) {
                             if (nr - 1 == 0) return 0.0;
-                            if (ii <= 0) return (cd(ii + 1, jj) - cd(ii, jj)) / g.dr;
-                            if (ii >= nr - 1) return (cd(ii, jj) - cd(ii - 1, jj)) / g.dr;
-                            return (cd(ii + 1, jj) - cd(ii - 1, jj)) / (2.0 * g.dr);
+                            if (ii <= 0) return exact_quot(cd(ii + 1, jj) - cd(ii, jj), p.dr);
+                            if (ii >= nr - 1) return exact_quot(cd(ii, jj) - cd(ii - 1, jj), p.dr);
+                            return exact_quot(cd(ii + 1, jj) - cd(ii - 1, jj), p.dr2);
                         };
                         double const grad_r = 0.5 * (radial(i, j - 1) + radial(i, j));
-                        double const grad_z = (n_hi - n_lo) / g.dz;
+                        double const grad_z = exact_quot(n_hi - n_lo, p.dz);
                         diffusive = -(d_rz * grad_r + d_zz * grad_z);
                     } else if (j <= 0) {
                         diffusive = -2.0 * tensor(i, 0, 2) * n_hi / g.dz;
@@ -653,11 +735,10 @@ __global__ void limiter_kernel(TransportParams p, const double* __restrict__ old
     int64_t const nfz = static_cast<int64_t>(g.nr) * (g.nz + 1);
     u64 unlimited = 0, min_scale = bits(1.0);
     double before = 0.0, removed = 0.0, e_number = 0.0, e_limited = 0.0;
-    int64_t const stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < nc; k += stride) {
-        int const i = static_cast<int>(k % g.nr);
-        int const j = static_cast<int>(k / g.nr);
-        Metric const m = metric(g, i);
+    int const i = column();
+    Metric const m = metric(g, i);
+    for (int j = first_row(); j < g.nz && i < g.nr; j += row_stride()) {
+        int64_t const k = i + static_cast<int64_t>(g.nr) * j;
         for (int s = 0; s < 3; ++s) {
             if (!p.enabled[s]) {
                 scale3[s * nc + k] = 1.0;
@@ -665,10 +746,19 @@ __global__ void limiter_kernel(TransportParams p, const double* __restrict__ old
             }
             double const density = dmax(old3[s * nc + k], 0.0);
             double const out = outgoing(fr, fz, nfr, nfz, g.nr, s, i, j, m);
-            double const rate = density > 0.0 ? out / (density * dmax(m.volume, 1.0e-300)) : (out > 0.0 ? 1.0e300 : 0.0);
-            unlimited = bits(rate) > unlimited ? bits(rate) : unlimited;
+            // divided out only where it can exceed the largest so far
+            double const held = density * dmax(m.volume, 1.0e-300);
+            if (!(density > 0.0 && out < __longlong_as_double(static_cast<long long>(unlimited)) * held * kBelowOne)) {
+                double const rate = density > 0.0 ? out / held : (out > 0.0 ? 1.0e300 : 0.0);
+                unlimited = bits(rate) > unlimited ? bits(rate) : unlimited;
+            }
             double limiter = 1.0;
-            if (out > 0.0) limiter = density > 0.0 ? dmin(1.0, p.limiter_cfl * density * m.volume / (p.dt * out)) : 0.0;
+            if (out > 0.0) {
+                // the quotient is at least 1 where its numerator is at least
+                // its denominator
+                double const keep = p.limiter_cfl * density * m.volume, leave = p.dt * out;
+                limiter = density > 0.0 ? (keep >= leave ? 1.0 : dmin(1.0, keep / leave)) : 0.0;
+            }
             scale3[s * nc + k] = limiter;
             min_scale = bits(limiter) < min_scale ? bits(limiter) : min_scale;
             before += out;
@@ -706,8 +796,8 @@ __global__ void scale_faces_kernel(TransportParams p, const double* __restrict__
     for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < nfr + nfz; t += stride) {
         double v[3];
         if (t < nfr) {
-            int const i = static_cast<int>(t % (nr + 1));
-            int const j = static_cast<int>(t / (nr + 1));
+            int i, j;
+            split_index(t, nr + 1, i, j);
             for (int s = 0; s < 3; ++s) {
                 double x = fr[s * nfr + t];
                 if (x != 0.0) {
@@ -726,8 +816,8 @@ __global__ void scale_faces_kernel(TransportParams p, const double* __restrict__
             }
         } else {
             int64_t const f = t - nfr;
-            int const i = static_cast<int>(f % nr);
-            int const j = static_cast<int>(f / nr);
+            int i, j;
+            split_index(f, nr, i, j);
             for (int s = 0; s < 3; ++s) {
                 double x = fz[s * nfz + f];
                 if (x != 0.0) {
@@ -766,11 +856,11 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
     u64 rate_max = 0, speed_max = 0, min_density = ordered(0.0);
     int nonfinite = 0;
     double cs[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int64_t const stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < nc; k += stride) {
-        int const i = static_cast<int>(k % nr);
-        int const j = static_cast<int>(k / nr);
-        Metric const m = metric(g, i);
+    int const i = column();
+    Metric const m = metric(g, i);
+    ExactDivisor const volume = exact_divisor(dmax(m.volume, 1.0e-300));
+    for (int j = first_row(); j < g.nz && i < nr; j += row_stride()) {
+        int64_t const k = i + static_cast<int64_t>(nr) * j;
         int64_t const frl = i + static_cast<int64_t>(nr + 1) * j;
         int64_t const fzl = i + static_cast<int64_t>(nr) * j;
         double fl_r[3], fh_r[3], fl_z[3], fh_z[3];
@@ -788,11 +878,16 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
                 double out = dmax(fh_r[s], 0.0) * m.a_hi + dmax(-fl_r[s], 0.0) * m.a_lo;
                 out += (dmax(fh_z[s], 0.0) + dmax(-fl_z[s], 0.0)) * m.shell;
                 if (density > 0.0) {
-                    double const r = out / (density * dmax(m.volume, 1.0e-300));
-                    rate_max = bits(r) > rate_max ? bits(r) : rate_max;
-                    double const sp[4] = {-fl_r[s], fh_r[s], -fl_z[s], fh_z[s]};
-                    for (double x : sp) {
-                        double const sv = dmax(x, 0.0) / density;
+                    // divided out only where they can exceed the largest so
+                    // far; the fastest face is the one of the largest flux
+                    double const held = density * volume.b;
+                    if (!(out < __longlong_as_double(static_cast<long long>(rate_max)) * held * kBelowOne)) {
+                        double const r = out / held;
+                        rate_max = bits(r) > rate_max ? bits(r) : rate_max;
+                    }
+                    double const x = dmax(dmax(dmax(-fl_r[s], fh_r[s]), dmax(-fl_z[s], fh_z[s])), 0.0);
+                    if (!(x < __longlong_as_double(static_cast<long long>(speed_max)) * density * kBelowOne)) {
+                        double const sv = x / density;
                         speed_max = bits(sv) > speed_max ? bits(sv) : speed_max;
                     }
                 }
@@ -800,7 +895,7 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
                 if (moves) {
                     double const r_delta = fh_r[s] * m.a_hi - fl_r[s] * m.a_lo;
                     double const z_delta = (fh_z[s] - fl_z[s]) * m.shell;
-                    v = o - p.dt * (r_delta + z_delta) / dmax(m.volume, 1.0e-300);
+                    v = o - exact_quot(p.dt * (r_delta + z_delta), volume);
                 }
             }
             new3[s * nc + k] = v;
@@ -813,7 +908,7 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
         double const cz_hi = kQe * (fh_z[0] - fh_z[1] - fh_z[2]);
         double delta = cr_hi * m.a_hi - cr_lo * m.a_lo;
         delta += (cz_hi - cz_lo) * m.shell;
-        rho[k] -= p.dt * delta / dmax(m.volume, 1.0e-300);
+        rho[k] -= exact_quot(p.dt * delta, volume);
         // carrier centres of the new state
         double const pc = dmax(new3[k], 0.0) * m.volume;
         double const qc = dmax(new3[nc + k], 0.0) * m.volume;
@@ -942,7 +1037,8 @@ struct FluidState {
     double* sums = nullptr;
     u64* words = nullptr;
     bool chi_bound = false;
-    double* closure = nullptr;   // 11 columns
+    double* closure = nullptr;   // 11 columns, then the interval-polynomial rows
+    RreaRowIndex closure_rows{};
     int closure_n = 0;
     int blocks = 1;
     std::string error;
@@ -981,12 +1077,19 @@ bool mobility_table(rrea_gpu_fluid_config const& c)
 }
 bool attachment_table(rrea_gpu_fluid_config const& c) { return c.attachment_model == RREA_GPU_ATTACHMENT_EN_TABLE; }
 
+// A column launch of about s.blocks blocks of 32 columns x 8 rows.
+dim3 column_grid(FluidState const& s)
+{
+    int const x = (s.grid.nr + 31) / 32, rows = (s.grid.nz + 7) / 8;
+    return dim3(static_cast<unsigned>(x), static_cast<unsigned>(std::max(1, std::min(rows, s.blocks / x))));
+}
+
 rrea_dev::fluid::Closure dev_closure(FluidState const& s)
 {
     int const m = s.closure_n;
     double const* b = s.closure;
     return rrea_dev::fluid::Closure{m,          b,          b + m,      b + 2 * m, b + 3 * m, b + 4 * m,
-                                    b + 5 * m,  b + 6 * m,  b + 7 * m,  b + 8 * m, b + 9 * m, b + 10 * m};
+                                    b + 5 * m,  b + 6 * m,  b + 7 * m,  b + 8 * m, b + 9 * m, b + 10 * m, b, s.closure_rows};
 }
 
 cudaError_t reset_reductions(FluidState& s, cudaStream_t stream)
@@ -1048,6 +1151,10 @@ rrea_dev::fluid::TransportParams transport_params(FluidState const& s, double dt
     p.law[2] = electron_law(c);
     p.scalar_chi = c.transport_density_ratio;
     p.dt = dt;
+    p.dr = rrea_dev::exact_divisor(s.grid.dr);
+    p.dz = rrea_dev::exact_divisor(s.grid.dz);
+    p.dr2 = rrea_dev::exact_divisor(2.0 * s.grid.dr);
+    p.dz2 = rrea_dev::exact_divisor(2.0 * s.grid.dz);
     p.limiter_cfl = c.ion_drift_cfl * (1.0 - 512.0 * 2.220446049250313e-16);
     return p;
 }
@@ -1124,9 +1231,26 @@ cudaError_t fluid_load_closure(FluidState& s, std::vector<double> const& columns
     if (s.closure) cudaFree(s.closure);
     s.closure = nullptr;
     s.closure_n = 0;
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&s.closure), sizeof(double) * columns.size());
+    std::vector<double> data = columns;
+    while (data.size() % 4 != 0) data.push_back(0.0);
+    s.closure_rows = RreaRowIndex{};
+    s.closure_rows.span_key = -1;
+    double const* const en = columns.data();
+    if (nodes >= 2 && en[0] > 0.0) {
+        std::vector<std::vector<rrea_host::RowColumn>> cols;
+        for (int c : {2, 4, 5, 7, 9}) {   // k0, nu2, nu3, dl, dt
+            rrea_host::RowColumn col;
+            col.mode = RREA_INTERP_LOGLOG_ZERO_THRESHOLD;
+            col.x = en;
+            col.y = en + static_cast<size_t>(c) * nodes;
+            col.n = nodes;
+            cols.push_back({col});
+        }
+        rrea_host::push_rows(data, s.closure_rows, en[0], en[nodes - 1], cols);
+    }
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&s.closure), sizeof(double) * data.size());
     if (e != cudaSuccess) return e;
-    e = cudaMemcpy(s.closure, columns.data(), sizeof(double) * columns.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(s.closure, data.data(), sizeof(double) * data.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) s.closure_n = nodes;
     return e;
 }
@@ -1161,7 +1285,7 @@ int64_t fluid_cells(FluidState const& s) { return s.n; }
 cudaError_t fluid_take_sources(FluidState& s, const double* cells5, double dt, cudaStream_t stream)
 {
     note_launch();
-    rrea_dev::fluid::normalize_sources_kernel<<<s.blocks, 256, 0, stream>>>(dev_grid(s.grid), dt, cells5, s.se, s.sp,
+    rrea_dev::fluid::normalize_sources_kernel<<<column_grid(s), dim3(32, 8), 0, stream>>>(dev_grid(s.grid), dt, cells5, s.se, s.sp,
                                                                             s.sn);
     return cudaGetLastError();
 }
@@ -1190,7 +1314,7 @@ void launch_closure(FluidState& s, const double* er, const double* ez, cudaStrea
 {
     rrea_gpu_fluid_config const& c = s.cfg;
     note_launch();
-    rrea_dev::fluid::closure_kernel<<<s.blocks, 256, 0, stream>>>(
+    rrea_dev::fluid::closure_kernel<<<column_grid(s), dim3(32, 8), 0, stream>>>(
         dev_closure(s), dev_grid(s.grid), c.transport_density_ratio, s.chi_bound ? s.chi : nullptr, er, ez, s.ne, s.se,
         mobility_table(c) ? s.mu : nullptr, attachment_table(c) ? s.nu : nullptr, mobility_table(c) ? s.d3 : nullptr,
         s.words, s.sums, kWHeld, kWAbove, kWInvalid, kWMinEn, kWMaxEn, kSCount, kSHeldCount, kSSource);
@@ -1214,7 +1338,7 @@ void launch_transport(FluidState& s, double dt, const double* efr, const double*
         p, s.cur3, s.chi_bound ? s.chi : nullptr, table ? s.mu : nullptr, table ? s.d3 : nullptr, efr, efr_add, efz,
         efz_add, s.fr, s.fz, s.words, kWSigma);
     note_launch();
-    rrea_dev::fluid::limiter_kernel<<<s.blocks, 256, 0, stream>>>(p, s.cur3, s.fr, s.fz, s.scale3, s.words, s.sums,
+    rrea_dev::fluid::limiter_kernel<<<column_grid(s), dim3(32, 8), 0, stream>>>(p, s.cur3, s.fr, s.fz, s.scale3, s.words, s.sums,
                                                                   kWUnlimited, kWMinScale, kSBefore, kSRemoved,
                                                                   kSENumber, kSELimited);
     note_launch();
@@ -1222,7 +1346,7 @@ void launch_transport(FluidState& s, double dt, const double* efr, const double*
                                                                          jr_kin ? s.jr : nullptr,
                                                                          jz_kin ? s.jz : nullptr);
     note_launch();
-    rrea_dev::fluid::update_kernel<<<s.blocks, 256, 0, stream>>>(p, s.cur3, s.fr, s.fz, s.next3, s.rho,
+    rrea_dev::fluid::update_kernel<<<column_grid(s), dim3(32, 8), 0, stream>>>(p, s.cur3, s.fr, s.fz, s.next3, s.rho,
                                                                  s.chi_bound ? s.chi : nullptr, s.words, s.sums, kWRate,
                                                                  kWSpeed, kWMinDensity, kWNonfinite,
                                                                  centres ? kSCenter : -1);
