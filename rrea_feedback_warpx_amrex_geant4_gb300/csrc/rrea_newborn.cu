@@ -23,12 +23,15 @@ namespace {
 // advances anything that is not a photon or a positron as an electron).
 template <int NP, int SPECIES>
 __global__ void __launch_bounds__(128, RREA_NEWBORN_MIN_BLOCKS) newborn_kernel(const __grid_constant__ ElectronArgs A, rrea_gpu_secondary* __restrict__ items,
-                                                      int64_t n, uint32_t* __restrict__ alive)
+                                                      int64_t n, int claim, uint32_t* __restrict__ alive)
 {
     StepConstants const& C = c_step;
     __shared__ IonPairSlot ion_slots[128];  // one per thread; launched with 128 threads
-    for (int64_t ip = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; ip < n;
-         ip += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int const lane = threadIdx.x & 31;
+    int64_t const warp = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+    int64_t const warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    if (lane >= claim) return;
+    for (int64_t ip = warp * claim + lane; ip < n; ip += warps * claim) {
         int const raw = items[ip].species;
         int const sp = raw == 1 ? 1 : (raw == 2 ? 2 : 0);
         if (sp != SPECIES) continue;
@@ -176,7 +179,16 @@ cudaError_t newborn_step(rrea_dev::ElectronArgs const& args, rrea_gpu_secondary*
 {
     using namespace rrea_dev;
     if (n <= 0) return cudaSuccess;
-    int const blocks = grid_for(n, max_blocks);
+    // Items per warp: the fewest that two resident waves of the electron
+    // kernel hold.  Most newborns meet a discrete event or their end, so the
+    // lanes of a warp wait for one another's samplers: fewer lanes per warp
+    // shorten the longest warp, which is what a short queue waits for.
+    // Drains of a step's secondaries, items per warp 32 / 8 / 4 / 2 / 1:
+    // 1e4 plain-case electrons 0.94 / 0.74 / 0.68 / 0.66 / 0.69 ms, 6e4
+    // 1.12 / 1.00 / 0.92 / 0.92 / 1.00, 2e5 (16 at its best 1.31) 1.38 / 1.35.
+    int claim = 1;
+    while (claim < 32 && n > static_cast<int64_t>(max_blocks) * 4 * claim) claim *= 2;
+    int const blocks = grid_for((n + claim - 1) / claim * 32, max_blocks);
     for (int k = 0; k < 3; ++k) note_launch();
     // The species kernels touch disjoint items, so the positron and photon
     // ones run beside the electron one; each is a short wave whose length is
@@ -191,13 +203,13 @@ cudaError_t newborn_step(rrea_dev::ElectronArgs const& args, rrea_gpu_secondary*
         s2 = side[1];
     }
     if (periodic) {
-        newborn_kernel<4, 0><<<blocks, 128, 0, stream>>>(args, items, n, alive);
-        newborn_kernel<4, 1><<<blocks, 128, 0, s1>>>(args, items, n, alive);
-        newborn_kernel<4, 2><<<blocks, 128, 0, s2>>>(args, items, n, alive);
+        newborn_kernel<4, 0><<<blocks, 128, 0, stream>>>(args, items, n, claim, alive);
+        newborn_kernel<4, 1><<<blocks, 128, 0, s1>>>(args, items, n, claim, alive);
+        newborn_kernel<4, 2><<<blocks, 128, 0, s2>>>(args, items, n, claim, alive);
     } else {
-        newborn_kernel<1, 0><<<blocks, 128, 0, stream>>>(args, items, n, alive);
-        newborn_kernel<1, 1><<<blocks, 128, 0, s1>>>(args, items, n, alive);
-        newborn_kernel<1, 2><<<blocks, 128, 0, s2>>>(args, items, n, alive);
+        newborn_kernel<1, 0><<<blocks, 128, 0, stream>>>(args, items, n, claim, alive);
+        newborn_kernel<1, 1><<<blocks, 128, 0, s1>>>(args, items, n, claim, alive);
+        newborn_kernel<1, 2><<<blocks, 128, 0, s2>>>(args, items, n, claim, alive);
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && s1 != stream) {
