@@ -124,6 +124,27 @@ struct rrea_gpu_seed_schedule {
     rrea_host::SeedSchedule s;
 };
 
+// The words a phase, a drain or a commit leaves on the device for the host, in
+// one block: one memset clears them and one pinned copy brings them over
+// (eight bytes at a time into pageable memory, each read waited for by itself,
+// were a third of a small step's host time).
+struct DeviceWords {
+    // cleared before a drain's chunk; with `transported` and `work` before a phase
+    unsigned long long sec_count;
+    int status;
+    int pad;
+    unsigned long long transported;
+    // per chunk of a phase: dynamic scheduling counters of its kernel, of the
+    // full kernel over the common-history loop's records, and the records' count
+    unsigned long long work[3 * kPhaseChunks];
+    long long fail_index;
+    // payload check: failures, and INT64_MAX - the lowest failing index
+    unsigned long long invalid;
+    unsigned long long invalid_first;
+    int64_t total;                            // of the last scan that asked for it
+    unsigned long long accepted[kSpecies];    // records each tile takes at a commit
+};
+
 struct rrea_gpu_ctx {
     rrea_gpu_config cfg{};
     int64_t capacity = 0;
@@ -171,7 +192,8 @@ struct rrea_gpu_ctx {
     rrea_gpu_secondary* d_sec_unordered = nullptr;
     rrea_gpu_secondary* d_sec_ordered = nullptr;
     int64_t sec_capacity = 0;
-    unsigned long long* d_sec_count = nullptr;
+    DeviceWords* d_words = nullptr;
+    DeviceWords* h_words = nullptr;   // pinned
     uint32_t* d_sec_per_parent = nullptr;
     int64_t* d_offsets = nullptr;
     int64_t* d_scan_scratch = nullptr;
@@ -186,13 +208,7 @@ struct rrea_gpu_ctx {
     uint64_t* d_diag_sub = nullptr;
     uint64_t* d_diag_ev = nullptr;
     int32_t* d_diag_disp = nullptr;
-    int* d_status = nullptr;
-    long long* d_fail_index = nullptr;
-    unsigned long long* d_transported = nullptr;
-    // per chunk: dynamic scheduling counters of the phase kernel, of the full
-    // kernel over the common-history loop's records, and the records' count
-    unsigned long long* d_work = nullptr;
-    rrea_dev::ResumeRec* d_resume = nullptr;  // those records, one slot per tile slot
+    rrea_dev::ResumeRec* d_resume = nullptr;  // the common-history loop's records, one slot per tile slot
     // a drop-in phase call uploads its host tile in chunks on side[0] while
     // the kernels of earlier chunks run on `stream` and side[1]
     cudaEvent_t chunk_up[kPhaseChunks] = {};
@@ -233,7 +249,11 @@ struct rrea_gpu_ctx {
     bool part_valid[kSpecies] = {false, false, false};
     int64_t pc_cand_cap = 0;
     uint64_t* d_child_lineage = nullptr;
-    unsigned long long* d_invalid = nullptr;
+    // pinned staging of a drain: children per item of a chunk, lineages of its children
+    uint32_t* h_counts = nullptr;
+    int64_t counts_cap = 0;
+    uint64_t* h_lineage = nullptr;
+    int64_t lineage_cap = 0;
     // roots of the initial FIFO items (16 B each) on the device and in pinned
     // host memory, grown with the FIFO
     unsigned long long* d_roots = nullptr;
@@ -422,16 +442,15 @@ rrea_gpu_status rrea_gpu_create(const rrea_gpu_config* cfg, int64_t capacity, rr
     ctx->sec_capacity = 2 * capacity + 4096;
     size_t const nsec = static_cast<size_t>(ctx->sec_capacity);
     ok = ok && dalloc(&ctx->d_sec_unordered, nsec) == cudaSuccess && dalloc(&ctx->d_sec_ordered, nsec) == cudaSuccess
-        && dalloc(&ctx->d_sec_count, 1) == cudaSuccess && dalloc(&ctx->d_sec_per_parent, n) == cudaSuccess
+        && dalloc(&ctx->d_words, 1) == cudaSuccess && dalloc(&ctx->d_sec_per_parent, n) == cudaSuccess
+        && cudaMallocHost(reinterpret_cast<void**>(&ctx->h_words), sizeof(DeviceWords)) == cudaSuccess
         && dalloc(&ctx->d_offsets, n) == cudaSuccess
         && dalloc(&ctx->d_scan_scratch, static_cast<size_t>(rrea_launch::scan_scratch_elems(capacity))) == cudaSuccess
         && dalloc(&ctx->d_diag_sub, n) == cudaSuccess && dalloc(&ctx->d_diag_ev, n) == cudaSuccess
-        && dalloc(&ctx->d_diag_disp, n) == cudaSuccess && dalloc(&ctx->d_status, 1) == cudaSuccess
-        && dalloc(&ctx->d_fail_index, 1) == cudaSuccess && dalloc(&ctx->d_transported, 1) == cudaSuccess
+        && dalloc(&ctx->d_diag_disp, n) == cudaSuccess
         && dalloc(&ctx->d_alive, n) == cudaSuccess && dalloc(&ctx->d_child_lineage, nsec) == cudaSuccess
         && dalloc(&ctx->d_cost_scratch,
                   static_cast<size_t>(kPhaseChunks) * rrea_launch::cost_order_scratch_elems()) == cudaSuccess
-        && dalloc(&ctx->d_invalid, 1) == cudaSuccess && dalloc(&ctx->d_work, 3 * kPhaseChunks) == cudaSuccess
         && dalloc(&ctx->d_resume, n) == cudaSuccess
         && cudaEventCreate(&ctx->ev_start) == cudaSuccess && cudaEventCreate(&ctx->ev_stop) == cudaSuccess;
     if (!ok) return bail(RREA_GPU_ERR_CUDA);
@@ -469,7 +488,8 @@ rrea_gpu_status rrea_gpu_destroy(rrea_gpu_ctx* ctx)
     dfree(ctx->d_planes);
     dfree(ctx->d_sec_unordered);
     dfree(ctx->d_sec_ordered);
-    dfree(ctx->d_sec_count);
+    dfree(ctx->d_words);
+    if (ctx->h_words) cudaFreeHost(ctx->h_words);
     dfree(ctx->d_sec_per_parent);
     dfree(ctx->d_offsets);
     dfree(ctx->d_scan_scratch);
@@ -483,9 +503,6 @@ rrea_gpu_status rrea_gpu_destroy(rrea_gpu_ctx* ctx)
     dfree(ctx->d_diag_sub);
     dfree(ctx->d_diag_ev);
     dfree(ctx->d_diag_disp);
-    dfree(ctx->d_status);
-    dfree(ctx->d_fail_index);
-    dfree(ctx->d_transported);
     dfree(ctx->d_fifo);
     dfree(ctx->d_surv);
     dfree(ctx->d_commit_flags);
@@ -503,10 +520,10 @@ rrea_gpu_status rrea_gpu_destroy(rrea_gpu_ctx* ctx)
     rrea_launch::population_work_free(ctx->pop_work);
     dfree(ctx->d_pc_cand);
     dfree(ctx->d_child_lineage);
-    dfree(ctx->d_invalid);
+    if (ctx->h_counts) cudaFreeHost(ctx->h_counts);
+    if (ctx->h_lineage) cudaFreeHost(ctx->h_lineage);
     dfree(ctx->d_roots);
     if (ctx->h_roots) cudaFreeHost(ctx->h_roots);
-    dfree(ctx->d_work);
     dfree(ctx->d_resume);
     if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
     if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
@@ -801,7 +818,7 @@ rrea_dev::ElectronArgs sink_args(rrea_gpu_ctx* ctx, rrea_dev::StepConstants cons
     rrea_gpu_config const& c = ctx->cfg;
     rrea_dev::ElectronArgs a{};
     a.sec = ctx->d_sec_unordered;
-    a.sec_count = ctx->d_sec_count;
+    a.sec_count = &ctx->d_words->sec_count;
     a.sec_capacity = ctx->sec_capacity;
     a.sec_per_parent = ctx->d_sec_per_parent;
     a.cells = ctx->d_cells;
@@ -813,9 +830,9 @@ rrea_dev::ElectronArgs sink_args(rrea_gpu_ctx* ctx, rrea_dev::StepConstants cons
     a.diag_subcycles = ctx->diagnostics ? ctx->d_diag_sub : nullptr;
     a.diag_events = ctx->diagnostics ? ctx->d_diag_ev : nullptr;
     a.diag_disposition = ctx->diagnostics ? ctx->d_diag_disp : nullptr;
-    a.status = ctx->d_status;
-    a.fail_index = ctx->d_fail_index;
-    a.transported = ctx->d_transported;
+    a.status = &ctx->d_words->status;
+    a.fail_index = &ctx->d_words->fail_index;
+    a.transported = &ctx->d_words->transported;
     a.arena = ctx->d_arena;
     a.fv.cell_er = ctx->d_cell_er;
     a.fv.cell_ez = ctx->d_cell_ez;
@@ -849,6 +866,30 @@ rrea_dev::ElectronArgs sink_args(rrea_gpu_ctx* ctx, rrea_dev::StepConstants cons
         a.plane_bins = ctx->d_planes + ctx->n_planes;
     }
     return a;
+}
+
+// Brings the device words to ctx->h_words and waits for the stream.
+rrea_gpu_status read_words(rrea_gpu_ctx* ctx)
+{
+    RREA_CUDA(ctx, cudaMemcpyAsync(ctx->h_words, ctx->d_words, sizeof(DeviceWords), cudaMemcpyDeviceToHost, ctx->stream));
+    RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return RREA_GPU_OK;
+}
+
+// Pinned array of at least n elements; grown only where no copy into or out
+// of it is in flight.
+template <class T>
+rrea_gpu_status grow_pinned(rrea_gpu_ctx* ctx, T*& p, int64_t& cap, int64_t n)
+{
+    if (n <= cap) return RREA_GPU_OK;
+    RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    int64_t const want = std::max<int64_t>(n, 2 * cap);
+    cap = 0;
+    RREA_CUDA(ctx, cudaMallocHost(reinterpret_cast<void**>(&p), static_cast<size_t>(want) * sizeof(T)));
+    cap = want;
+    return RREA_GPU_OK;
 }
 
 // Uploads tile elements [off, off + len) of every column on `s`.
@@ -889,12 +930,10 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
     if (!(dt_s > 0.0) || !std::isfinite(dt_s)) return fail(ctx, RREA_GPU_ERR_ARGUMENT, "dt must be finite and positive");
     rrea_gpu_config const& c = ctx->cfg;
     rrea_dev::StepConstants const sc = step_constants(ctx, step, dt_s);
-    RREA_CUDA(ctx, rrea_launch::set_step_constants(sc, ctx->stream));
-    if (species == RREA_SPECIES_PHOTON) RREA_CUDA(ctx, rrea_launch::photon_constants(sc, ctx->stream));
-    if (species == RREA_SPECIES_POSITRON) RREA_CUDA(ctx, rrea_launch::positron_constants(sc, ctx->stream));
-    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_sec_count, 0, sizeof(unsigned long long), ctx->stream));
-    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
-    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_transported, 0, sizeof(unsigned long long), ctx->stream));
+    RREA_CUDA(ctx, species == RREA_SPECIES_PHOTON     ? rrea_launch::photon_constants(sc, ctx->stream)
+                   : species == RREA_SPECIES_POSITRON ? rrea_launch::positron_constants(sc, ctx->stream)
+                                                      : rrea_launch::set_step_constants(sc, ctx->stream));
+    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_words, 0, offsetof(DeviceWords, fail_index), ctx->stream));
 
     rrea_dev::ElectronArgs a = sink_args(ctx, sc);
     SpeciesTile& st = ctx->tiles[species];
@@ -929,9 +968,6 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         if (fit < min_blocks) min_blocks = fit;
     }
     bool const lean = species == RREA_SPECIES_ELECTRON && c.periodic_z == 0 && a.n_planes == 0 && a.n >= kLeanMinParticles;
-#ifndef RREA_STATIC_SCHEDULE
-    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long) * 3 * kPhaseChunks, ctx->stream));
-#endif
     RREA_CUDA(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
     if (host && chunks == 1) {
         if (ctx->prefetched[species]) {
@@ -980,7 +1016,7 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         if (b.diag_events) b.diag_events += off;
         if (b.diag_disposition) b.diag_disposition += off;
 #ifndef RREA_STATIC_SCHEDULE
-        b.work = ctx->d_work + k;
+        b.work = ctx->d_words->work + k;
         // a chunk of a drop-in tile is visited in its own scheduling order
         // (chunk-local indices at d_alive + off), built once the chunk has landed
         if (chunks > 1 && species != RREA_SPECIES_PHOTON && ctx->schedule_order && len >= kScheduleMinParticles) {
@@ -1001,13 +1037,13 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
                                                       c.periodic_z != 0, cs));
         } else if (lean) {
             b.resume = ctx->d_resume + off;
-            b.resume_count = ctx->d_work + 2 * kPhaseChunks + k;
+            b.resume_count = ctx->d_words->work + 2 * kPhaseChunks + k;
             RREA_CUDA(ctx, rrea_launch::electron_lean(b, blocks > 0 ? blocks : 1, ctx->launch_threads, ctx->launch_min_blocks, cs));
             // the rest: about one electron in twenty, so the variant with
             // registers for a quarter of the SM's threads
             b.resumed = 1;
             b.order = nullptr;
-            b.work = ctx->d_work + kPhaseChunks + k;
+            b.work = ctx->d_words->work + kPhaseChunks + k;
             RREA_CUDA(ctx, rrea_launch::electron_step(b, ctx->num_sms * 8, 128, 8, false, cs));
         } else {
             RREA_CUDA(ctx, rrea_launch::electron_step(b, blocks > 0 ? blocks : 1, ctx->launch_threads, min_blocks,
@@ -1034,22 +1070,21 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
     RREA_CUDA(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
     if (a.n > 0) {
         if (a.segments) {
-            RREA_CUDA(ctx, rrea_launch::netchord_deposit(a.segments, a.n, ctx->net, dt_s, ctx->d_status,
-                                                         ctx->d_fail_index, ctx->num_sms * 8, ctx->stream));
+            RREA_CUDA(ctx, rrea_launch::netchord_deposit(a.segments, a.n, ctx->net, dt_s, a.status, a.fail_index,
+                                                         ctx->num_sms * 8, ctx->stream));
         }
     }
-    unsigned long long count = 0;
-    unsigned long long transported = 0;
-    int status = 0;
-    long long fail_index = -1;
-    RREA_CUDA(ctx, cudaMemcpyAsync(&count, ctx->d_sec_count, sizeof(count), cudaMemcpyDeviceToHost, ctx->stream));
-    RREA_CUDA(ctx, cudaMemcpyAsync(&status, ctx->d_status, sizeof(status), cudaMemcpyDeviceToHost, ctx->stream));
-    RREA_CUDA(ctx, cudaMemcpyAsync(&fail_index, ctx->d_fail_index, sizeof(fail_index), cudaMemcpyDeviceToHost,
-                                   ctx->stream));
-    RREA_CUDA(ctx, cudaMemcpyAsync(&transported, ctx->d_transported, sizeof(transported), cudaMemcpyDeviceToHost,
-                                   ctx->stream));
-    RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    ctx->last_transported = static_cast<int64_t>(transported);
+    // the parents' offsets are formed while the host waits for the words
+    RREA_CUDA(ctx, rrea_launch::exclusive_scan_counts(ctx->d_sec_per_parent, a.n, ctx->d_offsets, ctx->d_scan_scratch,
+                                                      nullptr, ctx->stream));
+    {
+        rrea_gpu_status const s = read_words(ctx);
+        if (s != RREA_GPU_OK) return s;
+    }
+    unsigned long long const count = ctx->h_words->sec_count;
+    int const status = ctx->h_words->status;
+    long long const fail_index = ctx->h_words->fail_index;
+    ctx->last_transported = static_cast<int64_t>(ctx->h_words->transported);
     ctx->last_kernel_ms = 0.0f;
     if (a.n > 0) RREA_CUDA(ctx, cudaEventElapsedTime(&ctx->last_kernel_ms, ctx->ev_start, ctx->ev_stop));
     if (status != 0) {
@@ -1063,9 +1098,8 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         return fail(ctx, RREA_GPU_ERR_CAPACITY, "secondary buffer overflow");
     }
     ctx->last_secondaries = static_cast<int64_t>(count);
-    RREA_CUDA(ctx, rrea_launch::order_secondaries(ctx->d_sec_per_parent, a.n, ctx->d_offsets, ctx->d_scan_scratch,
-                                                  ctx->d_sec_unordered, ctx->last_secondaries, ctx->d_sec_ordered,
-                                                  ctx->stream));
+    RREA_CUDA(ctx, rrea_launch::scatter_ordered(ctx->d_offsets, ctx->d_sec_unordered, ctx->last_secondaries,
+                                                ctx->d_sec_ordered, ctx->stream));
     return RREA_GPU_OK;
 }
 
@@ -1240,14 +1274,13 @@ rrea_gpu_status drain_fifo(rrea_gpu_ctx* ctx, int32_t step, double dt_s, int64_t
     ctx->last_drain_items = 0;
     RREA_CUDA(ctx, rrea_launch::newborn_constants(sc, ctx->stream));
     auto check_payloads = [&](rrea_gpu_secondary const* items, int64_t n, int mode) -> rrea_gpu_status {
-        unsigned long long invalid = 0;
-        long long first = INT64_MAX;
-        RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_invalid, 0, sizeof(unsigned long long), ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(ctx->d_fail_index, &first, sizeof(first), cudaMemcpyHostToDevice, ctx->stream));
-        RREA_CUDA(ctx, rrea_launch::validate_fifo(items, n, mode, ctx->d_invalid, ctx->d_fail_index, ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&invalid, ctx->d_invalid, sizeof(invalid), cudaMemcpyDeviceToHost, ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&first, ctx->d_fail_index, sizeof(first), cudaMemcpyDeviceToHost, ctx->stream));
-        RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        RREA_CUDA(ctx, cudaMemsetAsync(&ctx->d_words->invalid, 0, 2 * sizeof(unsigned long long), ctx->stream));
+        RREA_CUDA(ctx, rrea_launch::validate_fifo(items, n, mode, &ctx->d_words->invalid, &ctx->d_words->invalid_first,
+                                                  ctx->stream));
+        rrea_gpu_status const rs = read_words(ctx);
+        if (rs != RREA_GPU_OK) return rs;
+        unsigned long long const invalid = ctx->h_words->invalid;
+        long long const first = INT64_MAX - static_cast<long long>(ctx->h_words->invalid_first);
         if (invalid == 0) return RREA_GPU_OK;
         return fail(ctx, mode == 0 ? RREA_GPU_ERR_ARGUMENT : RREA_GPU_ERR_INVALID_STATE,
                     std::string(mode == 0 ? "transient FIFO received an invalid birth payload"
@@ -1310,14 +1343,11 @@ rrea_gpu_status drain_fifo(rrea_gpu_ctx* ctx, int32_t step, double dt_s, int64_t
         }
         return RREA_GPU_OK;
     };
-    std::vector<uint32_t> counts;
-    std::vector<uint64_t> lineage;
     int64_t cursor = 0, tail = n_initial;
     size_t root_base = 0;
     while (cursor < tail) {
         int64_t const chunk = std::min<int64_t>(tail - cursor, ctx->capacity);
-        RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_sec_count, 0, sizeof(unsigned long long), ctx->stream));
-        RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
+        RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_words, 0, offsetof(DeviceWords, transported), ctx->stream));
         rrea_dev::ElectronArgs a = sink_args(ctx, sc);
         a.diag_subcycles = nullptr;
         a.diag_events = nullptr;
@@ -1327,32 +1357,25 @@ rrea_gpu_status drain_fifo(rrea_gpu_ctx* ctx, int32_t step, double dt_s, int64_t
         RREA_CUDA(ctx, rrea_launch::newborn_step(a, items, chunk, ctx->d_alive, ctx->num_sms * 8, c.periodic_z != 0,
                                                  ctx->stream, ctx->side, ctx->fork_ev, ctx->join_ev));
         if (a.segments) {
-            RREA_CUDA(ctx, rrea_launch::netchord_deposit(a.segments, chunk, ctx->net, dt_s, ctx->d_status,
-                                                         ctx->d_fail_index, ctx->num_sms * 8, ctx->stream));
+            RREA_CUDA(ctx, rrea_launch::netchord_deposit(a.segments, chunk, ctx->net, dt_s, a.status, a.fail_index,
+                                                         ctx->num_sms * 8, ctx->stream));
         }
-        unsigned long long count = 0;
-        int status = 0;
-        long long fail_index = -1;
-        int64_t last_offset = 0;
-        uint32_t last_alive = 0;
         RREA_CUDA(ctx, rrea_launch::exclusive_scan_counts(ctx->d_alive, chunk, ctx->d_offsets, ctx->d_scan_scratch,
-                                                          ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&count, ctx->d_sec_count, sizeof(count), cudaMemcpyDeviceToHost, ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&status, ctx->d_status, sizeof(status), cudaMemcpyDeviceToHost, ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&fail_index, ctx->d_fail_index, sizeof(fail_index), cudaMemcpyDeviceToHost,
-                                       ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&last_offset, ctx->d_offsets + (chunk - 1), sizeof(last_offset),
-                                       cudaMemcpyDeviceToHost, ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&last_alive, ctx->d_alive + (chunk - 1), sizeof(last_alive),
-                                       cudaMemcpyDeviceToHost, ctx->stream));
-        counts.resize(static_cast<size_t>(chunk));
-        RREA_CUDA(ctx, cudaMemcpyAsync(counts.data(), ctx->d_sec_per_parent, static_cast<size_t>(chunk) * sizeof(uint32_t),
+                                                          &ctx->d_words->total, ctx->stream));
+        s = grow_pinned(ctx, ctx->h_counts, ctx->counts_cap, chunk);
+        if (s != RREA_GPU_OK) return s;
+        uint32_t const* const counts = ctx->h_counts;
+        RREA_CUDA(ctx, cudaMemcpyAsync(ctx->h_counts, ctx->d_sec_per_parent, static_cast<size_t>(chunk) * sizeof(uint32_t),
                                        cudaMemcpyDeviceToHost, ctx->stream));
         if (!roots_built) {
             s = build_roots();
             if (s != RREA_GPU_OK) return s;
         }
-        RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        s = read_words(ctx);
+        if (s != RREA_GPU_OK) return s;
+        unsigned long long const count = ctx->h_words->sec_count;
+        int const status = ctx->h_words->status;
+        long long const fail_index = ctx->h_words->fail_index;
         if (status != 0) {
             return fail(ctx, static_cast<rrea_gpu_status>(status),
                         "newborn transport guard failed (status " + std::to_string(status) + ") at FIFO item "
@@ -1362,7 +1385,7 @@ rrea_gpu_status drain_fifo(rrea_gpu_ctx* ctx, int32_t step, double dt_s, int64_t
             return fail(ctx, RREA_GPU_ERR_CAPACITY, "newborn child buffer overflow");
         }
         // survivors of the chunk, in FIFO order
-        int64_t const survivors = last_offset + static_cast<int64_t>(last_alive);
+        int64_t const survivors = ctx->h_words->total;
         s = grow_records(ctx, ctx->d_surv, ctx->surv_cap, ctx->n_surv + survivors, 0, ctx->n_surv);
         if (s != RREA_GPU_OK) return s;
         RREA_CUDA(ctx, rrea_launch::compact_survivors(items, ctx->d_alive, ctx->d_offsets, chunk,
@@ -1371,26 +1394,29 @@ rrea_gpu_status drain_fifo(rrea_gpu_ctx* ctx, int32_t step, double dt_s, int64_t
         // children: lineage per root in merge order, then appended behind the tail
         int64_t const n_children = static_cast<int64_t>(count);
         if (n_children > 0) {
-            lineage.resize(static_cast<size_t>(n_children));
-            size_t j = 0;
+            s = grow_pinned(ctx, ctx->h_lineage, ctx->lineage_cap, n_children);
+            if (s != RREA_GPU_OK) return s;
+            uint64_t* const lineage = ctx->h_lineage;
+            int64_t j = 0;
             for (int64_t i = 0; i < chunk; ++i) {
-                uint32_t const ci = counts[static_cast<size_t>(i)];
+                uint32_t const ci = counts[i];
                 if (ci == 0) continue;
                 uint32_t const s = slot[static_cast<size_t>(ctx->last_drain_items) - root_base + static_cast<size_t>(i)];
                 uint64_t& nx = next[s];
                 for (uint32_t t = 0; t < ci; ++t) {
-                    if (nx >= rrea_dev::kLineageCap || j >= lineage.size()) {
+                    if (nx >= rrea_dev::kLineageCap || j >= n_children) {
                         return fail(ctx, RREA_GPU_ERR_RNG_OVERFLOW, "transient FIFO lineage overflow");
                     }
                     lineage[j++] = nx++;
                     slot.push_back(s);
                 }
             }
-            if (j != lineage.size()) return fail(ctx, RREA_GPU_ERR_INVALID_STATE, "newborn child count mismatch");
-            RREA_CUDA(ctx, rrea_launch::order_secondaries(ctx->d_sec_per_parent, chunk, ctx->d_offsets,
-                                                          ctx->d_scan_scratch, ctx->d_sec_unordered, n_children,
-                                                          ctx->d_sec_ordered, ctx->stream));
-            RREA_CUDA(ctx, cudaMemcpyAsync(ctx->d_child_lineage, lineage.data(),
+            if (j != n_children) return fail(ctx, RREA_GPU_ERR_INVALID_STATE, "newborn child count mismatch");
+            RREA_CUDA(ctx, rrea_launch::exclusive_scan_counts(ctx->d_sec_per_parent, chunk, ctx->d_offsets,
+                                                              ctx->d_scan_scratch, nullptr, ctx->stream));
+            RREA_CUDA(ctx, rrea_launch::scatter_ordered(ctx->d_offsets, ctx->d_sec_unordered, n_children,
+                                                        ctx->d_sec_ordered, ctx->stream));
+            RREA_CUDA(ctx, cudaMemcpyAsync(ctx->d_child_lineage, lineage,
                                            static_cast<size_t>(n_children) * sizeof(uint64_t), cudaMemcpyHostToDevice,
                                            ctx->stream));
             // make room behind the tail; items before the cursor are no longer needed
@@ -1693,9 +1719,9 @@ rrea_gpu_status rrea_gpu_commit_survivors_resident(rrea_gpu_ctx* ctx, int64_t* c
             ctx->d_commit_scan = nullptr;
             ctx->commit_cap = 0;
             int64_t const cap = n + n / 2 + 1024;
-            if (dalloc(&ctx->d_commit_flags, static_cast<size_t>(cap)) != cudaSuccess
-                || dalloc(&ctx->d_commit_offsets, static_cast<size_t>(cap)) != cudaSuccess
-                || dalloc(&ctx->d_commit_scan, static_cast<size_t>(rrea_launch::scan_scratch_elems(cap))) != cudaSuccess) {
+            if (dalloc(&ctx->d_commit_flags, static_cast<size_t>(kSpecies * cap)) != cudaSuccess
+                || dalloc(&ctx->d_commit_offsets, static_cast<size_t>(kSpecies * cap)) != cudaSuccess
+                || dalloc(&ctx->d_commit_scan, static_cast<size_t>(rrea_launch::scan_scratch_elems(kSpecies * cap))) != cudaSuccess) {
                 cudaGetLastError();
                 return fail(ctx, RREA_GPU_ERR_CUDA, "commit scratch allocation failed");
             }
@@ -1703,17 +1729,13 @@ rrea_gpu_status rrea_gpu_commit_survivors_resident(rrea_gpu_ctx* ctx, int64_t* c
         }
         // all three species are ranked before any tile changes, so a full
         // tile leaves every tile as it was
+        RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_words->accepted, 0, sizeof(ctx->d_words->accepted), ctx->stream));
+        RREA_CUDA(ctx, rrea_launch::commit_rank(ctx->d_surv, n, ctx->d_commit_flags, ctx->d_commit_offsets,
+                                                ctx->d_commit_scan, ctx->d_words->accepted, ctx->stream));
+        rrea_gpu_status const rs = read_words(ctx);
+        if (rs != RREA_GPU_OK) return rs;
         for (int species = 0; species < kSpecies; ++species) {
-            RREA_CUDA(ctx, rrea_launch::commit_rank(ctx->d_surv, n, species, ctx->d_commit_flags,
-                                                    ctx->d_commit_offsets, ctx->d_commit_scan, ctx->stream));
-            int64_t last_off = 0;
-            uint32_t last_flag = 0;
-            RREA_CUDA(ctx, cudaMemcpyAsync(&last_off, ctx->d_commit_offsets + n - 1, sizeof(last_off),
-                                           cudaMemcpyDeviceToHost, ctx->stream));
-            RREA_CUDA(ctx, cudaMemcpyAsync(&last_flag, ctx->d_commit_flags + n - 1, sizeof(last_flag),
-                                           cudaMemcpyDeviceToHost, ctx->stream));
-            RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            added[species] = last_off + last_flag;
+            added[species] = static_cast<int64_t>(ctx->h_words->accepted[species]);
             if (ctx->tiles[species].n + added[species] > ctx->capacity) {
                 return fail(ctx, RREA_GPU_ERR_CAPACITY, "committed survivors exceed the resident tile capacity");
             }
@@ -1721,8 +1743,6 @@ rrea_gpu_status rrea_gpu_commit_survivors_resident(rrea_gpu_ctx* ctx, int64_t* c
         for (int species = 0; species < kSpecies; ++species) {
             if (added[species] == 0) continue;
             SpeciesTile& st = ctx->tiles[species];
-            RREA_CUDA(ctx, rrea_launch::commit_rank(ctx->d_surv, n, species, ctx->d_commit_flags,
-                                                    ctx->d_commit_offsets, ctx->d_commit_scan, ctx->stream));
             const int64_t* ids = nullptr;
             if (ctx->n_instances > 0) {
                 RREA_CUDA(ctx, rrea_launch::ensemble_survivor_ids(ctx->d_surv, n, species,
@@ -1730,7 +1750,8 @@ rrea_gpu_status rrea_gpu_commit_survivors_resident(rrea_gpu_ctx* ctx, int64_t* c
                                                                   ctx->d_inst_next_id, ctx->ens_work, &ids,
                                                                   ctx->stream));
             }
-            RREA_CUDA(ctx, rrea_launch::commit_scatter(ctx->d_surv, n, species, ctx->d_commit_offsets, columns(st),
+            RREA_CUDA(ctx, rrea_launch::commit_scatter(ctx->d_surv, n, species,
+                                                       ctx->d_commit_offsets + species * n, columns(st),
                                                        st.n, ctx->next_id[species], ids, ctx->stream));
             ctx->part_valid[species] = false;
             st.n += added[species];
@@ -1771,18 +1792,14 @@ rrea_gpu_status rrea_gpu_compact_resident(rrea_gpu_ctx* ctx, int32_t species, in
             ctx->spare_ready = true;
         }
         RREA_CUDA(ctx, rrea_launch::compact_tile(columns(st), n, ctx->d_sec_per_parent, ctx->d_offsets,
-                                                 ctx->d_scan_scratch, columns(ctx->spare), ctx->stream));
-        int64_t last_off = 0;
-        uint32_t last_flag = 0;
-        RREA_CUDA(ctx, cudaMemcpyAsync(&last_off, ctx->d_offsets + n - 1, sizeof(last_off), cudaMemcpyDeviceToHost,
-                                       ctx->stream));
-        RREA_CUDA(ctx, cudaMemcpyAsync(&last_flag, ctx->d_sec_per_parent + n - 1, sizeof(last_flag),
-                                       cudaMemcpyDeviceToHost, ctx->stream));
-        RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+                                                 ctx->d_scan_scratch, &ctx->d_words->total, columns(ctx->spare),
+                                                 ctx->stream));
+        rrea_gpu_status const rs = read_words(ctx);
+        if (rs != RREA_GPU_OK) return rs;
         for (int f = 0; f < kTileDoubles; ++f) std::swap(st.d[f], ctx->spare.d[f]);
         std::swap(st.id, ctx->spare.id);
         std::swap(st.cpu, ctx->spare.cpu);
-        st.n = last_off + last_flag;
+        st.n = ctx->h_words->total;
         ctx->part_valid[species] = false;
     }
     if (n_live) *n_live = st.n;
@@ -2236,12 +2253,11 @@ rrea_gpu_status rrea_gpu_count_live(rrea_gpu_ctx* ctx, int32_t species, int64_t*
 {
     if (!ctx || !live || species < 0 || species >= kSpecies) return RREA_GPU_ERR_ARGUMENT;
     SpeciesTile const& st = ctx->tiles[species];
-    RREA_CUDA(ctx, cudaMemsetAsync(ctx->d_transported, 0, sizeof(unsigned long long), ctx->stream));
-    RREA_CUDA(ctx, rrea_launch::count_live(st.id, st.n, ctx->d_transported, ctx->num_sms * 4, ctx->stream));
-    unsigned long long count = 0;
-    RREA_CUDA(ctx, cudaMemcpyAsync(&count, ctx->d_transported, sizeof(count), cudaMemcpyDeviceToHost, ctx->stream));
-    RREA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    *live = static_cast<int64_t>(count);
+    RREA_CUDA(ctx, cudaMemsetAsync(&ctx->d_words->transported, 0, sizeof(unsigned long long), ctx->stream));
+    RREA_CUDA(ctx, rrea_launch::count_live(st.id, st.n, &ctx->d_words->transported, ctx->num_sms * 4, ctx->stream));
+    rrea_gpu_status const rs = read_words(ctx);
+    if (rs != RREA_GPU_OK) return rs;
+    *live = static_cast<int64_t>(ctx->h_words->transported);
     return RREA_GPU_OK;
 }
 

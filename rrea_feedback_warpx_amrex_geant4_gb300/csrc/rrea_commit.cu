@@ -29,17 +29,33 @@ __device__ __forceinline__ bool commit_accepts(rrea_gpu_secondary const& s, int 
     return s.species == species && s.weight > 0.0 && (species != RREA_SPECIES_PHOTON || s.energy_eV > 0.0);
 }
 
-__global__ void commit_flags_kernel(const rrea_gpu_secondary* __restrict__ surv, int64_t n, int species,
-                                    uint32_t* __restrict__ flags)
+// One pass over the records for all species: three rows of flags, the
+// accepted counts per species.
+__global__ void commit_flags_kernel(const rrea_gpu_secondary* __restrict__ surv, int64_t n,
+                                    uint32_t* __restrict__ flags, unsigned long long* __restrict__ accepted)
 {
+    unsigned int mine[3] = {0, 0, 0};
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        flags[i] = commit_accepts(surv[i], species) ? 1u : 0u;
+        rrea_gpu_secondary const& s = surv[i];
+#pragma unroll
+        for (int species = 0; species < 3; ++species) {
+            unsigned int const f = commit_accepts(s, species) ? 1u : 0u;
+            flags[species * n + i] = f;
+            mine[species] += f;
+        }
+    }
+#pragma unroll
+    for (int species = 0; species < 3; ++species) {
+        unsigned int const warp_total = __reduce_add_sync(0xffffffffu, mine[species]);
+        if ((threadIdx.x & 31) == 0 && warp_total) {
+            atomicAdd(accepted + species, static_cast<unsigned long long>(warp_total));
+        }
     }
 }
 
-// Appends accepted records of `species` at tile index base + offsets[i],
-// with ids first_id + offsets[i] on cpu 0, or (ensemble mode, ids given)
+// Appends accepted records of `species` at tile index base + rank, rank the
+// record's offset in the species' row, with ids first_id + rank on cpu 0, or (ensemble mode, ids given)
 // the per-instance ids on the root's instance.
 __global__ void commit_scatter_kernel(const rrea_gpu_secondary* __restrict__ surv, int64_t n, int species,
                                       const int64_t* __restrict__ offsets, TileColumns t, int64_t base,
@@ -49,7 +65,8 @@ __global__ void commit_scatter_kernel(const rrea_gpu_secondary* __restrict__ sur
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         rrea_gpu_secondary const s = surv[i];
         if (!commit_accepts(s, species)) continue;
-        int64_t const k = base + offsets[i];
+        int64_t const rank = offsets[i] - offsets[0];
+        int64_t const k = base + rank;
         double px = s.dir_x, py = s.dir_y, pz = s.dir_z;
         double const norm = sqrt(px * px + py * py + pz * pz);
         if (species == RREA_SPECIES_PHOTON) {
@@ -77,7 +94,7 @@ __global__ void commit_scatter_kernel(const rrea_gpu_secondary* __restrict__ sur
         double const v[kTileColumns] = {r, s.z, th, px, py, pz, s.weight, r, s.z, th, px, py, pz};
 #pragma unroll
         for (int f = 0; f < kTileColumns; ++f) t.d[f][k] = v[f];
-        t.id[k] = ids ? ids[i] : first_id + offsets[i];
+        t.id[k] = ids ? ids[i] : first_id + rank;
         t.cpu[k] = ids ? static_cast<int32_t>(s.root_key >> 40) : 0;
     }
 }
@@ -171,13 +188,13 @@ unsigned grid_for(int64_t n, int threads)
 
 namespace rrea_launch {
 
-cudaError_t commit_rank(const rrea_gpu_secondary* surv, int64_t n, int species, uint32_t* flags, int64_t* offsets,
-                        int64_t* scan_scratch, cudaStream_t stream)
+cudaError_t commit_rank(const rrea_gpu_secondary* surv, int64_t n, uint32_t* flags, int64_t* offsets,
+                        int64_t* scan_scratch, unsigned long long* accepted, cudaStream_t stream)
 {
     if (n <= 0) return cudaSuccess;
     note_launch();
-    rrea_dev::commit_flags_kernel<<<rrea_dev::grid_for(n, 256), 256, 0, stream>>>(surv, n, species, flags);
-    return exclusive_scan_counts(flags, n, offsets, scan_scratch, stream);
+    rrea_dev::commit_flags_kernel<<<rrea_dev::grid_for(n, 256), 256, 0, stream>>>(surv, n, flags, accepted);
+    return exclusive_scan_counts(flags, 3 * n, offsets, scan_scratch, nullptr, stream);
 }
 
 cudaError_t commit_scatter(const rrea_gpu_secondary* surv, int64_t n, int species, const int64_t* offsets,
@@ -192,12 +209,12 @@ cudaError_t commit_scatter(const rrea_gpu_secondary* surv, int64_t n, int specie
 }
 
 cudaError_t compact_tile(rrea_dev::TileColumns const& src, int64_t n, uint32_t* flags, int64_t* offsets,
-                         int64_t* scan_scratch, rrea_dev::TileColumns const& dst, cudaStream_t stream)
+                         int64_t* scan_scratch, int64_t* total, rrea_dev::TileColumns const& dst, cudaStream_t stream)
 {
     if (n <= 0) return cudaSuccess;
     note_launch();
     rrea_dev::valid_flags_kernel<<<rrea_dev::grid_for(n, 256), 256, 0, stream>>>(src.id, n, flags);
-    cudaError_t const e = exclusive_scan_counts(flags, n, offsets, scan_scratch, stream);
+    cudaError_t const e = exclusive_scan_counts(flags, n, offsets, scan_scratch, total, stream);
     if (e != cudaSuccess) return e;
     note_launch();
     rrea_dev::compact_tile_kernel<<<rrea_dev::grid_for(n, 256), 256, 0, stream>>>(src, n, offsets, dst);

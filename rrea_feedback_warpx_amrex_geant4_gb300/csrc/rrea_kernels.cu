@@ -72,7 +72,11 @@ __global__ void count_live_kernel(const int64_t* __restrict__ id, int64_t n, uns
 
 // Exclusive scan of per-parent secondary counts (uint32 -> int64 offsets),
 // three passes: block sums, scan of block sums, block-local scan + offset.
+// Up to kScanOneBlock counts one block does it alone, which a small step pays a
+// dozen times: three launches of 3 us and the gaps between them against one of
+// 4.0 us at 300 counts, 5.0 at 3,000, 9.0 at 10,000 and 15 at 16,384.
 constexpr int kScanBlock = 1024;
+constexpr int64_t kScanOneBlock = 8 * kScanBlock;
 
 __device__ __forceinline__ int64_t block_exclusive_scan(int64_t v, int64_t& total)
 {
@@ -128,13 +132,38 @@ __global__ void __launch_bounds__(kScanBlock) scan_block_offsets(int64_t* __rest
 
 __global__ void __launch_bounds__(kScanBlock) scan_apply(const uint32_t* __restrict__ counts, int64_t n,
                                                          const int64_t* __restrict__ block_offsets,
-                                                         int64_t* __restrict__ offsets)
+                                                         int64_t* __restrict__ offsets, int64_t* __restrict__ sum)
 {
     int64_t const i = blockIdx.x * static_cast<int64_t>(kScanBlock) + threadIdx.x;
     int64_t const v = i < n ? counts[i] : 0;
     int64_t total;
     int64_t const p = block_exclusive_scan(v, total);
     if (i < n) offsets[i] = block_offsets[blockIdx.x] + p;
+    if (sum && i == n - 1) *sum = block_offsets[blockIdx.x] + p + v;
+}
+
+// One block, each thread a run of consecutive counts.
+__global__ void __launch_bounds__(kScanBlock) scan_one_block(const uint32_t* __restrict__ counts, int n,
+                                                             int64_t* __restrict__ offsets, int64_t* __restrict__ sum)
+{
+    constexpr int kRun = static_cast<int>(kScanOneBlock / kScanBlock);
+    int const run = (n + kScanBlock - 1) / kScanBlock;
+    int const first = threadIdx.x * run;
+    uint32_t v[kRun];
+    int64_t mine = 0;
+#pragma unroll
+    for (int k = 0; k < kRun; ++k) {
+        v[k] = k < run && first + k < n ? counts[first + k] : 0U;
+        mine += v[k];
+    }
+    int64_t total;
+    int64_t at = block_exclusive_scan(mine, total);
+#pragma unroll
+    for (int k = 0; k < kRun; ++k) {
+        if (k < run && first + k < n) offsets[first + k] = at;
+        at += v[k];
+    }
+    if (sum && threadIdx.x == 0) *sum = total;
 }
 
 __global__ void scatter_secondaries(const rrea_gpu_secondary* __restrict__ in, int64_t count,
@@ -229,33 +258,33 @@ cudaError_t count_live(const int64_t* id, int64_t n, unsigned long long* out, in
 int64_t scan_scratch_elems(int64_t n) { return (n + rrea_dev::kScanBlock - 1) / rrea_dev::kScanBlock + 1; }
 
 cudaError_t exclusive_scan_counts(const uint32_t* counts, int64_t n, int64_t* offsets, int64_t* block_scratch,
-                                  cudaStream_t stream)
+                                  int64_t* total, cudaStream_t stream)
 {
     if (n <= 0) return cudaSuccess;
+    if (n <= rrea_dev::kScanOneBlock) {
+        note_launch();
+        rrea_dev::scan_one_block<<<1, rrea_dev::kScanBlock, 0, stream>>>(counts, static_cast<int>(n), offsets, total);
+        return cudaGetLastError();
+    }
     for (int k = 0; k < 3; ++k) note_launch();
     int64_t const nblocks = (n + rrea_dev::kScanBlock - 1) / rrea_dev::kScanBlock;
     rrea_dev::scan_block_sums<<<static_cast<unsigned>(nblocks), rrea_dev::kScanBlock, 0, stream>>>(counts, n,
                                                                                                   block_scratch);
     rrea_dev::scan_block_offsets<<<1, rrea_dev::kScanBlock, 0, stream>>>(block_scratch, nblocks);
     rrea_dev::scan_apply<<<static_cast<unsigned>(nblocks), rrea_dev::kScanBlock, 0, stream>>>(counts, n, block_scratch,
-                                                                                             offsets);
+                                                                                             offsets, total);
     return cudaGetLastError();
 }
 
-cudaError_t order_secondaries(const uint32_t* counts, int64_t n, int64_t* offsets, int64_t* block_scratch,
-                              const rrea_gpu_secondary* unordered, int64_t count, rrea_gpu_secondary* ordered,
-                              cudaStream_t stream)
+cudaError_t scatter_ordered(const int64_t* offsets, const rrea_gpu_secondary* unordered, int64_t count,
+                            rrea_gpu_secondary* ordered, cudaStream_t stream)
 {
-    if (n <= 0) return cudaSuccess;
-    cudaError_t const e = exclusive_scan_counts(counts, n, offsets, block_scratch, stream);
-    if (e != cudaSuccess) return e;
-    if (count > 0) {
-        note_launch();
-        int const threads = 256;
-        int64_t const blocks = (count + threads - 1) / threads;
-        rrea_dev::scatter_secondaries<<<static_cast<unsigned>(blocks < 65535 ? blocks : 65535), threads, 0, stream>>>(
-            unordered, count, offsets, ordered);
-    }
+    if (count <= 0) return cudaSuccess;
+    note_launch();
+    int const threads = 256;
+    int64_t const blocks = (count + threads - 1) / threads;
+    rrea_dev::scatter_secondaries<<<static_cast<unsigned>(blocks < 65535 ? blocks : 65535), threads, 0, stream>>>(
+        unordered, count, offsets, ordered);
     return cudaGetLastError();
 }
 

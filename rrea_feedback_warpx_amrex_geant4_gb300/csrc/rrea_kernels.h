@@ -69,7 +69,7 @@ cudaError_t maxwell_step(int nr, int nz, double dr, double dz, double dt, int su
 // adoption of the chunk's ordered children into the FIFO tail.
 cudaError_t newborn_constants(rrea_dev::StepConstants const& sc, cudaStream_t stream);
 cudaError_t validate_fifo(const rrea_gpu_secondary* items, int64_t n, int mode, unsigned long long* invalid,
-                          long long* first, cudaStream_t stream);
+                          unsigned long long* first_from_top, cudaStream_t stream);
 // The positron and photon kernels run on side[0] and side[1] (joined back
 // into `stream`) when the side streams and events are given.
 cudaError_t newborn_step(rrea_dev::ElectronArgs const& args, rrea_gpu_secondary* items, int64_t n, uint32_t* alive,
@@ -85,26 +85,28 @@ cudaError_t eval_math(const double* arena, int which, const double* x, int64_t n
 cudaError_t count_live(const int64_t* id, int64_t n, unsigned long long* out, int blocks, cudaStream_t stream);
 int64_t scan_scratch_elems(int64_t n);
 // Exclusive scan of per-parent counts into offsets (block_scratch holds
-// scan_scratch_elems(n) elements); the first half of order_secondaries.
+// scan_scratch_elems(n) elements); their sum into *total where it is given.
 cudaError_t exclusive_scan_counts(const uint32_t* counts, int64_t n, int64_t* offsets, int64_t* block_scratch,
-                                  cudaStream_t stream);
-cudaError_t order_secondaries(const uint32_t* counts, int64_t n, int64_t* offsets, int64_t* block_scratch,
-                              const rrea_gpu_secondary* unordered, int64_t count, rrea_gpu_secondary* ordered,
-                              cudaStream_t stream);
+                                  int64_t* total, cudaStream_t stream);
+// Records to offsets[parent] + lineage.
+cudaError_t scatter_ordered(const int64_t* offsets, const rrea_gpu_secondary* unordered, int64_t count,
+                            rrea_gpu_secondary* ordered, cudaStream_t stream);
 
-// Resident commit of the drain survivors of one species (rrea_commit.cu):
-// commit_rank flags the records the species accepts and scans them
-// (offsets[n-1] + flags[n-1] accepted); commit_scatter writes them to tile
-// rows base + rank with ids first_id + rank.
-cudaError_t commit_rank(const rrea_gpu_secondary* surv, int64_t n, int species, uint32_t* flags, int64_t* offsets,
-                        int64_t* scan_scratch, cudaStream_t stream);
+// Resident commit of the drain survivors (rrea_commit.cu).  commit_rank flags
+// the records each species' tile accepts, three rows of n in species order,
+// scans them as one row of 3 n (flags, offsets and scratch for that many) and
+// adds the accepted counts to accepted[0..2]; commit_scatter, given a species'
+// row of the offsets, writes its records to tile rows base + rank with ids
+// first_id + rank.
+cudaError_t commit_rank(const rrea_gpu_secondary* surv, int64_t n, uint32_t* flags, int64_t* offsets,
+                        int64_t* scan_scratch, unsigned long long* accepted, cudaStream_t stream);
 cudaError_t commit_scatter(const rrea_gpu_secondary* surv, int64_t n, int species, const int64_t* offsets,
                            rrea_dev::TileColumns const& tile, int64_t base, int64_t first_id, const int64_t* ids,
                            cudaStream_t stream);
-// Stable compaction of the valid (id > 0) rows of src into dst; offsets[n-1]
-// + flags[n-1] is the new row count.
+// Stable compaction of the valid (id > 0) rows of src into dst; the new row
+// count into *total.
 cudaError_t compact_tile(rrea_dev::TileColumns const& src, int64_t n, uint32_t* flags, int64_t* offsets,
-                         int64_t* scan_scratch, rrea_dev::TileColumns const& dst, cudaStream_t stream);
+                         int64_t* scan_scratch, int64_t* total, rrea_dev::TileColumns const& dst, cudaStream_t stream);
 
 // Charge-exact thinning of CIC support groups (rrea_resample.cu): group g is
 // rows [offsets[g], offsets[g+1]) of fr, fz, w (w updated in place).

@@ -102,9 +102,9 @@ __global__ void adopt_children_kernel(const rrea_gpu_secondary* __restrict__ ord
 // Payload checks of the FIFO: mode 0 the birth payloads entering it
 // (O/RreaSecondaryCommit.cpp:337-373), mode 1 the final survivors at their
 // transported endpoint (:480-515).  Counts the failures and keeps the
-// lowest failing index.
+// lowest failing index, as its distance below INT64_MAX (both start at zero).
 __global__ void validate_fifo_kernel(const rrea_gpu_secondary* __restrict__ items, int64_t n, int mode,
-                                     unsigned long long* __restrict__ invalid, long long* __restrict__ first)
+                                     unsigned long long* __restrict__ invalid, unsigned long long* __restrict__ first_from_top)
 {
     StepConstants const& C = c_step;
     rrea_gpu_config const& cfg = C.cfg;
@@ -130,7 +130,7 @@ __global__ void validate_fifo_kernel(const rrea_gpu_secondary* __restrict__ item
         }
         if (!ok) {
             atomicAdd(invalid, 1ULL);
-            atomicMin(first, static_cast<long long>(i));
+            atomicMax(first_from_top, static_cast<unsigned long long>(INT64_MAX - i));
         }
     }
 }
@@ -165,11 +165,12 @@ cudaError_t newborn_constants(rrea_dev::StepConstants const& sc, cudaStream_t st
 }
 
 cudaError_t validate_fifo(const rrea_gpu_secondary* items, int64_t n, int mode, unsigned long long* invalid,
-                          long long* first, cudaStream_t stream)
+                          unsigned long long* first_from_top, cudaStream_t stream)
 {
     if (n <= 0) return cudaSuccess;
     note_launch();
-    rrea_dev::validate_fifo_kernel<<<rrea_dev::grid_for(n, 65535), 128, 0, stream>>>(items, n, mode, invalid, first);
+    rrea_dev::validate_fifo_kernel<<<rrea_dev::grid_for(n, 65535), 128, 0, stream>>>(items, n, mode, invalid,
+                                                                                      first_from_top);
     return cudaGetLastError();
 }
 

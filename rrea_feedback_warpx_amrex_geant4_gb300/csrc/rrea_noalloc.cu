@@ -147,7 +147,7 @@ extern "C" rrea_gpu_status rrea_gpu_order_secondaries_noalloc(const uint32_t* d_
     cudaStream_t const s = static_cast<cudaStream_t>(stream);
 
     e = cudaMemsetAsync(err_word, 0, sizeof(unsigned long long), s);
-    if (e == cudaSuccess) e = rrea_launch::exclusive_scan_counts(d_counts, n_parents, offsets, block_sums, s);
+    if (e == cudaSuccess) e = rrea_launch::exclusive_scan_counts(d_counts, n_parents, offsets, block_sums, nullptr, s);
     int const threads = 256;
     int64_t blocks = (n_secondaries + threads - 1) / threads;
     if (blocks < 1) blocks = 1;

@@ -716,7 +716,7 @@ cudaError_t population_thin(PopulationInput const& in, PopulationWork*& work, Po
         if (part == 0) flags_live_kernel<<<blocks_for(n), 256, 0, s>>>(in.id, n, p.flags);
         else flags_cand_kernel<<<blocks_for(n), 256, 0, s>>>(in.cand, n, in.species, p.flags);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, s)) != cudaSuccess) return e;
+        if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
         note_launch();
         scatter_members_kernel<<<blocks_for(n), 256, 0, s>>>(p.flags, p.offsets, n, counts[0], p.members);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -754,7 +754,7 @@ cudaError_t population_thin(PopulationInput const& in, PopulationWork*& work, Po
     sorted_kernel<<<blocks_for(n), 256, 0, s>>>(perm, n, p.kb, p.k2, p.k3, p.fr, p.fz, p.w, p.sfr, p.sfz, p.sw,
                                                 p.sw0, p.k2s, p.k3s, p.flags);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
     note_launch();
     group_begin_kernel<<<blocks_for(n), 256, 0, s>>>(p.flags, p.offsets, n, p.begin);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -877,7 +877,7 @@ cudaError_t population_thin_instances(PopulationInput const& in, PopulationWork*
     note_launch();
     flags_due_kernel<<<blocks_for(in.n_tile), 256, 0, s>>>(in.id, in.cpu, in.n_tile, due_k, n_inst, p.flags);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan_counts(p.flags, in.n_tile, p.offsets, p.scan_scratch, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_counts(p.flags, in.n_tile, p.offsets, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
     note_launch();
     scatter_members_kernel<<<blocks_for(in.n_tile), 256, 0, s>>>(p.flags, p.offsets, in.n_tile, 0, p.members);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -913,7 +913,7 @@ cudaError_t population_thin_instances(PopulationInput const& in, PopulationWork*
     heads_instances_kernel<<<blocks_for(n), 256, 0, s>>>(perm, n, p.kb, p.ka, p.k2, p.k3, p.fr, p.fz, p.w, p.sfr,
                                                          p.sfz, p.sw, p.sw0, p.k2s, p.k3s, p.flags);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
     note_launch();
     group_begin_kernel<<<blocks_for(n), 256, 0, s>>>(p.flags, p.offsets, n, p.begin);
     int status = 0;
@@ -995,7 +995,7 @@ cudaError_t population_split(rrea_dev::TileColumns const& t, int64_t n, double m
     note_launch();
     split_flags_kernel<<<blocks_for(n), 256, 0, s>>>(t.d[6], t.id, n, min_w, p.flags);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
     int64_t last_off = 0;
     uint32_t last_flag = 0;
     if ((e = cudaMemcpyAsync(&last_off, p.offsets + n - 1, sizeof(last_off), cudaMemcpyDeviceToHost, s)) ||
@@ -1032,7 +1032,7 @@ cudaError_t population_merge(MergeInput const& in, PopulationWork*& work, MergeS
     note_launch();
     flags_live_kernel<<<blocks_for(nt), 256, 0, s>>>(in.id, nt, p.flags);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan_counts(p.flags, nt, p.offsets, p.scan_scratch, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_counts(p.flags, nt, p.offsets, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
     note_launch();
     scatter_members_kernel<<<blocks_for(nt), 256, 0, s>>>(p.flags, p.offsets, nt, 0, p.members);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1056,7 +1056,7 @@ cudaError_t population_merge(MergeInput const& in, PopulationWork*& work, MergeS
     note_launch();
     merge_heads_kernel<<<blocks_for(n), 256, 0, s>>>(p.kb, n, p.flags);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_counts(p.flags, n, p.offsets, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
     note_launch();
     group_begin_kernel<<<blocks_for(n), 256, 0, s>>>(p.flags, p.offsets, n, p.begin);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1064,7 +1064,7 @@ cudaError_t population_merge(MergeInput const& in, PopulationWork*& work, MergeS
     note_launch();
     merge_pairs_kernel<<<blocks_for(n), 256, 0, s>>>(p.kb, p.flags, p.offsets, p.begin, n, pair_head);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan_counts(pair_head, n, p.cap_prefix, p.scan_scratch, s)) != cudaSuccess) return e;
+    if ((e = exclusive_scan_counts(pair_head, n, p.cap_prefix, p.scan_scratch, nullptr, s)) != cudaSuccess) return e;
     int64_t groups_off = 0, pairs_off = 0;
     uint32_t groups_flag = 0, pairs_flag = 0;
     if ((e = cudaMemcpyAsync(&groups_off, p.offsets + n - 1, sizeof(groups_off), cudaMemcpyDeviceToHost, s)) ||
