@@ -55,7 +55,7 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
     double run_x, run_y, run_z = z0;
     {
         double s, c;
-        sincos(A.prev_theta[ip], &s, &c);
+        fsincos(arena, A.prev_theta[ip], s, c);
         run_x = r0 * c;
         run_y = r0 * s;
     }
@@ -196,7 +196,7 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
         A.uy[ip] = um * dy;
         A.uz[ip] = um * dz;
         A.r[ip] = r;
-        A.theta[ip] = atan2(run_y, run_x);
+        A.theta[ip] = fatan2(arena, run_y, run_x);
         A.z[ip] = run_z;
         if (A.segments) {
             SegmentRec& s = A.segments[ip];

@@ -122,8 +122,11 @@ __device__ __forceinline__ dd dd_log(dd x)
     dd const xm{ldexp(x.hi, -e), ldexp(x.lo, -e)};
     dd const s = dd_div(dd_sub(xm, dd_from(1.0)), dd_add(xm, dd_from(1.0)));
     dd const s2 = dd_mul(s, s);
-    dd acc{kDdInvOdd[22][0], kDdInvOdd[22][1]};
-    for (int n = 21; n >= 0; --n) {
+    // the terms from s^22 on, below 2^-55 of the sum, in plain doubles
+    double tail = kDdInvOdd[22][0];
+    for (int n = 21; n >= 11; --n) tail = fma(tail, s2.hi, kDdInvOdd[n][0]);
+    dd acc = dd_add(dd_mul_d(s2, tail), dd{kDdInvOdd[10][0], kDdInvOdd[10][1]});
+    for (int n = 9; n >= 0; --n) {
         acc = dd_add(dd_mul(acc, s2), dd{kDdInvOdd[n][0], kDdInvOdd[n][1]});
     }
     dd const lm = dd_mul_d(dd_mul(s, acc), 2.0);

@@ -277,14 +277,14 @@ __device__ __noinline__ void clip_chord(double x0, double y0, double z0, double 
 
 // ClipRz as the reference calls it, on cylindrical ends (r, theta, z).
 template <int NP>
-__device__ __forceinline__ void clip_rz(double r0, double th0, double z0, double r1, double th1, double z1,
+__device__ __forceinline__ void clip_rz(const double* __restrict__ arena, double r0, double th0, double z0, double r1, double th1, double z1,
                                         Geom const& g, Path<NP>& p, Err& err)
 {
     bool const finite = finite_bits(th0) && finite_bits(th1);
     double s0 = 0.0, c0 = 1.0, s1 = 0.0, c1 = 1.0;
     if (finite) {
-        sincos(th0, &s0, &c0);
-        sincos(th1, &s1, &c1);
+        fsincos(arena, th0, s0, c0);
+        fsincos(arena, th1, s1, c1);
     }
     double const x0 = r0 * c0, y0 = r0 * s0, x1 = r1 * c1, y1 = r1 * s1;
     if (finite && !lt0(r0) && !lt0(r1) && clip_inside(x0, y0, z0, r0 * r0, x1, y1, z1, r1 * r1, g, p)) return;
@@ -300,17 +300,19 @@ __device__ __forceinline__ void clip_rz(double r0, double th0, double z0, double
 // (hypot(x, y), atan2(y, x), z) and turns back into r cos(theta),
 // r sin(theta).  Clipping the Cartesian ends directly gives the same chord to
 // within an ulp of each coordinate and saves an atan2 and a sincos per end.
+// True for a chord inside the domain (clip_inside).
 template <int NP>
-__device__ __forceinline__ void clip_xyz(double x0, double y0, double z0, double x1, double y1, double z1, Geom const& g,
+__device__ __forceinline__ bool clip_xyz(double x0, double y0, double z0, double x1, double y1, double z1, Geom const& g,
                                          Path<NP>& p, Err& err)
 {
-    if (clip_inside(x0, y0, z0, fma(x0, x0, y0 * y0), x1, y1, z1, fma(x1, x1, y1 * y1), g, p)) return;
+    if (clip_inside(x0, y0, z0, fma(x0, x0, y0 * y0), x1, y1, z1, fma(x1, x1, y1 * y1), g, p)) return true;
     bool const finite = finite_bits(x0) && finite_bits(y0) && finite_bits(x1) && finite_bits(y1);
     Path<NP> out;   // the out-of-line call's, so that p stays in registers
     Err e;
     clip_chord(x0, y0, z0, rz_radius(x0, y0), x1, y1, z1, rz_radius(x1, y1), finite, g, out, e);
     p = out;
     if (e.code) err.set(e.code);
+    return false;
 }
 
 // ------------------------------------------------------------ kinematics

@@ -789,7 +789,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
     normalize(dx, dy, dz);
     double const seed_th = A.prev_theta[ip];
     double sth, cth;
-    sincos(seed_th, &sth, &cth);
+    fsincos(arena, seed_th, sth, cth);
     double run_x = prev_r * cth;
     double run_y = prev_r * sth;
     double run_z = A.prev_z[ip];
@@ -1328,7 +1328,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
         A.uy[ip] = um * dy;
         A.uz[ip] = um * dz;
         A.r[ip] = rz_radius(run_x, run_y);
-        A.theta[ip] = atan2(run_y, run_x);
+        A.theta[ip] = fatan2(arena, run_y, run_x);
         A.z[ip] = run_z;
         put_segment(A.r[ip], run_z);
         return finish(0);
@@ -1367,7 +1367,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
     A.uy[ip] = um * dy;
     A.uz[ip] = um * dz;
     A.r[ip] = end_r;
-    A.theta[ip] = atan2(run_y, run_x);
+    A.theta[ip] = fatan2(arena, run_y, run_x);
     A.z[ip] = run_z;
     put_segment(end_r, run_z);
     return finish(0);

@@ -121,25 +121,84 @@ __device__ __forceinline__ double fsqrt(double x)
     return __double2hiint(x) > 0 ? x * frsqrt(x) : 0.0;
 }
 
-// sin and cos of 2 pi u for u in [0, 1): the nearest of 256 table angles and
-// the remainder r (|r| <= pi/256, exact up to the product by 2 pi/256), whose
-// sin and cos - 1 are r - r^3/6 + r^5/120 and -r^2/2 + r^4/24 - r^6/720, the
-// terms from r^4 on in FP32; within 2^-52 absolutely, for 14 FP64 slots
-// against 31 of a reduction of 2 pi u.  It takes the angle itself, where the
-// reference rounds 2 pi u (to 4e-16) first.
-__device__ __forceinline__ void sincos_turn(const double* __restrict__ arena, double u, double& s, double& c)
+// sin and cos of the table angle 2 pi j/256 plus r, |r| <= pi/256: sin r and
+// cos r - 1 are r - r^3/6 + r^5/120 and -r^2/2 + r^4/24 - r^6/720, the terms
+// from r^4 on in FP32; within 2^-52 absolutely.
+constexpr double kTurnStep = 2.45436926061702587187e-02;     // RN(2 pi / 256)
+constexpr double kTurnStepLo = 9.56755311833869693105e-19;   // RN(2 pi / 256 - kTurnStep)
+constexpr double kInvTurnStep = 4.07436654315252084757e+01;  // RN(256 / (2 pi))
+__device__ __forceinline__ void sincos_step(const double* __restrict__ arena, int j, double r, double& s, double& c)
 {
-    constexpr double magic = 6755399441055744.0;   // 1.5 2^52: the sum's low word is the nearest integer
-    double const t = fma(u, 256.0, magic);
-    int const j = __double2loint(t) & 255;
-    double const r = fma(u, 256.0, magic - t) * 2.45436926061702596755e-02;   // 2 pi / 256
-    double2 const tab = __ldg(reinterpret_cast<const double2*>(arena + RREA_ARENA_TURN_TABLE) + j);
+    double2 const tab = __ldg(reinterpret_cast<const double2*>(arena + RREA_ARENA_TURN_TABLE) + (j & 255));
     double const r2 = r * r;
     float const q = narrow_f32(r2);
     double const cm = r2 * (widen_f32(q * (1.0f / 24.0f - q * (1.0f / 720.0f))) - 0.5);
     double const sr = fma(r * r2, widen_f32(q * (1.0f / 120.0f)) - 1.0 / 6.0, r);
     s = fma(tab.y, sr, fma(tab.x, cm, tab.x));
     c = fma(-tab.x, sr, fma(tab.y, cm, tab.y));
+}
+// sin and cos of 2 pi u for u in [0, 1): the nearest of 256 table angles and
+// the remainder (exact up to the product by 2 pi/256), 14 FP64 slots against
+// 31 of a reduction of 2 pi u.  It takes the angle itself, where the
+// reference rounds 2 pi u (to 4e-16) first.
+__device__ __forceinline__ void sincos_turn(const double* __restrict__ arena, double u, double& s, double& c)
+{
+    constexpr double magic = 6755399441055744.0;   // 1.5 2^52: the sum's low word is the nearest integer
+    double const t = fma(u, 256.0, magic);
+    sincos_step(arena, __double2loint(t), fma(u, 256.0, magic - t) * kTurnStep, s, c);
+}
+// sin and cos of an angle in radians, |a| < 2^10 (the rest goes to CUDA's):
+// the remainder against the nearest table angle by two multiply-adds.
+static __device__ __noinline__ double2 sincos_any(double a)
+{
+    double2 v;
+    sincos(a, &v.x, &v.y);
+    return v;
+}
+__device__ __forceinline__ void fsincos(const double* __restrict__ arena, double a, double& s, double& c)
+{
+    if ((__double2hiint(a) & 0x7fffffff) >= 0x40900000) {   // |a| >= 2^10, infinite or NaN
+        double2 const v = sincos_any(a);
+        s = v.x;
+        c = v.y;
+        return;
+    }
+    constexpr double magic = 6755399441055744.0;
+    double const t = fma(a, kInvTurnStep, magic);
+    double const k = t - magic;
+    sincos_step(arena, __double2loint(t), fma(-k, kTurnStepLo, fma(-k, kTurnStep, a)), s, c);
+}
+
+// atan2(y, x): the FP32 angle names the nearest of 256 table angles a, the
+// point is turned by -a to (u, v) (v with the rounding of its second product
+// recovered, so that it keeps its relative accuracy), and with t = v/u,
+// |t| < tan(pi/250), the angle is a + t - t^3/3 + t^5/5 - t^7/7 + t^9/9 (the
+// last two terms in FP32; the next is below 2^-67): within two ulps, for 20
+// FP64 slots against 46.  Points nearer than 2^-100 to the axis or farther
+// than 2^100 go to CUDA's.
+static __device__ __noinline__ double atan2_any(double y, double x) { return atan2(y, x); }
+
+__device__ __forceinline__ double fatan2(const double* __restrict__ arena, double y, double x)
+{
+    int const j = __float2int_rn(atan2f(narrow_f32(y), narrow_f32(x)) * static_cast<float>(kInvTurnStep));
+    double2 const tab = __ldg(reinterpret_cast<const double2*>(arena + RREA_ARENA_TURN_TABLE) + (j & 255));
+    double const u = fma(x, tab.y, y * tab.x);
+    uint32_t const hi = static_cast<uint32_t>(__double2hiint(u));
+    if (hi - 0x39b00000u > 0x0c800000u) return atan2_any(y, x);
+    double const p = x * tab.x;
+    double const v = fma(y, tab.y, -p) - fma(x, tab.x, -p);
+    // v / u: an FP32 reciprocal, one Newton step, the quotient's residual
+    float y32;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y32) : "f"(narrow_f32(u)));
+    double w = widen_f32(y32);
+    w = fma(w, fma(-u, w, 1.0), w);
+    double const t0 = v * w;
+    double const t = fma(w, fma(-u, t0, v), t0);
+    double const t2 = t * t;
+    float const q = narrow_f32(t2);
+    double const s = fma(t2, 0.2 - widen_f32(q * (1.0f / 7.0f - q * (1.0f / 9.0f))), -1.0 / 3.0);
+    double const k = __longlong_as_double(0x4338000000000000LL + j) - 6755399441055744.0;   // j as a double
+    return fma(k, kTurnStep, fma(k, kTurnStepLo, fma(t * t2, s, t)));
 }
 
 }  // namespace rrea_dev

@@ -625,8 +625,8 @@ __device__ int advance_photon_newborn(StepConstants const& C, ElectronArgs const
         build_intervals(path, g, A.prof, rho, iv, err);
         PhotonRates rates;
         if (!photon_rates(C, arena, energy, rates, err)) return -1;
-        double const mfp = mfp_from_inverse(rates.total(), err);
-        double const tau = density_path(iv, path, path.in_begin, path.in_end) / mfp;
+        double const rate = rate_from_inverse(rates.total(), err);
+        double const tau = density_path(iv, path, path.in_begin, path.in_end) * rate;
         Selection const sel =
             select_hazard(arena, tau, 0.0, 0.0, 1, rng.uniform(idx, kChNewbornCompetingOpticalDepth),
                           []() { return 0.0; });
@@ -647,7 +647,7 @@ __device__ int advance_photon_newborn(StepConstants const& C, ElectronArgs const
             p.birth_fraction = 1.0;
             return 1;
         }
-        double const f = fraction_at_density_path(iv, path, path.in_begin, path.in_end, sel.sampled * mfp, err);
+        double const f = fraction_at_density_path(iv, path, path.in_begin, path.in_end, sel.sampled / rate, err);
         if (!(finite_bits(f) && f >= path.in_begin && f <= path.in_end && path.in_end > path.in_begin)) {
             err.set(RREA_GPU_ERR_INVALID_STATE);
             return -1;
@@ -722,7 +722,7 @@ __device__ int advance_photon_newborn(StepConstants const& C, ElectronArgs const
                     err.set(RREA_GPU_ERR_RANGE);
                     return -1;
                 }
-                double const cth = sample_photoelectron_cos(ee, rng.uniform(idx, kChPhotoelectronCos));
+                double const cth = sample_photoelectron_cos(arena, ee, rng.uniform(idx, kChPhotoelectronCos));
                 double sx, sy, sz;
                 cone_direction(arena, dx, dy, dz, cth, rng.uniform(idx, kChPhotoelectronAzimuth), sx, sy, sz);
                 child(0, 6, px, py, pz, sx, sy, sz, ee, b);

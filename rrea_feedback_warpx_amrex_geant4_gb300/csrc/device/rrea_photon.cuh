@@ -62,8 +62,8 @@ __device__ __forceinline__ double wrap_unit(double v)
 
 // Photon coefficients at one energy: Compton, photoelectric, pair (nuclear),
 // pair (triplet) inverse lengths at STP (S/RreaInteractionTables.cpp:
-// 2272-2296).  The four tables share one energy grid in the schema-6 bundle,
-// so a single bracket serves all four.
+// 2272-2296), from one row of interval polynomials; a flagged row (an energy
+// between two nodes within 1e-9 of one another) interpolates as the reference.
 struct PhotonRates {
     double compton, pe, nuclear, triplet;
     __device__ __forceinline__ double total() const { return compton + pe + nuclear + triplet; }
@@ -76,19 +76,19 @@ __device__ __forceinline__ bool photon_rates(StepConstants const& C, const doubl
         err.set(RREA_GPU_ERR_RANGE);
         return false;
     }
-    if (ix.photon_grid_shared) {
-        Bracket b;
-        if (!bracket_hot(arena, ix.hot[RREA_T_PH_COMPTON], e, b, err)) return false;
-        r.compton = eval_hot(arena, ix.hot[RREA_T_PH_COMPTON], b, err);
-        r.pe = eval_hot(arena, ix.hot[RREA_T_PH_PHOTOELECTRIC], b, err);
-        r.nuclear = eval_hot(arena, ix.hot[RREA_T_PH_PAIR_NUCLEAR], b, err);
-        r.triplet = eval_hot(arena, ix.hot[RREA_T_PH_PAIR_TRIPLET], b, err);
-    } else {
-        r.compton = interpolate(arena, ix.hot[RREA_T_PH_COMPTON], e, err);
-        r.pe = interpolate(arena, ix.hot[RREA_T_PH_PHOTOELECTRIC], e, err);
-        r.nuclear = interpolate(arena, ix.hot[RREA_T_PH_PAIR_NUCLEAR], e, err);
-        r.triplet = interpolate(arena, ix.hot[RREA_T_PH_PAIR_TRIPLET], e, err);
+    RowHit h;
+    if (find_row(arena, ix.photon_rows, e, h) && row_flags(h) == 0U) {
+        // a linear piece that starts at a zero node may round below it
+        r.compton = max0(row_value(h, 0));
+        r.pe = max0(row_value(h, 1));
+        r.nuclear = max0(row_value(h, 2));
+        r.triplet = max0(row_value(h, 3));
+        return true;
     }
+    r.compton = interpolate(arena, ix.hot[RREA_T_PH_COMPTON], e, err);
+    r.pe = interpolate(arena, ix.hot[RREA_T_PH_PHOTOELECTRIC], e, err);
+    r.nuclear = interpolate(arena, ix.hot[RREA_T_PH_PAIR_NUCLEAR], e, err);
+    r.triplet = interpolate(arena, ix.hot[RREA_T_PH_PAIR_TRIPLET], e, err);
     return err.code == 0;
 }
 
@@ -187,28 +187,30 @@ __device__ __forceinline__ void sample_photoelectric(StepConstants const& C, con
     electron = max0(e - bnd);
 }
 
-// SamplePhotoelectronCosTheta, S/RreaInteractionTables.cpp:2949-3044:
-// Sauter-Gavrila angle by bisection of the closed-form CDF in t = 1 - beta
-// cos(theta).  The reference evaluates in long double; its primitive
+// SamplePhotoelectronCosTheta, S/RreaInteractionTables.cpp:2949-3044: the
+// Sauter-Gavrila angle as the root of the closed-form CDF in t = 1 - beta
+// cos(theta), which the reference bisects in long double.  The primitive
 //   P(x) = -c/(3x^3) - (2+bc)/(2x^2) - (2b-1)/x - b log x
 // cancels heavily at low energy (the density is O(gamma-1) while the terms
-// are O(1)), which costs plain FP64 up to 1e-11 in cos(theta).  Here the
-// bisection runs on doubles and each comparison P(mid) < target is decided
-// in FP64 when the FP64 value clears a rigorous error bound, and in
-// double-double otherwise (Ziv's strategy), so every decision is the exact
-// one; the answer is then within one bisection ulp of the exact root.
-__device__ __forceinline__ dd sg_prim_dd(dd b, dd c, dd twopbc, dd twobm1, double x)
+// are O(1)), which costs plain FP64 up to 1e-11 in cos(theta).  Here Newton
+// steps, kept inside the bracket by halving it, use the FP64 value while it
+// clears a bound on its error, and the double-double one from there on
+// (Ziv's strategy), so every side of the bracket is the exact one; a step
+// from a double-double value below half an ulp ends the search.  One lane in
+// many thousand comes here and its warp, often the launch, waits for it: a
+// step of 4,000 photons with one such event takes 0.25 ms, 0.85 with a
+// bisection.
+__device__ __forceinline__ dd sg_prim_dd(dd b, dd c3, dd halfpbc, dd twobm1, double x)
 {
-    dd const X = dd_from(x);
-    dd const x2 = two_prod(x, x);
-    dd const x3 = dd_mul_d(x2, x);
-    dd const t1 = dd_neg(dd_div(c, dd_mul_d(x3, 3.0)));
-    dd const t2 = dd_neg(dd_div(twopbc, dd_mul_d(x2, 2.0)));
-    dd const t3 = dd_neg(dd_div(twobm1, X));
-    dd const t4 = dd_neg(dd_mul(b, dd_log(X)));
+    dd const i1 = dd_div(dd_from(1.0), dd_from(x));
+    dd const i2 = dd_mul(i1, i1);
+    dd const t1 = dd_neg(dd_mul(c3, dd_mul(i2, i1)));
+    dd const t2 = dd_neg(dd_mul(halfpbc, i2));
+    dd const t3 = dd_neg(dd_mul(twobm1, i1));
+    dd const t4 = dd_neg(dd_mul(b, dd_log(dd_from(x))));
     return dd_add(dd_add(dd_add(t1, t2), t3), t4);
 }
-static __device__ __noinline__ double sample_photoelectron_cos(double k, double draw)
+static __device__ __noinline__ double sample_photoelectron_cos(const double* __restrict__ arena, double k, double draw)
 {
     double const u = clamp_unit(draw);
     if (le0(u)) return -1.0;
@@ -233,38 +235,54 @@ static __device__ __noinline__ double sample_photoelectron_cos(double k, double 
     dd const c = dd_neg(inv_g2);
     dd const twopbc = dd_add(dd_from(2.0), dd_mul(b, c));
     dd const twobm1 = dd_sub(dd_mul_d(b, 2.0), dd_from(1.0));
+    dd const c3 = dd_div(c, dd_from(3.0)), halfpbc = dd_mul_d(twopbc, 0.5);
     dd const one_p_beta = dd_add(dd_from(1.0), beta);
     dd const t_lo = dd_div(inv_g2, one_p_beta);
     dd const t_hi = one_p_beta;
     // the end points as doubles (the bisection variable)
-    dd const f_lo = sg_prim_dd(b, c, twopbc, twobm1, t_lo.hi);
-    dd const f_hi = sg_prim_dd(b, c, twopbc, twobm1, t_hi.hi);
+    dd const f_lo = sg_prim_dd(b, c3, halfpbc, twobm1, t_lo.hi);
+    dd const f_hi = sg_prim_dd(b, c3, halfpbc, twobm1, t_hi.hi);
     dd const total = dd_sub(f_hi, f_lo);
     if (!(gt0(total.hi)) || !finite_bits(total.hi)) return __longlong_as_double(0x7ff8000000000000LL);
     dd const target = dd_add(dd_mul(two_sum(1.0, -u), f_hi), dd_mul_d(f_lo, u));
     double const bd = b.hi, cd = c.hi, pbd = twopbc.hi, bm1d = twobm1.hi, tgt = target.hi;
     double lo = t_lo.hi, hi = t_hi.hi;
+    double tt = sqrt(lo * hi);
 #pragma unroll 1
     for (int it = 0; it < 128; ++it) {
-        double const mid = 0.5 * (lo + hi);
-        if (mid == lo || mid == hi) break;
+        // t between the ends: a step's target, else the middle (of the
+        // logarithms while the ends are far apart)
+        if (!(tt > lo && tt < hi)) tt = hi > 4.0 * lo ? sqrt(lo * hi) : 0.5 * (lo + hi);
+        if (!(tt > lo && tt < hi)) {
+            tt = 0.5 * (lo + hi);
+            break;
+        }
         // FP64 value with a bound on its error: every term carries at most a
-        // few roundings (and the libm log one ulp), so 32 eps of the summed
+        // few roundings (and the logarithm two ulps), so 32 eps of the summed
         // magnitudes covers them with margin.
-        double const m2 = mid * mid;
-        double const t1 = -cd / (3.0 * m2 * mid);
-        double const t2 = -pbd / (2.0 * m2);
-        double const t3 = -bm1d / mid;
-        double const t4 = -bd * log(mid);
-        double const p = ((t1 + t2) + t3) + t4;
+        double const i1 = 1.0 / tt, i2 = i1 * i1;
+        double const t1 = cd * (i1 * i2) * (-1.0 / 3.0);
+        double const t2 = -0.5 * pbd * i2;
+        double const t3 = -bm1d * i1;
+        double const t4 = -bd * flog(arena, tt);
+        double diff = (((t1 + t2) + t3) + t4) - tgt;
         double const bound = 32.0 * kEps * (fabs(t1) + fabs(t2) + fabs(t3) + fabs(t4) + fabs(tgt));
-        bool below;
-        if (p - tgt < -bound) below = true;
-        else if (p - tgt > bound) below = false;
-        else below = dd_lt(sg_prim_dd(b, c, twopbc, twobm1, mid), target);
-        if (below) lo = mid; else hi = mid;
+        bool const settled = fabs(diff) > bound;
+        bool below = diff < 0.0;
+        if (!settled) {
+            dd const d = dd_sub(sg_prim_dd(b, c3, halfpbc, twobm1, tt), target);
+            diff = d.hi;
+            below = d.hi < 0.0 || (d.hi == 0.0 && d.lo < 0.0);
+        }
+        if (below) lo = tt; else hi = tt;
+        double const slope = i1 * fma(i1, fma(i1, fma(i1, cd, pbd), bm1d), -bd);
+        double const step = diff / slope;
+        if (!settled && fabs(step) <= 0.5 * kEps * tt) {
+            tt -= step;
+            break;
+        }
+        tt -= step;
     }
-    double const tt = 0.5 * (lo + hi);
     dd const cosv = dd_div(dd_sub(dd_from(1.0), dd_from(tt)), beta);
     return fmax(-1.0, fmin(1.0, cosv.hi));
 }
@@ -515,6 +533,76 @@ __device__ __forceinline__ void rotate_to_axis(double ax, double ay, double az, 
     normalize(ox, oy, oz);
 }
 
+// The photon's chord over the step.  True when it lies strictly inside an
+// absorbing domain: no face, no escape.
+template <int NP>
+__device__ __forceinline__ bool photon_chord(StepConstants const& C, ElectronArgs const& A, Geom const& g, int64_t ip,
+                                             double ux, double uy, double uz, double inv_u, Path<NP>& path, Err& err)
+{
+    const double* __restrict__ arena = A.arena;
+    double const pr0 = A.prev_r[ip], pz0 = A.prev_z[ip], pth0 = A.prev_theta[ip];
+    if (!A.straight_push) {
+        clip_rz(arena, pr0, pth0, pz0, A.r[ip], A.theta[ip], A.z[ip], g, path, err);
+        return false;
+    }
+    // WarpX's photon push (x += c dt u/|u|) on the Cartesian image of the
+    // RZ start point; the tile arrays alias prev_* in this mode.  The
+    // chord is clipped between its Cartesian ends (as clip_xyz).
+    double const f = kC * C.dt_s * inv_u;
+    double s0 = 0.0, c0 = 1.0;
+    bool const finite = finite_bits(pth0);
+    if (finite) fsincos(arena, pth0, s0, c0);
+    double const x0 = pr0 * c0, y0 = pr0 * s0;
+    double const x1 = x0 + ux * f, y1 = y0 + uy * f, z1 = pz0 + uz * f;
+    if (finite && !lt0(pr0) && clip_inside(x0, y0, pz0, pr0 * pr0, x1, y1, z1, fma(x1, x1, y1 * y1), g, path)) {
+        return true;
+    }
+    Path<NP> out;   // the out-of-line call's, so that path stays in registers
+    Err e;
+    clip_chord(x0, y0, pz0, pr0, x1, y1, z1, rz_radius(x1, y1), finite, g, out, e);
+    path = out;
+    if (e.code) err.set(e.code);
+    return false;
+}
+
+// The common flight: a chord inside the domain without an interaction.  One
+// photon in some hundred meets one per step, and its warp ran the samplers
+// with one lane (290 FP64 slots per warp where a photon's own flight takes
+// 140).  True when the photon is written back; false, with nothing written,
+// when the full loop must take it (an interaction, a face, an error).
+__device__ __forceinline__ bool fly_photon(StepConstants const& C, ElectronArgs const& A, int64_t ip)
+{
+    Geom const g = make_geom(C);
+    double const ux = A.ux[ip], uy = A.uy[ip], uz = A.uz[ip];
+    double const u2 = ux * ux + uy * uy + uz * uz;
+    if (!gt0(u2) || le0(A.w[ip])) return false;
+    double const inv_u = frsqrt(u2);
+    double energy = u2 * inv_u;
+    energy = fma(0.5 * inv_u, fma(-energy, energy, u2), energy);
+    if (energy < C.photon_cutoff_eV) return false;
+    Err err;
+    Path<1> path;
+    if (!photon_chord(C, A, g, ip, ux, uy, uz, inv_u, path, err)) return false;
+    Intervals<1> iv;
+    build_intervals(path, g, A.prof, C.density_ratio, iv, err);
+    PhotonRates rates;
+    if (!photon_rates(C, A.arena, energy, rates, err)) return false;
+    double const tau = density_path(iv, path, path.in_begin, path.in_end) * rate_from_inverse(rates.total(), err);
+    uint64_t idx;
+    if (err.code || !finite_bits(tau) || lt0(tau) || !live_hazard_index(2, 0, 0, idx)) return false;
+    RngStream rng;
+    rng.init(C.cfg.rng_seed, static_cast<uint64_t>(llabs(A.id[ip])) ^ (static_cast<uint64_t>(A.cpu ? A.cpu[ip] : 0) << 40),
+             C.step_key);
+    // (select_hazard's test: no event whatever the roundings)
+    if (!(__double2hiint(rng.uniform(idx, kChPhotonOpticalDepth)) > max(__double2hiint(tau) + 1, 0x3e100000))) return false;
+    double x, y, z;
+    point_at_full(path, g, path.in_end, x, y, z);
+    A.r[ip] = rz_radius(x, y);
+    A.theta[ip] = fatan2(A.arena, y, x);
+    A.z[ip] = z;
+    return true;
+}
+
 // Photon tile: (r, theta, z) is the pusher's end point, prev_* the start;
 // (ux, uy, uz) is the photon momentum in eV.  Returns the disposition
 // (0 survive, 1 escape, 2 absorbed, -1 error) and the hazard draws made.
@@ -534,9 +622,11 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
     uint64_t const key = static_cast<uint64_t>(llabs(A.id[ip])) ^ (static_cast<uint64_t>(A.cpu ? A.cpu[ip] : 0) << 40);
     double const weight = A.w[ip];
     double ux = A.ux[ip], uy = A.uy[ip], uz = A.uz[ip];
-    double energy = sqrt(ux * ux + uy * uy + uz * uz);
-    double dx = ux, dy = uy, dz = uz;
-    normalize(dx, dy, dz);
+    double const u2 = ux * ux + uy * uy + uz * uz;
+    double const inv_u = gt0(u2) ? frsqrt(u2) : 0.0;
+    double energy = u2 * inv_u;
+    energy = fma(0.5 * inv_u, fma(-energy, energy, u2), energy);   // the square root to half an ulp
+    double dx = ux * inv_u, dy = uy * inv_u, dz = gt0(u2) ? uz * inv_u : 1.0;
     double const pr0 = A.prev_r[ip], pz0 = A.prev_z[ip];
     if (pr0 > cfg.r_hi + 1.0e-9 * cfg.r_hi || pz0 < cfg.z_lo - 1.0e-9 || pz0 > cfg.z_hi + 1.0e-9 * cfg.z_hi) {
         err.set(RREA_GPU_ERR_GEOMETRY);
@@ -544,25 +634,8 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
     }
     RngStream rng;
     rng.init(cfg.rng_seed, key, C.step_key);
-    double const pth0 = A.prev_theta[ip];
-    double r1, th1, z1;
-    if (A.straight_push) {
-        // WarpX's photon push (x += c dt u/|u|) on the Cartesian image of the
-        // RZ start point; the tile arrays alias prev_* in this mode.
-        double const f = gt0(energy) ? kC * dt_s / energy : 0.0;
-        double s0, c0;
-        sincos(pth0, &s0, &c0);
-        double const x1 = pr0 * c0 + ux * f, y1 = pr0 * s0 + uy * f;
-        z1 = pz0 + uz * f;
-        r1 = rz_radius(x1, y1);
-        th1 = atan2(y1, x1);
-    } else {
-        r1 = A.r[ip];
-        th1 = A.theta[ip];
-        z1 = A.z[ip];
-    }
     Path<NP> path;
-    clip_rz(pr0, pth0, pz0, r1, th1, z1, g, path, err);
+    bool inside = photon_chord(C, A, g, ip, ux, uy, uz, inv_u, path, err);
     if (err.code) return -1;
 
     int process = 0;
@@ -585,8 +658,8 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
             err.set(RREA_GPU_ERR_RNG_OVERFLOW);
             return -1;
         }
-        bool esc, esc_inv;
-        clipped_escape_policy(path, g, rz_radius(path.ex, path.ey), path.ez, esc, esc_inv);
+        bool esc = false, esc_inv = false;
+        if (!inside) clipped_escape_policy(path, g, rz_radius(path.ex, path.ey), path.ez, esc, esc_inv);
         double const ds = path.in_length;
         Intervals<NP> iv;
         build_intervals(path, g, A.prof, rho, iv, err);
@@ -603,7 +676,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
             double x, y, z;
             point_at_full(path, g, path.in_end, x, y, z);
             A.r[ip] = rz_radius(x, y);
-            A.theta[ip] = atan2(y, x);
+            A.theta[ip] = fatan2(arena, y, x);
             A.z[ip] = wrap_z(g, z);
             if (!esc) return 0;
             if (esc_inv) A.id[ip] = -A.id[ip];
@@ -612,8 +685,8 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
         if (le0(ds)) return commit_no_event();
         PhotonRates rates;
         if (!photon_rates(C, arena, energy, rates, err)) return -1;
-        double const mfp = mfp_from_inverse(rates.total(), err);
-        double const tau = chord_dpath / mfp;
+        double const rate = rate_from_inverse(rates.total(), err);
+        double const tau = chord_dpath * rate;
         uint64_t idx;
         if (!live_hazard_index(2, 0, ordinal, idx)) {
             err.set(RREA_GPU_ERR_RNG_OVERFLOW);
@@ -628,7 +701,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
             return -1;
         }
         if (!sel.event) return commit_no_event();
-        double const f = fraction_at_density_path(iv, path, path.in_begin, path.in_end, sel.sampled * mfp, err);
+        double const f = fraction_at_density_path(iv, path, path.in_begin, path.in_end, sel.sampled / rate, err);
         if (!(finite_bits(f) && f >= path.in_begin && f <= path.in_end && path.in_end > path.in_begin)) {
             err.set(RREA_GPU_ERR_INVALID_STATE);
             return -1;
@@ -690,12 +763,12 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
             A.uz[ip] = energy * dz;
             double const xt = px + dx * remaining, yt = py + dy * remaining, zt = pz + dz * remaining;
             Path<NP> next;
-            clip_xyz(px, py, pz, xt, yt, zt, g, next, err);
+            inside = clip_xyz(px, py, pz, xt, yt, zt, g, next, err);
             if (err.code) return -1;
             double nx, ny, nz;
             point_at_full(next, g, next.in_end, nx, ny, nz);
             A.r[ip] = rz_radius(nx, ny);
-            A.theta[ip] = atan2(ny, nx);
+            A.theta[ip] = fatan2(arena, ny, nx);
             A.z[ip] = wrap_z(g, nz);
             if (!(gt0(remaining))) return 0;
             path = next;
@@ -715,7 +788,7 @@ __device__ __forceinline__ int transport_photon(StepConstants const& C, Electron
                     err.set(RREA_GPU_ERR_RANGE);
                     return -1;
                 }
-                double const cth = sample_photoelectron_cos(ee, rng.uniform(idx, kChPhotoelectronCos));
+                double const cth = sample_photoelectron_cos(arena, ee, rng.uniform(idx, kChPhotoelectronCos));
                 if (!finite_bits(cth)) {
                     err.set(RREA_GPU_ERR_INVALID_STATE);
                     return -1;

@@ -749,6 +749,9 @@ void TableSet::LoadRows()
         cols[RREA_RATE_ANGLE_ENERGY].push_back(fraction(m_index.wentzel[s].e, m_index.wentzel[s].ne));
         push_rows(m_arena, m_index.rate_rows[s], m_index.charged_min_eV, m_index.charged_max_eV, cols);
     }
+    std::vector<std::vector<RowColumn>> photon(RREA_PHOTON_COLUMNS);
+    for (int c = 0; c < RREA_PHOTON_COLUMNS; ++c) photon[c].push_back(table(RREA_T_PH_COMPTON + c));
+    push_rows(m_arena, m_index.photon_rows, m_index.photon_min_eV, m_index.photon_max_eV, photon);
     for (RreaAngleIndex* ai : {&m_index.gs[0], &m_index.gs[1], &m_index.wentzel[0], &m_index.wentzel[1]}) {
         push_rows(m_arena, ai->p_rows, a[ai->p], a[ai->p + ai->np - 1], {{fraction(ai->p, ai->np)}});
         ai->u_rows.span_key = -1;

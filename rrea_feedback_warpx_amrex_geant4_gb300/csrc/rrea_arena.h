@@ -128,6 +128,9 @@ enum RreaRateColumn {
     RREA_RATE_COLUMNS = 7,
 };
 
+// Columns of the photon rows: the tables from RREA_T_PH_COMPTON on, in order.
+enum { RREA_PHOTON_COLUMNS = 4 };
+
 typedef struct {
     int32_t n;
     int32_t pad;
@@ -188,6 +191,7 @@ typedef struct {
     RreaAngleIndex wentzel[2];         // WentzelVI, E > transition
     int64_t hard_moller_mean_secondary;  // on the hard-Moller rate grid
     RreaRowIndex rate_rows[2];         // 0 electron, 1 positron
+    RreaRowIndex photon_rows;
     RreaPhotoelectricIndex pe;
     RreaPairBankIndex pair[2];         // 0 nuclear, 1 triplet
     int64_t total_doubles;

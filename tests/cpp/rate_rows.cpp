@@ -196,6 +196,9 @@ int main(int argc, char** argv)
         }
         check(set, ix.rate_rows[s], cols, true, s == 0 ? "electron rates" : "positron rates");
     }
+    std::vector<std::vector<Column>> photon(RREA_PHOTON_COLUMNS);
+    for (int c = 0; c < RREA_PHOTON_COLUMNS; ++c) photon[c].push_back(table(RREA_T_PH_COMPTON + c));
+    check(set, ix.photon_rows, photon, false, "photon rates");
     for (RreaAngleIndex const* a : {&ix.gs[0], &ix.gs[1], &ix.wentzel[0], &ix.wentzel[1]}) {
         check(set, a->p_rows, {{Column{2, 0, set.at(a->p), nullptr, a->np}}}, true, "path");
         check(set, a->u_rows, {{Column{2, 0, set.at(a->u + 1), nullptr, a->nu - 2}}}, true, "cdf");
