@@ -108,6 +108,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
     double const thr = C.hm_threshold_eV;
     double const rho = C.density_ratio;
     double const w_air = C.tix.w_air_eV_per_pair;
+    double const inv_pair_energy = 1.0 / fmax(w_air, 1.0);
     double const w = p.weight;
     uint64_t const key = p.root_key;
     // an ensemble instance is the root particle's cpu ordinal (key bits 40+)
@@ -181,10 +182,9 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
         return 0;
     }
     if (!(gt0(residual))) return 1;
-    double const u = proper_velocity_from_kinetic(k);
-    double const gam = sqrt(1.0 + u * u / (kC * kC));
     double const residual_dt = C.dt_s * residual;
-    double const chord = (u / gam) * residual_dt;
+    double birth_gb;
+    double const chord = charged_speed(k, birth_gb) * residual_dt;
     if (!(gt0(chord))) return k >= cut ? 1 : 0;
     double const ex0 = p.x + chord * dx, ey0 = p.y + chord * dy, ez0 = p.z + chord * dz;
     Path<NP> path;
@@ -245,11 +245,12 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
         double const ss = frozen_rate(rate_value(C, arena, rc, stop_e, kRateSoft, err, rate_base) * 1.0, err);
         if (err.code) return false;
         double const total = sc + ss;
-        double eff = b;
+        double eff = b, path_m = 0.0;
         bool reaches = false, valid = false;
         if (finite_bits(b) && finite_bits(e) && finite_bits(k) && finite_bits(cut) && e >= b && k >= cut && ge0(cut)) {
             double const to_cut = k - cut;
-            double const req = total * density_path(iv, path, b, e);
+            path_m = density_path(iv, path, b, e);
+            double const req = total * path_m;
             if (finite_bits(req) && ge0(req)) {
                 valid = true;
                 if (req < to_cut) {
@@ -264,6 +265,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
                             reaches = false;
                         }
                     }
+                    path_m = density_path(iv, path, b, eff);
                 }
             }
         }
@@ -271,22 +273,23 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
             err.set(RREA_GPU_ERR_INVALID_STATE);
             return false;
         }
-        double const path_m = density_path(iv, path, b, eff);
         double const raw_col = sc * path_m;
         double const raw_soft = ss * path_m;
         double const avail = max0(k - cut);
         double const drag = reaches ? avail : fmin(raw_col + raw_soft, avail);
         double const col = fmin(raw_col, drag);
-        for (int t = 0; col > 0.0 && gt0(raw_col) && t < iv.n; ++t) {
-            double const bb = fmax(b, iv.begin[t]), ee = fmin(eff, iv.end[t]);
+        for (int t = 0; gt0(col) && gt0(raw_col) && t < iv.n; ++t) {
+            double const bb = NP == 1 ? b : fmax(b, iv.begin[t]), ee = NP == 1 ? eff : fmin(eff, iv.end[t]);
             if (ee > bb) {
                 double const raw = path.full * (ee - bb) * iv.density[t] * sc;
-                double const loss = col * raw / raw_col;
-                double const pw = w * loss / fmax(w_air, 1.0);
+                // with one interval raw is raw_col (the same products), and
+                // col * raw / raw_col is col to within an ulp
+                double const loss = NP == 1 ? col : col * raw / raw_col;
+                double const pw = w * loss * inv_pair_energy;
                 if (gt0(pw)) {
                     double x, y, z;
                     point_at_full(path, g, 0.5 * (bb + ee), x, y, z);
-                    double sr = rz_radius(x, y), sz = z;
+                    double sr = fsqrt(fma(x, x, y * y)), sz = z;
                     // a source that rounds off the half-open domain falls back to the birth point
                     if (!(finite_bits(sr) && finite_bits(sz) && sr >= g.rlo && sr < g.rhi && sz >= g.zlo && sz < g.zhi)) {
                         sr = rz_radius(p.x, p.y);
@@ -518,7 +521,7 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
         {
             double x, y, z;
             point_at_full(path, g, se, x, y, z);
-            if (!in_half_open(g, x, y, z)) {
+            if (!(NP == 1 && strictly_inside(g, fma(x, x, y * y), z)) && !in_half_open(g, x, y, z)) {
                 exited = true;
                 break;
             }

@@ -1354,7 +1354,7 @@ rrea_gpu_status drain_fifo(rrea_gpu_ctx* ctx, int32_t step, double dt_s, int64_t
         a.diag_disposition = nullptr;
         a.segments = ctx->netchord ? ctx->d_seg : nullptr;
         rrea_gpu_secondary* const items = ctx->d_fifo + cursor;
-        RREA_CUDA(ctx, rrea_launch::newborn_step(a, items, chunk, ctx->d_alive, ctx->num_sms * 8, c.periodic_z != 0,
+        RREA_CUDA(ctx, rrea_launch::newborn_step(a, items, chunk, ctx->d_alive, ctx->num_sms, c.periodic_z != 0,
                                                  ctx->stream, ctx->side, ctx->fork_ev, ctx->join_ev));
         if (a.segments) {
             RREA_CUDA(ctx, rrea_launch::netchord_deposit(a.segments, chunk, ctx->net, dt_s, a.status, a.fail_index,

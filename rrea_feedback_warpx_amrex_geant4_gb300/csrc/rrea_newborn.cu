@@ -175,21 +175,23 @@ cudaError_t validate_fifo(const rrea_gpu_secondary* items, int64_t n, int mode, 
 }
 
 cudaError_t newborn_step(rrea_dev::ElectronArgs const& args, rrea_gpu_secondary* items, int64_t n, uint32_t* alive,
-                         int max_blocks, bool periodic, cudaStream_t stream, cudaStream_t const side[2],
+                         int num_sms, bool periodic, cudaStream_t stream, cudaStream_t const side[2],
                          cudaEvent_t fork, cudaEvent_t const join[2])
 {
     using namespace rrea_dev;
     if (n <= 0) return cudaSuccess;
-    // Items per warp: the fewest that two resident waves of the electron
-    // kernel hold.  Most newborns meet a discrete event or their end, so the
-    // lanes of a warp wait for one another's samplers: fewer lanes per warp
-    // shorten the longest warp, which is what a short queue waits for.
-    // Drains of a step's secondaries, items per warp 32 / 8 / 4 / 2 / 1:
-    // 1e4 plain-case electrons 0.94 / 0.74 / 0.68 / 0.66 / 0.69 ms, 6e4
-    // 1.12 / 1.00 / 0.92 / 0.92 / 1.00, 2e5 (16 at its best 1.31) 1.38 / 1.35.
+    // Items per warp: the fewest that leave one warp per scheduler.  Most
+    // newborns meet a discrete event or their end, so the lanes of a warp
+    // wait for one another's samplers: fewer lanes shorten the longest warp,
+    // which is what a short queue waits for, while more warps than schedulers
+    // share their FP64 pipes.  Drains of a scale-up step's secondaries, items
+    // per warp 1 / 2 / 4 / 8 / 16 / 32: 322 items 0.69 / 0.74 / 0.81 / 0.83 ms,
+    // 921 0.77 / 0.76 / 0.81 / 0.93, 3,013 1.21 / 1.05 / 1.05 / 1.09 / 1.23 /
+    // 1.31, 8,937 - / - / 1.47 / 1.41 / 1.34 / 1.36, 17,824 - / - / 2.57 /
+    // 1.92 / 1.75 / 1.60, 62,823 - / - / 12.0 / 8.22 / 3.97 / 2.97.
     int claim = 1;
-    while (claim < 32 && n > static_cast<int64_t>(max_blocks) * 4 * claim) claim *= 2;
-    int const blocks = grid_for((n + claim - 1) / claim * 32, max_blocks);
+    while (claim < 32 && n > static_cast<int64_t>(num_sms) * 4 * claim) claim *= 2;
+    int const blocks = grid_for((n + claim - 1) / claim * 32, num_sms * 8);
     for (int k = 0; k < 3; ++k) note_launch();
     // The species kernels touch disjoint items, so the positron and photon
     // ones run beside the electron one; each is a short wave whose length is

@@ -1,5 +1,5 @@
 """The newborn kernels at the queue lengths where the items per warp change
-(one per warp up to 32 per SM, then doubling) and past the last doubling,
+(one per warp up to 4 per SM, then doubling) and past the last doubling,
 where warps loop: the drain of that many records against the oracle's.
 Tolerances as in test_gpu_newborn.py."""
 import numpy as np
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 SMS = 152
 
 
-@pytest.mark.parametrize("n", [1, 31, 32 * SMS, 32 * SMS + 1, 64 * SMS + 1, 1024 * SMS + 33])
+@pytest.mark.parametrize("n", [1, 31, 4 * SMS, 4 * SMS + 1, 8 * SMS + 1, 128 * SMS + 33, 32 * SMS, 32 * SMS + 1, 64 * SMS + 1, 1024 * SMS + 33])
 def test_drain_lengths_match_oracle(mods, n):  # noqa: F811
     gpu, workloads, oracle, compare = mods
     cfg, ctx, field = _setup(gpu, workloads, "scaleup_c1", 1 << 18)
