@@ -20,14 +20,6 @@
 
 namespace rrea_dev {
 
-// TransportDensityRatioAtZ for a bound profile; NaN outside it.
-static __device__ __noinline__ double lean_density(DensityProfile const& prof, double uniform, double z)
-{
-    Err err;
-    double const v = density_ratio_at_z(prof, uniform, z, err);
-    return err.code ? __longlong_as_double(0x7ff8000000000000LL) : positive_or(v, uniform);
-}
-
 // One electron through the outer step.  True when it is done (survived and
 // written back); false with `rec` filled when the full loop must take over.
 __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronArgs const& A, int64_t ip,
@@ -66,23 +58,6 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
     double const rho = C.density_ratio;
     constexpr uint32_t kRates = 1u << RREA_RATE_COLLISION | 1u << RREA_RATE_SOFT | 1u << RREA_RATE_HARD
         | 1u << RREA_RATE_BREMS;
-    // the two open channels' rates at energy e (competing_rates), row in rc
-    auto channels = [&](double e, double& s0, double& s1) {
-        s0 = C.hm_enabled && gt0(hm_thr) && e > 2.0 * hm_thr ? max0(row_value(rc.hit, RREA_RATE_HARD)) : 0.0;
-        s1 = e > C.photon_cutoff_eV ? max0(row_value(rc.hit, RREA_RATE_BREMS)) : 0.0;
-        // an open channel of rate zero counts as one per 1e99 m
-        if (eq0(s0) && C.hm_enabled && gt0(hm_thr) && e > 2.0 * hm_thr) s0 = 1.0e-99;
-        if (eq0(s1) && e > C.photon_cutoff_eV) s1 = 1.0e-99;
-    };
-    auto density = [&](Path<1> const& p) {
-        return A.prof.n == 0 ? rho : lean_density(A.prof, rho, fma(0.5, p.dz, p.sz));
-    };
-    double gb = 0.0;
-    auto chord = [&](double dt, Path<1>& p) {
-        double const sc = charged_speed(k, gb) * dt;
-        double const ex = fma(sc, dx, run_x), ey = fma(sc, dy, run_y), ez = fma(sc, dz, run_z);
-        return clip_inside<1, true>(run_x, run_y, run_z, 0.0, ex, ey, ez, fma(ex, ex, ey * ey), g, p);
-    };
     // every later chord starts where one that lay inside ended
     if (!strictly_inside(g, fma(run_x, run_x, run_y * run_y), run_z)) return false;
 
@@ -92,12 +67,16 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
     uint32_t subcycles;
     {
         Path<1> path;
-        if (!chord(dt_s, path)) return false;
+        double gb;
+        double const sc = charged_speed(k, gb) * dt_s;
+        double const ex = fma(sc, dx, run_x), ey = fma(sc, dy, run_y), ez = fma(sc, dz, run_z);
+        if (!clip_inside<1, true>(run_x, run_y, run_z, 0.0, ex, ey, ez, fma(ex, ex, ey * ey), g, path)) return false;
         if (!rate_bracket(C, arena, rc, k, err) || row_flags(rc.hit) & (kRates | 1u << RREA_RATE_ELASTIC)) return false;
-        double const dpath = path.full * density(path);
+        double const dpath = path.full
+            * (A.prof.n == 0 ? rho : common_density(A.prof, rho, fma(0.5, path.dz, path.sz)));
         FieldRange const dfw = path_field_work(fv, g, path, q, 0.0, 1.0, err);
-        double s0, s1;
-        channels(k, s0, s1);
+        double s0, s1, s2;
+        common_rates<false>(C, rc, k, s0, s1, s2);
         double const target = cfg.max_optical_depth_per_substep;
         double const by_tau = ceil(((s0 * dpath) + (s1 * dpath)) / target);
         double const gs_n = row_value(rc.hit, RREA_RATE_ELASTIC) * dpath;
@@ -116,103 +95,53 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
     double const pairs_per_eV = weight / fmax(C.tix.w_air_eV_per_pair, 1.0);
     double dpath_sum = 0.0, length_sum = 0.0;
 
-    for (uint32_t sub = 0;; ++sub) {
-        // the state the full loop resumes from
-        rec.k = k;
-        rec.dx = dx;
-        rec.dy = dy;
-        rec.dz = dz;
-        rec.sub = sub;
-        if (sub >= subcycles) break;
+    Running p{run_x, run_y, run_z, dx, dy, dz, k};
+    uint32_t sub = 0;
+    for (; sub < subcycles; ++sub) {
+        uint64_t hazard;
         Path<1> path;
-        bool go = chord(sub_dt, path);
-        double pair_weight = 0.0;
-        if (go) {
-            double const rho_s = density(path);
-            FieldRange const field = path_field_work(fv, g, path, q, 0.0, 1.0, err);
-            half_kick(field, 0.5 * sub_dt, q, gb, k, dx, dy, dz);
-            go = k >= cutoff && rate_bracket(C, arena, rc, k, err) && !(row_flags(rc.hit) & kRates);
-            if (go) {
-                double const dpath = path.full * rho_s;
-                double s0, s1;
-                channels(k, s0, s1);
-                double const tau = s0 * dpath + s1 * dpath;
-                uint64_t index;
-                go = finite_bits(tau) && live_hazard_index(0, sub, 0, index);
-                // (select_hazard's test: no event whatever the roundings)
-                double const u1 = rng.uniform(index, kChElectronCompetingOpticalDepth);
-                go = go && __double2hiint(u1) > max(__double2hiint(tau) + 1, 0x3e100000);
-                // drag to the end of the substep, short of the cutoff
-                double const sc = max0(row_value(rc.hit, RREA_RATE_COLLISION));
-                double const ss = max0(row_value(rc.hit, RREA_RATE_SOFT));
-                double const room = k - cutoff;
-                double const raw = sc * dpath;
-                double const drag = fmin(raw + ss * dpath, room);
-                go = go && (sc + ss) * dpath < room && !err.code;
-                pair_weight = pairs_per_eV * fmin(raw, drag);
-                k -= drag;
-                // elastic deflection, O/RreaTransportStep.H:371-423
-                go = go && rate_bracket(C, arena, rc, k, err) && !(row_flags(rc.hit) >> RREA_RATE_ELASTIC & 1u);
-                if (go) {
-                    double const gs_n = row_value(rc.hit, RREA_RATE_ELASTIC) * dpath;
-                    // (sample_gs_cos' checks; the rows cover the certified energies)
-                    go = gs_n >= C.tix.gs_few_collision_threshold && gs_n < C.tix.gs_isotropic_above_n;
-                    if (go) {
-                        bool const wentzel = !(k <= C.tix.gs_wentzel_transition_eV);
-                        double const ct = sample_gs_angle_rows(
-                            C, arena, rc, wentzel ? C.tix.wentzel[0] : C.tix.gs[0], 0, wentzel ? 1 : 0, k, gs_n,
-                            rng.uniform(static_cast<uint64_t>(sub) << 8, kChElectronGsAngle), err);
-                        double nx, ny, nz;
-                        cone_unit(arena, dx, dy, dz, ct, rng.uniform(static_cast<uint64_t>(sub) << 8, kChElectronGsAzimuth),
-                                  nx, ny, nz);
-                        dx = nx;
-                        dy = ny;
-                        dz = nz;
-                        half_kick(field, 0.5 * sub_dt, q, gamma_beta(k), k, dx, dy, dz);
-                        go = k >= cutoff && !err.code;
-                    }
-                }
-                dpath_sum += go ? dpath : 0.0;
-                length_sum += go ? path.full : 0.0;
-            }
+        double dpath;
+        if (!live_hazard_index(0, sub, 0, hazard)) break;
+        if (!common_substep<false>(C, A, g, fv, rng,
+                                   SubstepDraws{hazard, static_cast<uint64_t>(sub) << 8, kChElectronCompetingOpticalDepth,
+                                                kChElectronGsAngle, kChElectronGsAzimuth},
+                                   sub_dt, pairs_per_eV, ion_pairs, rc, p, path, dpath)) {
+            break;
         }
-        if (!go) break;
-        // the substep stands: its ion pairs and the new position
-        if (gt0(pair_weight)) {
-            double const x = fma(0.5, path.dx, path.sx), y = fma(0.5, path.dy, path.sy);
-            ion_pairs.add(C, A.cells, fsqrt(fma(x, x, y * y)), fma(0.5, path.dz, path.sz),
-                          pair_weight);
-        }
-        run_x = path.sx + path.dx;
-        run_y = path.sy + path.dy;
-        run_z = path.sz + path.dz;
+        dpath_sum += dpath;
+        length_sum += path.full;
     }
     // a low-energy survivor's gate needs the field and the mean drag
-    if (rec.sub == subcycles && k > hm_thr && gt0(hm_thr) && k <= C.tix.charged_max_eV) {
+    if (sub == subcycles && p.k > hm_thr && gt0(hm_thr) && p.k <= C.tix.charged_max_eV) {
         // CommitSurvivorChargedWriteback, O/RreaTransportStep.H:874-905
-        double const um = proper_velocity_from_kinetic(k);
-        double const r = rz_radius(run_x, run_y);
-        A.ux[ip] = um * dx;
-        A.uy[ip] = um * dy;
-        A.uz[ip] = um * dz;
+        double const um = proper_velocity_from_kinetic(p.k);
+        double const r = rz_radius(p.x, p.y);
+        A.ux[ip] = um * p.dx;
+        A.uy[ip] = um * p.dy;
+        A.uz[ip] = um * p.dz;
         A.r[ip] = r;
-        A.theta[ip] = fatan2(arena, run_y, run_x);
-        A.z[ip] = run_z;
+        A.theta[ip] = fatan2(arena, p.y, p.x);
+        A.z[ip] = p.z;
         if (A.segments) {
             SegmentRec& s = A.segments[ip];
             s.a[0] = r0;
             s.a[1] = z0;
             s.a[2] = r;
-            s.a[3] = run_z;
+            s.a[3] = p.z;
             s.a[4] = q * weight;
             s.faces = 0u;
             s.kind = 1;
         }
         return true;
     }
-    rec.x = run_x;
-    rec.y = run_y;
-    rec.z = run_z;
+    rec.x = p.x;
+    rec.y = p.y;
+    rec.z = p.z;
+    rec.dx = p.dx;
+    rec.dy = p.dy;
+    rec.dz = p.dz;
+    rec.k = p.k;
+    rec.sub = sub;
     rec.dpath = dpath_sum;
     rec.length = length_sum;
     return false;

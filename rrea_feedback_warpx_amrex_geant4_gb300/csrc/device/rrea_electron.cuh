@@ -741,6 +741,113 @@ __device__ __noinline__ double cutoff_bisection(Intervals<NP> iv, Path<NP> path,
     return 0.5 * (lo + hi);
 }
 
+// TransportDensityRatioAtZ for a bound profile; NaN outside it.
+static __device__ __noinline__ double common_density(DensityProfile const& prof, double uniform, double z)
+{
+    Err err;
+    double const v = density_ratio_at_z(prof, uniform, z, err);
+    return err.code ? __longlong_as_double(0x7ff8000000000000LL) : positive_or(v, uniform);
+}
+
+// A charged particle between two substeps.
+struct Running {
+    double x, y, z, dx, dy, dz, k;
+};
+
+// The counter-RNG draws of a substep: the first hazard's index and depth
+// channel, the elastic deflection's index and channels.
+struct SubstepDraws {
+    uint64_t hazard, elastic;
+    uint64_t depth, angle, azimuth;
+};
+
+// Rates of the open channels at energy e, its row in rc (competing_rates,
+// competing_rates_positron): an open channel of rate zero counts as one per
+// 1e99 m.
+template <bool POS>
+__device__ __forceinline__ void common_rates(StepConstants const& C, RateCache const& rc, double e, double& s0,
+                                             double& s1, double& s2)
+{
+    double const thr = C.hm_threshold_eV;
+    bool const hard = POS ? !(gt0(thr) && e <= thr) : C.hm_enabled && gt0(thr) && e > 2.0 * thr;
+    bool const brems = e > C.photon_cutoff_eV;
+    s0 = hard ? max0(row_value(rc.hit, RREA_RATE_HARD)) : 0.0;
+    s1 = brems ? max0(row_value(rc.hit, RREA_RATE_BREMS)) : 0.0;
+    s2 = POS ? max0(row_value(rc.hit, RREA_RATE_ANNIHILATION)) : 0.0;
+    if (hard && eq0(s0)) s0 = 1.0e-99;
+    if (brems && eq0(s1)) s1 = 1.0e-99;
+    if (POS && eq0(s2)) s2 = 1.0e-99;
+}
+
+// The common substep: it starts (the caller knows) and ends strictly inside an
+// absorbing domain, draws no event, stays above the cutoff and scatters by the
+// multiple-scattering tables.  Nineteen in twenty are that.  True with p
+// advanced, the ion pairs added and the chord, its density path and the rate
+// row in the references; false with p untouched when the general substep must
+// take it from the same state with the same draws.
+template <bool POS>
+__device__ __forceinline__ bool common_substep(StepConstants const& C, ElectronArgs const& A, Geom const& g,
+                                               FieldView const& fv, RngStream const& rng, SubstepDraws const& draws,
+                                               double sub_dt, double pairs_per_eV, IonPairCache& ion_pairs,
+                                               RateCache& rc, Running& p, Path<1>& path, double& dpath)
+{
+    constexpr double q = POS ? 1.0 : -1.0;
+    constexpr int species = POS ? 1 : 0;
+    constexpr int base = POS ? RREA_T_P_COLLISION : RREA_T_E_COLLISION;
+    constexpr uint32_t rates = 1u << RREA_RATE_COLLISION | 1u << RREA_RATE_SOFT | 1u << RREA_RATE_HARD
+        | 1u << RREA_RATE_BREMS | (POS ? 1u << RREA_RATE_ANNIHILATION : 0u);
+    const double* __restrict__ arena = A.arena;
+    double const cutoff = C.cfg.low_energy_cutoff_eV;
+    double k = p.k, dx = p.dx, dy = p.dy, dz = p.dz;
+    {
+        double gb;
+        double const sc = charged_speed(k, gb) * sub_dt;
+        double const ex = fma(sc, dx, p.x), ey = fma(sc, dy, p.y), ez = fma(sc, dz, p.z);
+        if (!clip_inside<1, true>(p.x, p.y, p.z, 0.0, ex, ey, ez, fma(ex, ex, ey * ey), g, path)) return false;
+        double const rho = A.prof.n == 0 ? C.density_ratio
+                                         : common_density(A.prof, C.density_ratio, fma(0.5, path.dz, path.sz));
+        Err err;
+        FieldRange const field = path_field_work(fv, g, path, q, 0.0, 1.0, err);
+        half_kick(field, 0.5 * sub_dt, q, gb, k, dx, dy, dz);
+        if (!(k >= cutoff) || !rate_bracket(C, arena, rc, k, err, base) || row_flags(rc.hit) & rates) return false;
+        dpath = path.full * rho;
+        double s0, s1, s2;
+        common_rates<POS>(C, rc, k, s0, s1, s2);
+        double const tau = POS ? s0 * dpath + s1 * dpath + s2 * dpath : s0 * dpath + s1 * dpath;
+        // (select_hazard's test: no event whatever the roundings)
+        double const u1 = rng.uniform(draws.hazard, draws.depth);
+        bool go = finite_bits(tau) && __double2hiint(u1) > max(__double2hiint(tau) + 1, 0x3e100000);
+        // drag to the end of the substep, short of the cutoff
+        double const sc_col = max0(row_value(rc.hit, RREA_RATE_COLLISION));
+        double const sc_soft = max0(row_value(rc.hit, RREA_RATE_SOFT));
+        double const room = k - cutoff;
+        double const raw = sc_col * dpath;
+        double const drag = fmin(raw + sc_soft * dpath, room);
+        go = go && (sc_col + sc_soft) * dpath < room && !err.code;
+        k -= drag;
+        // elastic deflection, O/RreaTransportStep.H:371-423
+        if (!go || !rate_bracket(C, arena, rc, k, err, base) || row_flags(rc.hit) >> RREA_RATE_ELASTIC & 1u) return false;
+        double const gs_n = row_value(rc.hit, RREA_RATE_ELASTIC) * dpath;
+        // (sample_gs_cos' checks; the rows cover the certified energies)
+        if (!(gs_n >= C.tix.gs_few_collision_threshold && gs_n < C.tix.gs_isotropic_above_n)) return false;
+        bool const wentzel = !(k <= C.tix.gs_wentzel_transition_eV);
+        double const ct = sample_gs_angle_rows(C, arena, rc, wentzel ? C.tix.wentzel[species] : C.tix.gs[species], species,
+                                               wentzel ? 1 : 0, k, gs_n, rng.uniform(draws.elastic, draws.angle), err);
+        double nx, ny, nz;
+        cone_unit(arena, dx, dy, dz, ct, rng.uniform(draws.elastic, draws.azimuth), nx, ny, nz);
+        half_kick(field, 0.5 * sub_dt, q, gamma_beta(k), k, nx, ny, nz);
+        if (!(k >= cutoff) || err.code) return false;
+        // the substep stands: its ion pairs and the new position
+        double const pairs = pairs_per_eV * fmin(raw, drag);
+        if (gt0(pairs)) {
+            double const x = fma(0.5, path.dx, path.sx), y = fma(0.5, path.dy, path.sy);
+            ion_pairs.add(C, A.cells, fsqrt(fma(x, x, y * y)), fma(0.5, path.dz, path.sz), pairs);
+        }
+        p = Running{path.sx + path.dx, path.sy + path.dy, path.sz + path.dz, nx, ny, nz, k};
+    }
+    return true;
+}
+
 // One charged particle through one outer step.  POS = false is the electron
 // loop (O/RreaElectronTransport.cpp); POS = true the positron loop
 // (O/RreaPositronTransport.cpp:9-878), which shares the substep and event

@@ -335,8 +335,35 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
         }
     };
 
+    bool const common = NP == 1 && (POS || A.n_planes == 0);
     for (uint64_t sub = 0; sub < substeps; ++sub) {
         if (k < cut) break;
+        if constexpr (NP == 1) {
+            uint64_t idx;
+            if (common && strictly_inside(g, fma(run_x, run_x, run_y * run_y), run_z)
+                && pack_transient(true, root_sp, nb_lineage, sub, 0, 0, idx)) {
+                Running now{run_x, run_y, run_z, dx, dy, dz, k};
+                Path<1> chord_path;
+                double dpath;
+                if (common_substep<POS>(C, A, g, fv, rng,
+                                        SubstepDraws{idx, idx, kChNewbornCompetingOpticalDepth,
+                                                     POS ? kChNewbornPositronGsAngle : kChNewbornElectronGsAngle,
+                                                     POS ? kChNewbornPositronGsAzimuth : kChNewbornElectronGsAzimuth},
+                                        sub_dt, w * inv_pair_energy, ion_pairs, rc, now, chord_path, dpath)) {
+                    run_x = now.x;
+                    run_y = now.y;
+                    run_z = now.z;
+                    dx = now.dx;
+                    dy = now.dy;
+                    dz = now.dz;
+                    k = now.k;
+                    path = chord_path;
+                    final_fraction = 1.0;
+                    completed = sub + 1U;
+                    continue;
+                }
+            }
+        }
         double sb, se;
         {
             // RreaBuildRunningChargedChord with the residual dt as the step bound
