@@ -433,9 +433,17 @@ __device__ __forceinline__ void store(double* __restrict__ s, int64_t n, int64_t
     s[5 * n + i] = st.alive ? 1.0 : 0.0;
 }
 
+// Blocks of 64 threads, one particle per thread, registers for eleven blocks
+// per SM: the SMs' shares of 1e5 particles then differ by 7 % where blocks of
+// 128 in a grid of 4 per SM left a fifth of the threads a second particle
+// (forward and reverse of 96 steps: 50.6 ms with those, 48.8 with these; with
+// registers for eight or six blocks, or blocks of 32, 50.3 to 51.7).
+constexpr int kThreads = 64;
+constexpr int kResident = 11;
+
 // Forward over every step: checkpoints ckpt[c] (6 x n each) at the steps
 // c * C; final state and the loss.
-__global__ void forward_kernel(Params p, const double* __restrict__ e, const double* __restrict__ arena,
+__global__ void __launch_bounds__(kThreads, kResident) forward_kernel(Params p, const double* __restrict__ e, const double* __restrict__ arena,
                                const double* __restrict__ seeds, const double* __restrict__ w,
                                const uint64_t* __restrict__ id, double* __restrict__ ckpt,
                                double* __restrict__ final_state, double* __restrict__ partials)
@@ -456,7 +464,7 @@ __global__ void forward_kernel(Params p, const double* __restrict__ e, const dou
                        - p.lambda * (sig((st.z - p.z_p) / p.tau_z) - sig((z_init - p.z_p) / p.tau_z)));
     }
     // the loss is summed in a fixed order (warp tree, the warps of a block
-    // in turn, then the blocks in turn by sum_partials_kernel), so the same
+    // in turn, then the blocks by sum_partials_kernel), so the same
     // nodes give the same loss to the bit and finite differences of the loss
     // carry only its rounding
     __shared__ double warp_sums[32];
@@ -470,24 +478,32 @@ __global__ void forward_kernel(Params p, const double* __restrict__ e, const dou
     }
 }
 
-// The block partials summed in order with Neumaier's compensation, so the
-// loss is the correctly rounded sum of the partials to within an ulp or two
-// and a difference of two losses carries only their final roundings.
+// The block partials summed in a fixed order with Neumaier's compensation (a
+// warp's lanes each over every 32nd, then the lanes in turn), so the loss is the
+// correctly rounded sum of the partials to within an ulp or two and a
+// difference of two losses carries only their final roundings.
 __global__ void sum_partials_kernel(const double* __restrict__ partials, int count, double* loss)
 {
     double s = 0.0, c = 0.0;
-    for (int k = 0; k < count; ++k) {
-        double const x = partials[k];
+    auto add = [&](double x) {
         double const t = s + x;
         c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
         s = t;
+    };
+    for (int k = threadIdx.x; k < count; k += 32) add(partials[k]);
+    for (int lane = 1; lane < 32; ++lane) {
+        double const other = __shfl_sync(0xffffffffu, s, lane), low = __shfl_sync(0xffffffffu, c, lane);
+        if (threadIdx.x == 0) {
+            add(other);
+            c += low;
+        }
     }
-    *loss = s + c;
+    if (threadIdx.x == 0) *loss = s + c;
 }
 
 // Reverse pass over one checkpoint segment [t0, t1): recompute onto the tape
 // (substep inputs, 6 x n per entry), then run the adjoint back through it.
-__global__ void reverse_segment_kernel(Params p, const double* __restrict__ e, const double* __restrict__ arena,
+__global__ void __launch_bounds__(kThreads, kResident) reverse_segment_kernel(Params p, const double* __restrict__ e, const double* __restrict__ arena,
                                        const uint64_t* __restrict__ id, const double* __restrict__ ckpt, int t0,
                                        int t1, double* __restrict__ tape, double* __restrict__ aux,
                                        double* __restrict__ adj, double* __restrict__ grad)
@@ -579,7 +595,7 @@ void adjoint_free(AdjointState* s)
 }
 
 cudaError_t adjoint_stage(AdjointSetup const& in, const double* seeds6, const double* w, const uint64_t* id,
-                          int blocks, AdjointState*& out)
+                          int num_sms, AdjointState*& out)
 {
     adjoint_free(out);
     out = nullptr;
@@ -607,7 +623,8 @@ cudaError_t adjoint_stage(AdjointSetup const& in, const double* seeds6, const do
     p.rows = in.rows;
     p.inv_dz = 1.0 / in.dz_node;
     p.kick = -(rrea_dev::kC * rrea_dev::kInvMeC2) * 0.5 * p.h;
-    s->blocks = blocks;
+    int64_t const want = (in.n + rrea_dev::adj::kThreads - 1) / rrea_dev::adj::kThreads;
+    s->blocks = static_cast<int>(want < 1 ? 1 : want < num_sms * 64 ? want : num_sms * 64);
     int64_t const n = in.n;
     int64_t const n_ckpt = (in.steps + in.ckpt_every - 1) / in.ckpt_every;
     cudaError_t e = cudaSuccess;
@@ -623,7 +640,7 @@ cudaError_t adjoint_stage(AdjointSetup const& in, const double* seeds6, const do
     alloc(&s->aux, static_cast<int64_t>(in.ckpt_every) * in.substeps * rrea_dev::adj::kAux * n);
     alloc(&s->adj, 5 * n);
     alloc(&s->loss, 1);
-    alloc(&s->partials, blocks);
+    alloc(&s->partials, s->blocks);
     alloc(&s->ends, n);
     p.ends = s->ends;
     p.replay = 0;
@@ -647,11 +664,11 @@ cudaError_t adjoint_forward(AdjointState& s, const double* arena, const double* 
     rrea_dev::adj::Params p = s.p;
     p.replay = replay ? 1 : 0;
     note_launch();
-    rrea_dev::adj::forward_kernel<<<s.blocks, 128, 0, stream>>>(p, e_nodes, arena, s.seeds, s.w, s.id, s.ckpt,
+    rrea_dev::adj::forward_kernel<<<s.blocks, rrea_dev::adj::kThreads, 0, stream>>>(p, e_nodes, arena, s.seeds, s.w, s.id, s.ckpt,
                                                                s.final_state, s.partials);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     note_launch();
-    rrea_dev::adj::sum_partials_kernel<<<1, 1, 0, stream>>>(s.partials, s.blocks, s.loss);
+    rrea_dev::adj::sum_partials_kernel<<<1, 32, 0, stream>>>(s.partials, s.blocks, s.loss);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (!replay) s.recorded = true;
     e = cudaMemcpyAsync(&loss, s.loss, sizeof(double), cudaMemcpyDeviceToHost, stream);
@@ -676,7 +693,7 @@ cudaError_t adjoint_backward(AdjointState& s, const double* arena, const double*
         int const t0 = c * p.ckpt_every;
         int const t1 = t0 + p.ckpt_every < p.steps ? t0 + p.ckpt_every : p.steps;
         note_launch();
-        rrea_dev::adj::reverse_segment_kernel<<<s.blocks, 128, shmem, stream>>>(
+        rrea_dev::adj::reverse_segment_kernel<<<s.blocks, rrea_dev::adj::kThreads, shmem, stream>>>(
             p, e_nodes, arena, s.id, s.ckpt + static_cast<int64_t>(c) * 6 * p.n, t0, t1, s.tape, s.aux, s.adj, grad);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }

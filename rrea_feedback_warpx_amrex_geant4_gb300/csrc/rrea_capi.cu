@@ -3039,7 +3039,7 @@ rrea_gpu_status rrea_gpu_adjoint_stage(rrea_gpu_ctx* ctx, const rrea_gpu_adjoint
     in.col = ix.hot[RREA_T_E_COLLISION];
     in.soft = ix.hot[RREA_T_E_SOFT_RAD];
     in.rows = ix.rate_rows[0];
-    RREA_CUDA(ctx, rrea_launch::adjoint_stage(in, seeds.data(), weight, id, ctx->num_sms * 4, ctx->adjoint));
+    RREA_CUDA(ctx, rrea_launch::adjoint_stage(in, seeds.data(), weight, id, ctx->num_sms, ctx->adjoint));
     return RREA_GPU_OK;
 }
 
