@@ -146,9 +146,10 @@ static __device__ __noinline__ double2 drag_power_fallback(Params const& p, cons
     return make_double2(p.rho * total, p.rho * dk);
 }
 
-// rho S(K) and its K-derivative (0 outside the tables, as there).
-template <bool Derivative>
-__device__ __forceinline__ double drag_power(Params const& p, const double* __restrict__ arena, double k, double& dk)
+// rho S(K) and, when asked for, its K-derivative (0 outside the tables, as
+// there).
+__device__ __forceinline__ double drag_power(Params const& p, const double* __restrict__ arena, double k,
+                                             bool derivative, double& dk)
 {
     dk = 0.0;
     RowHit h;
@@ -158,7 +159,7 @@ __device__ __forceinline__ double drag_power(Params const& p, const double* __re
         dk = r.y;
         return r.x;
     }
-    if constexpr (Derivative) dk = p.rho * ((row_slope(h, RREA_RATE_COLLISION) + row_slope(h, RREA_RATE_SOFT)) * h.rec[1]);
+    if (derivative) dk = p.rho * ((row_slope(h, RREA_RATE_COLLISION) + row_slope(h, RREA_RATE_SOFT)) * h.rec[1]);
     return p.rho * (max0(row_value(h, RREA_RATE_COLLISION)) + max0(row_value(h, RREA_RATE_SOFT)));
 }
 
@@ -236,7 +237,7 @@ constexpr int kAux = 7;
 // tape beside the substep's input state.
 __device__ __forceinline__ void substep(Params const& p, const double* __restrict__ e,
                                         const double* __restrict__ arena, uint64_t id, int step, int sub, State& st,
-                                        int32_t& end, double* __restrict__ aux = nullptr, int64_t i = 0)
+                                        int32_t& end, double* __restrict__ aux, int64_t i)
 {
     if (!st.alive) return;
     double const q = -1.0;
@@ -259,7 +260,7 @@ __device__ __forceinline__ void substep(Params const& p, const double* __restric
     double const z1 = st.z + ldz;
     // drag
     double ds;
-    double const sp = aux ? drag_power<true>(p, arena, k1, ds) : drag_power<false>(p, arena, k1, ds);
+    double const sp = drag_power(p, arena, k1, aux != nullptr, ds);
     double const loss = sp * L;
     if (aux) {
         aux[i] = sp;
@@ -442,11 +443,13 @@ constexpr int kThreads = 64;
 constexpr int kResident = 11;
 
 // Forward over every step: checkpoints ckpt[c] (6 x n each) at the steps
-// c * C; final state and the loss.
+// c * C; from step tape_from on the tape of the reverse pass (its entries
+// start there); final state and the loss.
 __global__ void __launch_bounds__(kThreads, kResident) forward_kernel(Params p, const double* __restrict__ e, const double* __restrict__ arena,
                                const double* __restrict__ seeds, const double* __restrict__ w,
                                const uint64_t* __restrict__ id, double* __restrict__ ckpt,
-                               double* __restrict__ final_state, double* __restrict__ partials)
+                               double* __restrict__ final_state, double* __restrict__ partials, int tape_from,
+                               double* __restrict__ tape, double* __restrict__ aux)
 {
     double acc = 0.0;
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < p.n;
@@ -456,7 +459,13 @@ __global__ void __launch_bounds__(kThreads, kResident) forward_kernel(Params p, 
         int32_t end = p.replay ? p.ends[i] : -1;
         for (int t = 0; t < p.steps; ++t) {
             if (t % p.ckpt_every == 0) store(ckpt + static_cast<int64_t>(t / p.ckpt_every) * 6 * p.n, p.n, i, st);
-            for (int q = 0; q < p.substeps; ++q) substep(p, e, arena, id[i], t, q, st, end);
+            for (int q = 0; q < p.substeps; ++q) {
+                // one call for both, so that a taped run takes the steps of an untaped one to the bit
+                bool const taped = t >= tape_from;
+                int64_t const k = static_cast<int64_t>(t - tape_from) * p.substeps + q;
+                if (taped) store(tape + k * 6 * p.n, p.n, i, st);
+                substep(p, e, arena, id[i], t, q, st, end, taped ? aux + k * kAux * p.n : nullptr, i);
+            }
         }
         if (!p.replay) p.ends[i] = end;
         store(final_state, p.n, i, st);
@@ -501,22 +510,46 @@ __global__ void sum_partials_kernel(const double* __restrict__ partials, int cou
     if (threadIdx.x == 0) *loss = s + c;
 }
 
-// Reverse pass over one checkpoint segment [t0, t1): recompute onto the tape
-// (substep inputs, 6 x n per entry), then run the adjoint back through it.
+// tape[0]: whether this reverse pass can use the tape: it is still the forward
+// pass's (tape[1]) and the field nodes are the forward pass's, to the bit.  A
+// pass that cannot overwrites the tape, as does one with segments that need a
+// slot of it (`overwritten`).
+__global__ void tape_usable_kernel(const double* __restrict__ a, const double* __restrict__ b, int n, int overwritten,
+                                   int* tape)
+{
+    __shared__ int differ;
+    if (threadIdx.x == 0) differ = 0;
+    __syncthreads();
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        if (__double_as_longlong(a[k]) != __double_as_longlong(b[k])) differ = 1;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        tape[0] = tape[1] && !differ;
+        if (!tape[0] || overwritten) tape[1] = 0;
+    }
+}
+
+// Reverse pass over one checkpoint segment [t0, t1): unless the forward pass
+// left the segment's tape and it is usable (taped, *taped != 0), recompute onto the tape (substep inputs, 6 x n per entry); then run the
+// adjoint back through it.
 __global__ void __launch_bounds__(kThreads, kResident) reverse_segment_kernel(Params p, const double* __restrict__ e, const double* __restrict__ arena,
                                        const uint64_t* __restrict__ id, const double* __restrict__ ckpt, int t0,
                                        int t1, double* __restrict__ tape, double* __restrict__ aux,
-                                       double* __restrict__ adj, double* __restrict__ grad)
+                                       double* __restrict__ adj, double* __restrict__ grad,
+                                       const int* __restrict__ taped)
 {
     extern __shared__ double g[];
     for (int k = threadIdx.x; k < p.n_nodes; k += blockDim.x) g[k] = 0.0;
     __syncthreads();
     int64_t const entries = static_cast<int64_t>(t1 - t0) * p.substeps;
+    bool const kept = taped && *taped != 0;
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < p.n;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        State st = load(ckpt, p.n, i);
         int32_t end = p.ends[i];
-        for (int t = t0; t < t1; ++t) {
+        State st{};
+        if (!kept) st = load(ckpt, p.n, i);
+        for (int t = t0; t < t1 && !kept; ++t) {
             for (int q = 0; q < p.substeps; ++q) {
                 int64_t const k = static_cast<int64_t>(t - t0) * p.substeps + q;
                 store(tape + k * 6 * p.n, p.n, i, st);
@@ -563,6 +596,10 @@ __global__ void seed_adjoint_kernel(Params p, const double* __restrict__ final_s
 
 namespace rrea_launch {
 
+// Device memory a staged problem's tape may take where it is more than the one
+// segment every reverse pass needs.
+constexpr int64_t kTapeBytes = int64_t{8} << 30;
+
 struct AdjointState {
     rrea_dev::adj::Params p{};
     int64_t cap = 0;
@@ -571,14 +608,20 @@ struct AdjointState {
     uint64_t* id = nullptr;
     double* ckpt = nullptr;    // n_ckpt x 6 x n
     double* final_state = nullptr;
-    double* tape = nullptr;    // C x substeps x 6 x n
-    double* aux = nullptr;     // C x substeps x kAux x n
+    double* tape = nullptr;    // kept x C x substeps x 6 x n
+    double* aux = nullptr;     // kept x C x substeps x kAux x n
+    int kept = 1;              // segments the tape holds, the last ones
+    double* nodes = nullptr;   // field nodes of the last recording forward
+    int* tape_state = nullptr; // tape_usable_kernel's two words
+    bool taped = false;        // the last forward left a tape
     double* adj = nullptr;     // 5 x n
     double* loss = nullptr;
     double* partials = nullptr;   // one loss partial per forward block
     int32_t* ends = nullptr;   // n end records (Params::ends)
     bool recorded = false;     // a recording forward has run
     int blocks = 1;
+    int segments() const { return (p.steps + p.ckpt_every - 1) / p.ckpt_every; }
+    int first_kept() const { return segments() > kept ? segments() - kept : 0; }
 };
 
 void adjoint_free(AdjointState* s)
@@ -586,7 +629,7 @@ void adjoint_free(AdjointState* s)
     if (!s) return;
     for (void* ptr : {static_cast<void*>(s->seeds), static_cast<void*>(s->w), static_cast<void*>(s->id),
                       static_cast<void*>(s->ckpt), static_cast<void*>(s->final_state), static_cast<void*>(s->tape),
-                      static_cast<void*>(s->aux),
+                      static_cast<void*>(s->aux), static_cast<void*>(s->nodes), static_cast<void*>(s->tape_state),
                       static_cast<void*>(s->adj), static_cast<void*>(s->loss), static_cast<void*>(s->partials),
                       static_cast<void*>(s->ends)}) {
         if (ptr) cudaFree(ptr);
@@ -636,8 +679,29 @@ cudaError_t adjoint_stage(AdjointSetup const& in, const double* seeds6, const do
     alloc(&s->id, n);
     alloc(&s->ckpt, n_ckpt * 6 * n);
     alloc(&s->final_state, 6 * n);
-    alloc(&s->tape, static_cast<int64_t>(in.ckpt_every) * in.substeps * 6 * n);
-    alloc(&s->aux, static_cast<int64_t>(in.ckpt_every) * in.substeps * rrea_dev::adj::kAux * n);
+    // The forward pass leaves the tape of the last segments, as many as fit
+    // in kTapeBytes (at least one, which the reverse pass needs for any
+    // other), so that those are not computed a second time: 1e5 electrons
+    // over 96 steps in three segments, forward and reverse
+    // 48.8 to 32.7 ms (an entry is written and read once, 4 GB in all, where
+    // computing it again took a third of the reverse pass).
+    int64_t const entries = static_cast<int64_t>(in.ckpt_every) * in.substeps;
+    int64_t const entry_bytes = (6 + rrea_dev::adj::kAux) * static_cast<int64_t>(sizeof(double)) * (n > 0 ? n : 1);
+    int64_t const fit = kTapeBytes / entry_bytes / entries;
+    s->kept = static_cast<int>(fit < 1 ? 1 : fit < n_ckpt ? fit : n_ckpt);
+    alloc(&s->tape, s->kept * entries * 6 * n);
+    alloc(&s->aux, s->kept * entries * rrea_dev::adj::kAux * n);
+    if (e == cudaErrorMemoryAllocation && s->kept > 1) {
+        cudaGetLastError();
+        if (s->tape) cudaFree(s->tape);
+        s->tape = nullptr;
+        s->kept = 1;
+        e = cudaSuccess;
+        alloc(&s->tape, entries * 6 * n);
+        alloc(&s->aux, entries * rrea_dev::adj::kAux * n);
+    }
+    alloc(&s->nodes, in.n_nodes);
+    alloc(&s->tape_state, 2);
     alloc(&s->adj, 5 * n);
     alloc(&s->loss, 1);
     alloc(&s->partials, s->blocks);
@@ -663,14 +727,23 @@ cudaError_t adjoint_forward(AdjointState& s, const double* arena, const double* 
     cudaError_t e = cudaSuccess;
     rrea_dev::adj::Params p = s.p;
     p.replay = replay ? 1 : 0;
+    // a frozen forward moves the checkpoints but leaves no tape
+    s.taped = false;
+    if (!replay) {
+        e = cudaMemcpyAsync(s.nodes, e_nodes, sizeof(double) * static_cast<size_t>(p.n_nodes), cudaMemcpyDeviceToDevice,
+                            stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(s.tape_state + 1, 1, sizeof(int), stream);
+        if (e != cudaSuccess) return e;
+    }
+    int const tape_from = replay ? p.steps : s.first_kept() * p.ckpt_every;
     note_launch();
-    rrea_dev::adj::forward_kernel<<<s.blocks, rrea_dev::adj::kThreads, 0, stream>>>(p, e_nodes, arena, s.seeds, s.w, s.id, s.ckpt,
-                                                               s.final_state, s.partials);
+    rrea_dev::adj::forward_kernel<<<s.blocks, rrea_dev::adj::kThreads, 0, stream>>>(
+        p, e_nodes, arena, s.seeds, s.w, s.id, s.ckpt, s.final_state, s.partials, tape_from, s.tape, s.aux);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     note_launch();
     rrea_dev::adj::sum_partials_kernel<<<1, 32, 0, stream>>>(s.partials, s.blocks, s.loss);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (!replay) s.recorded = true;
+    if (!replay) s.recorded = s.taped = true;
     e = cudaMemcpyAsync(&loss, s.loss, sizeof(double), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     return e;
@@ -687,14 +760,23 @@ cudaError_t adjoint_backward(AdjointState& s, const double* arena, const double*
     if (e != cudaSuccess) return e;
     note_launch();
     rrea_dev::adj::seed_adjoint_kernel<<<s.blocks, 256, 0, stream>>>(p, s.final_state, s.w, s.adj);
-    int const n_ckpt = (p.steps + p.ckpt_every - 1) / p.ckpt_every;
+    int const n_ckpt = s.segments();
+    if (s.taped) {
+        note_launch();
+        rrea_dev::adj::tape_usable_kernel<<<1, 256, 0, stream>>>(e_nodes, s.nodes, p.n_nodes, s.first_kept() > 0 ? 1 : 0,
+                                                               s.tape_state);
+    }
+    int64_t const entries = static_cast<int64_t>(p.ckpt_every) * p.substeps;
     size_t const shmem = sizeof(double) * static_cast<size_t>(p.n_nodes);
     for (int c = n_ckpt - 1; c >= 0; --c) {
         int const t0 = c * p.ckpt_every;
         int const t1 = t0 + p.ckpt_every < p.steps ? t0 + p.ckpt_every : p.steps;
+        // a segment without a tape takes the first slot: its segment is done by then
+        int64_t const slot = c > s.first_kept() ? c - s.first_kept() : 0;
         note_launch();
         rrea_dev::adj::reverse_segment_kernel<<<s.blocks, rrea_dev::adj::kThreads, shmem, stream>>>(
-            p, e_nodes, arena, s.id, s.ckpt + static_cast<int64_t>(c) * 6 * p.n, t0, t1, s.tape, s.aux, s.adj, grad);
+            p, e_nodes, arena, s.id, s.ckpt + static_cast<int64_t>(c) * 6 * p.n, t0, t1, s.tape + slot * entries * 6 * p.n,
+            s.aux + slot * entries * rrea_dev::adj::kAux * p.n, s.adj, grad, s.taped && c >= s.first_kept() ? s.tape_state : nullptr);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;
