@@ -52,7 +52,6 @@ __device__ __forceinline__ bool ne0(double x) { return (dbits(x) << 1) != 0ull; 
 // fmax(x, 0.0) and fmin(x, 0.0) (a NaN operand gives the zero, as fmax and
 // fmin return the other operand) with the comparison on the integer pipe.
 __device__ __forceinline__ double max0(double x) { return gt0(x) ? x : 0.0; }
-__device__ __forceinline__ double min0(double x) { return lt0(x) ? x : 0.0; }
 
 // Division by a divisor that is reused: one IEEE reciprocal y = RN(1/b),
 // then one product per quotient, q = RN(a*y), within 1.5 ulp of RN(a/b)
@@ -279,20 +278,6 @@ __device__ __forceinline__ double interpolate(const double* __restrict__ arena, 
     Bracket b;
     if (!bracket_hot(arena, h, q, b, err)) return 0.0;
     return eval_hot(arena, h, b, err);
-}
-
-// Whether a hot table is strictly positive at a prepared bracket, without
-// evaluating its exponential: an interior bracket with two positive nodes is
-// exp(finite) > 0 in the log-log modes (node logs are O(10), far from
-// underflow); every other case evaluates the value exactly as eval_hot does.
-__device__ __forceinline__ bool positive_hot(const double* __restrict__ arena, RreaTable1DIndex const& h,
-                                             Bracket& b, Err& err)
-{
-    if (b.kind == 3 && h.mode != RREA_INTERP_LINEAR && h.mode != RREA_INTERP_LOGX_LINEAR) {
-        const double* y = arena + h.y;
-        if (__ldg(y + b.hi - 1) > 0.0 && __ldg(y + b.hi) > 0.0) return true;
-    }
-    return eval_hot(arena, h, b, err) > 0.0;
 }
 
 // S/RreaInteractionTables.cpp:624-648 (interp_semilogx_strict).  `lq`, when

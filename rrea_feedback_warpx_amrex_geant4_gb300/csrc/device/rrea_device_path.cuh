@@ -277,8 +277,8 @@ __device__ __noinline__ void clip_chord(double x0, double y0, double z0, double 
 
 // ClipRz as the reference calls it, on cylindrical ends (r, theta, z).
 template <int NP>
-__device__ __forceinline__ void clip_rz(const double* __restrict__ arena, double r0, double th0, double z0, double r1, double th1, double z1,
-                                        Geom const& g, Path<NP>& p, Err& err)
+__device__ __forceinline__ void clip_rz(const double* __restrict__ arena, double r0, double th0, double z0, double r1,
+                                        double th1, double z1, Geom const& g, Path<NP>& p, Err& err)
 {
     bool const finite = finite_bits(th0) && finite_bits(th1);
     double s0 = 0.0, c0 = 1.0, s1 = 0.0, c1 = 1.0;

@@ -565,44 +565,6 @@ __device__ __forceinline__ bool photon_chord(StepConstants const& C, ElectronArg
     return false;
 }
 
-// The common flight: a chord inside the domain without an interaction.  One
-// photon in some hundred meets one per step, and its warp ran the samplers
-// with one lane (290 FP64 slots per warp where a photon's own flight takes
-// 140).  True when the photon is written back; false, with nothing written,
-// when the full loop must take it (an interaction, a face, an error).
-__device__ __forceinline__ bool fly_photon(StepConstants const& C, ElectronArgs const& A, int64_t ip)
-{
-    Geom const g = make_geom(C);
-    double const ux = A.ux[ip], uy = A.uy[ip], uz = A.uz[ip];
-    double const u2 = ux * ux + uy * uy + uz * uz;
-    if (!gt0(u2) || le0(A.w[ip])) return false;
-    double const inv_u = frsqrt(u2);
-    double energy = u2 * inv_u;
-    energy = fma(0.5 * inv_u, fma(-energy, energy, u2), energy);
-    if (energy < C.photon_cutoff_eV) return false;
-    Err err;
-    Path<1> path;
-    if (!photon_chord(C, A, g, ip, ux, uy, uz, inv_u, path, err)) return false;
-    Intervals<1> iv;
-    build_intervals(path, g, A.prof, C.density_ratio, iv, err);
-    PhotonRates rates;
-    if (!photon_rates(C, A.arena, energy, rates, err)) return false;
-    double const tau = density_path(iv, path, path.in_begin, path.in_end) * rate_from_inverse(rates.total(), err);
-    uint64_t idx;
-    if (err.code || !finite_bits(tau) || lt0(tau) || !live_hazard_index(2, 0, 0, idx)) return false;
-    RngStream rng;
-    rng.init(C.cfg.rng_seed, static_cast<uint64_t>(llabs(A.id[ip])) ^ (static_cast<uint64_t>(A.cpu ? A.cpu[ip] : 0) << 40),
-             C.step_key);
-    // (select_hazard's test: no event whatever the roundings)
-    if (!(__double2hiint(rng.uniform(idx, kChPhotonOpticalDepth)) > max(__double2hiint(tau) + 1, 0x3e100000))) return false;
-    double x, y, z;
-    point_at_full(path, g, path.in_end, x, y, z);
-    A.r[ip] = rz_radius(x, y);
-    A.theta[ip] = fatan2(A.arena, y, x);
-    A.z[ip] = z;
-    return true;
-}
-
 // Photon tile: (r, theta, z) is the pusher's end point, prev_* the start;
 // (ux, uy, uz) is the photon momentum in eV.  Returns the disposition
 // (0 survive, 1 escape, 2 absorbed, -1 error) and the hazard draws made.

@@ -429,7 +429,6 @@ void TableSet::Load(std::string const& config_path)
     };
     m_index.electron_grid_shared = shared(RREA_T_E_COLLISION, RREA_T_E_ELASTIC_TRANSPORT);
     m_index.positron_grid_shared = shared(RREA_T_P_COLLISION, RREA_T_P_ANNIHILATION);
-    m_index.photon_grid_shared = shared(RREA_T_PH_COMPTON, RREA_T_PH_PAIR_TRIPLET);
     // Certified-range coverage (RreaInteractionTables.cpp:1979-2017).
     for (int t = 0; t < RREA_T_COUNT; ++t) {
         RreaTable1DIndex const& h = m_index.hot[t];

@@ -28,8 +28,9 @@
 // it in elementary charges).
 //
 // Forward: one thread per particle, the state checkpointed every C steps.
-// Reverse: per checkpoint segment, last to first, the forward is recomputed
-// from the checkpoint onto a tape of substep inputs (with each substep's
+// Reverse: per checkpoint segment, last to first, from a tape of substep
+// inputs that the forward pass left or, for segments and nodes it did not, that
+// is computed again from the checkpoint (with each substep's
 // stopping power, its derivative and the frozen rotation, so the adjoint
 // evaluates neither tables nor the RNG again), then the adjoint runs back
 // through it.  A substep moves a particle a small part of a node spacing, so

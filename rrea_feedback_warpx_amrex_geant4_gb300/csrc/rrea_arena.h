@@ -204,10 +204,9 @@ typedef struct {
     double gs_isotropic_above_n;
     double gs_wentzel_transition_eV;
     double w_air_eV_per_pair;
-    // 1 when all five electron (six positron, four photon) coefficient tables
-    // share one bit-identical energy grid, so one bracket search serves all.
+    // 1 when all five electron (six positron) coefficient tables share one
+    // bit-identical energy grid.
     int32_t electron_grid_shared;
     int32_t positron_grid_shared;
-    int32_t photon_grid_shared;
     int32_t pad0;
 } RreaArenaIndex;
