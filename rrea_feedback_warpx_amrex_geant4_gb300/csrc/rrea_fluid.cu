@@ -106,6 +106,15 @@ __device__ __forceinline__ double shell_volume(double r_in, double r_out, double
     return kPi * (b * b - a * a) * dz;
 }
 
+// x > 0, isfinite(x) and dmax(x, 0.0), NaN and signed zero as there, on the
+// integer pipe (a comparison holds the FP64 pipe as long as a multiply-add).
+__device__ __forceinline__ bool gt0(double x)
+{
+    return static_cast<u64>(__double_as_longlong(x)) - 1ULL < 0x7ff0000000000000ULL;
+}
+__device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ double dmax0(double x) { return gt0(-x) ? 0.0 : x; }
+
 // MobilityLaw::At (I/LowEnergyFluidState.H:30-41)
 struct Law {
     int reduced;
@@ -117,7 +126,7 @@ struct Law {
 __device__ __forceinline__ double checked_ratio(const double* chi, int64_t k, double scalar)
 {
     double const v = chi ? chi[k] : scalar;
-    if (!isfinite(v) || v <= 0.0) return scalar > 0.0 ? scalar : 1.0;
+    if (!finite(v) || v <= 0.0) return scalar > 0.0 ? scalar : 1.0;
     return v;
 }
 
@@ -139,7 +148,7 @@ __device__ double pair_loss(double a, double b, double alpha, double dt)
         double const ratio = (small / large) * exp(-alpha * delta * dt);
         remaining = ratio >= 1.0 ? small : delta * ratio / (1.0 - ratio);
     }
-    return small - dmin(dmax(remaining, 0.0), small);
+    return small - dmin(dmax0(remaining), small);
 }
 
 struct Grid {
@@ -159,8 +168,9 @@ struct Grid {
 // The kernels are bound by the FP64 pipe (an operation holds it 64 cycles a
 // warp, a division or a root ten operations), so the divisions count: on
 // 256 x 2048 cells, with exact_quot and the closure's rows, closure 235 to
-// 96 us, face flux 240 to 126, react 137 to 112, update 197 to 128; the
-// coupled step 2.78 to 1.94 ms.
+// 96 us, face flux 240 to 126, react 137 to 112, update 197 to 128, the
+// coupled step 2.78 to 1.94 ms; with zero tests on the integer pipe closure
+// 93, face flux 124, react 108, update 124, the coupled step 1.88 ms.
 __device__ __forceinline__ int column() { return blockIdx.x * 32 + threadIdx.x; }
 __device__ __forceinline__ int first_row() { return blockIdx.y * 8 + threadIdx.y; }
 __device__ __forceinline__ int row_stride() { return gridDim.y * 8; }
@@ -191,7 +201,7 @@ __global__ void react_kernel(ReactParams p, double* __restrict__ ne, double* __r
         if (p.table) {
             nu = nu_cell[k];
             double const x = nu * p.dt;
-            if (x >= 0.0 && x < 0.0625) {
+            if (static_cast<u64>(__double_as_longlong(x)) < 0x3fb0000000000000ULL) {   // [0, 1/16)
                 // factor = dt (1 - e^-x) / x by its series (the next term is
                 // below 2^-57) and e^-x = 1 - x (1 - e^-x) / x: 13 FP64 slots
                 // for an exponential, an expm1 and a division (58)
@@ -206,30 +216,30 @@ __global__ void react_kernel(ReactParams p, double* __restrict__ ne, double* __r
                 f = fma(-x, f, 0.5);
                 f = fma(-x, f, 1.0);
                 decay = fma(-x, f, 1.0);
-                factor = nu > 0.0 ? f * p.dt : p.dt;
+                factor = gt0(nu) ? f * p.dt : p.dt;
             } else {
                 decay = exp(-x);
-                factor = nu > 0.0 ? -expm1(-x) / nu : p.dt;
+                factor = gt0(nu) ? -expm1(-x) / nu : p.dt;
             }
         }
-        double const e0 = dmax(ne[k], 0.0);
-        double const p0 = dmax(np[k], 0.0);
-        double const m0 = dmax(nn[k], 0.0);
+        double const e0 = dmax0(ne[k]);
+        double const p0 = dmax0(np[k]);
+        double const m0 = dmax0(nn[k]);
         if (w_rate >= 0) {
             double const att = p.table ? nu_cell[k] : p.nu_const;
             double const r = att + p.max_rate_det + p.a_ei_raw * (e0 + p0) + p.a_ii_raw * (p0 + m0);
             u64 const b = bits(fabs(r));
             rate_max = b > rate_max ? b : rate_max;
         }
-        double const s_low = dmax(se[k], 0.0);
-        double const d_pos = dmax(sp[k], 0.0) * p.dt;
-        double const d_neg = dmax(sn[k], 0.0) * p.dt;
+        double const s_low = dmax0(se[k]);
+        double const d_pos = dmax0(sp[k]) * p.dt;
+        double const d_neg = dmax0(sn[k]) * p.dt;
         double const d_low = s_low * p.dt;
         rho[k] += kQe * (d_pos - d_neg - d_low);
         double const expected = kQe * (p0 + d_pos - m0 - d_neg - e0 - d_low);
-        double const e1 = nu > 0.0 ? e0 * decay + s_low * factor : e0 + d_low;
-        double const attached = dmax(e0 + d_low - e1, 0.0);
-        double e = dmax(e1, 0.0);
+        double const e1 = gt0(nu) ? e0 * decay + s_low * factor : e0 + d_low;
+        double const attached = dmax0(e0 + d_low - e1);
+        double e = dmax0(e1);
         double q = p0 + d_pos;
         double m = m0 + d_neg + attached;
         if (p.det_fraction > 0.0) {
@@ -238,11 +248,11 @@ __global__ void react_kernel(ReactParams p, double* __restrict__ ne, double* __r
             e += freed;
         }
         double const l_ei = pair_loss(e, q, p.a_ei, p.dt);
-        e = dmax(e - l_ei, 0.0);
-        q = dmax(q - l_ei, 0.0);
+        e = dmax0(e - l_ei);
+        q = dmax0(q - l_ei);
         double const l_ii = pair_loss(q, m, p.a_ii, p.dt);
-        q = dmax(q - l_ii, 0.0);
-        m = dmax(m - l_ii, 0.0);
+        q = dmax0(q - l_ii);
+        m = dmax0(m - l_ii);
         ne[k] = e;
         np[k] = q;
         nn[k] = m;
@@ -274,8 +284,8 @@ __global__ void max_rate_kernel(ReactParams p, const double* __restrict__ ne, co
     int64_t const stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < p.n; k += stride) {
         double const att = p.table ? nu_cell[k] : p.nu_const;
-        double const r = att + p.max_rate_det + p.a_ei_raw * (dmax(ne[k], 0.0) + dmax(np[k], 0.0))
-            + p.a_ii_raw * (dmax(np[k], 0.0) + dmax(nn[k], 0.0));
+        double const r = att + p.max_rate_det + p.a_ei_raw * (dmax0(ne[k]) + dmax0(np[k]))
+            + p.a_ii_raw * (dmax0(np[k]) + dmax0(nn[k]));
         u64 const b = bits(fabs(r));
         m = b > m ? b : m;
     }
@@ -292,10 +302,10 @@ __global__ void conductivity_kernel(int64_t n, int electrons, int ions, Law pos,
     for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n; k += stride) {
         double const d = checked_ratio(chi, k, scalar_chi);
         double v = 0.0;
-        if (electrons) v += (mu_cell ? mu_cell[k] : ele.at(d)) * dmax(ne[k], 0.0);
-        if (ions) v += pos.at(d) * dmax(np[k], 0.0) + neg.at(d) * dmax(nn[k], 0.0);
+        if (electrons) v += (mu_cell ? mu_cell[k] : ele.at(d)) * dmax0(ne[k]);
+        if (ions) v += pos.at(d) * dmax0(np[k]) + neg.at(d) * dmax0(nn[k]);
         v *= kQe;
-        double const s = dmax(v, 0.0);
+        double const s = dmax0(v);
         sigma[k] = s;
         tau[k] = s > 0.0 ? kEps0 / s : 1.0e300;
     }
@@ -307,7 +317,7 @@ __global__ void charge_kernel(int64_t n, const double* __restrict__ ne, const do
 {
     int64_t const stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n; k += stride) {
-        double const p = dmax(np[k], 0.0), m = dmax(nn[k], 0.0), e = dmax(ne[k], 0.0);
+        double const p = dmax0(np[k]), m = dmax0(nn[k]), e = dmax0(ne[k]);
         double net = p - m - e;
         if (fabs(net) <= 64.0 * kEps * (p + m + e)) net = 0.0;
         rho[k] = kQe * net;
@@ -378,7 +388,7 @@ __device__ __noinline__ void closure_between(Closure const& t, double en, double
 __device__ __forceinline__ void closure_eval(Closure const& t, double en, int& status, double out[5])
 {
     out[0] = out[1] = out[2] = out[3] = out[4] = 0.0;
-    if (t.n == 0 || !isfinite(en) || en < 0.0) {
+    if (t.n == 0 || !finite(en) || en < 0.0) {
         status = 3;
         return;
     }
@@ -403,7 +413,7 @@ __device__ __forceinline__ void closure_eval(Closure const& t, double en, int& s
     if (find_row(t.arena, t.rows, en, h) && !row_flags(h)) {
 #pragma unroll
         for (int c = 0; c < 5; ++c) out[c] = row_value(h, c);
-        out[1] = dmax(out[1], 0.0);   // nu2 may be linear from a zero node
+        out[1] = dmax0(out[1]);   // nu2 may be linear from a zero node
         return;
     }
     closure_between(t, en, out);
@@ -447,7 +457,7 @@ __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const doubl
         e_mag = fma(0.5 * inv_e, fma(-e_mag, e_mag, e2), e_mag);
         double const ev = ne ? ne[k] : 0.0;
         double const sv = src ? src[k] : 0.0;
-        if (!isfinite(x) || !(x > 0.0) || !isfinite(e_mag) || !isfinite(ev) || !isfinite(sv)) {
+        if (!finite(x) || !(x > 0.0) || !finite(e_mag) || !finite(ev) || !finite(sv)) {
             ++invalid;
             continue;
         }
@@ -463,9 +473,9 @@ __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const doubl
         }
         min_en = bits(en) < min_en ? bits(en) : min_en;
         max_en = bits(en) > max_en ? bits(en) : max_en;
-        double const c = dmax(ev, 0.0) * volume;
+        double const c = dmax0(ev) * volume;
         count += c;
-        source += dmax(sv, 0.0) * volume;
+        source += dmax0(sv) * volume;
         if (status == 1) held_count += c;
         if (mu) mu[k] = exact_quot(co[0], by_x);
         if (nu) nu[k] = co[1] * x + co[2] * x * x;
@@ -506,7 +516,7 @@ __global__ void tensor_check_kernel(int64_t n, const double* __restrict__ d3, u6
         double const rr = d3[k], rz = d3[n + k], zz = d3[2 * n + k];
         double const det = rr * zz - rz * rz;
         double const det_scale = dmax(dmax(fabs(rr * zz), fabs(rz * rz)), 1.0);
-        if (!isfinite(rr) || !isfinite(rz) || !isfinite(zz) || rr < 0.0 || zz < 0.0
+        if (!finite(rr) || !finite(rz) || !finite(zz) || rr < 0.0 || zz < 0.0
             || det < -(512.0 * kEps * det_scale)) {
             bad = 1;
             continue;
@@ -548,7 +558,7 @@ struct TransportParams {
 // below 1e-30 m^-3.
 __device__ __forceinline__ double carrier(const double* __restrict__ old3, int64_t nc, int s, int64_t k)
 {
-    double const v = dmax(old3[s * nc + k], 0.0);
+    double const v = dmax0(old3[s * nc + k]);
     return v > kVacuum ? v : 0.0;
 }
 
@@ -569,9 +579,12 @@ __global__ void face_flux_kernel(TransportParams p, const double* __restrict__ o
     int64_t const nfz = static_cast<int64_t>(nr) * (nz + 1);
     bool const per = g.periodic_z != 0;
     u64 sig_max = 0;
+    // at one density the ions' (and a fixed electron) mobility is the launch's
+    double fixed[3];
+    for (int s = 0; s < 3; ++s) fixed[s] = p.law[s].at(checked_ratio(nullptr, 0, p.scalar_chi));
     auto mobility = [&](int s, int64_t k) {
-        if (s == 2 && p.from_field) return dmax(mu_cell[k], 0.0);
-        return p.law[s].at(checked_ratio(chi, k, p.scalar_chi));
+        if (s == 2 && p.from_field) return dmax0(mu_cell[k]);
+        return chi ? p.law[s].at(checked_ratio(chi, k, p.scalar_chi)) : fixed[s];
     };
     auto tensor = [&](int i, int j, int comp) { return d3[comp * nc + g.cell(i, j)]; };
     auto cd = [&](int i, int j) { return carrier(old3, nc, 2, g.cell(i, j)); };
@@ -634,8 +647,8 @@ __global__ void face_flux_kernel(TransportParams p, const double* __restrict__ o
             double const mu_face = has_lo && has_hi ? 0.5 * (mu_lo + mu_hi) : (has_lo ? mu_lo : mu_hi);
             double const velocity = (s == 0 ? 1.0 : -1.0) * mu_face * e_face;
             double donor = 0.0;
-            if (velocity > 0.0 && has_lo) donor = n_lo;
-            else if (velocity < 0.0 && has_hi) donor = n_hi;
+            if (gt0(velocity) && has_lo) donor = n_lo;
+            else if (gt0(-velocity) && has_hi) donor = n_hi;
             else if (velocity == 0.0 && has_lo && has_hi) donor = 0.5 * (n_lo + n_hi);
             double number_flux = velocity * donor;
             if (s == 2 && p.from_field) {
@@ -705,7 +718,7 @@ __device__ __forceinline__ Metric metric(Grid const& g, int i)
 {
     double const r_lo = g.r_lo + static_cast<double>(i) * g.dr;
     double const r_hi = r_lo + g.dr;
-    return Metric{shell_volume(r_lo, r_lo + g.dr, g.dz), kPi * dmax(r_hi * r_hi - r_lo * r_lo, 0.0),
+    return Metric{shell_volume(r_lo, r_lo + g.dr, g.dz), kPi * dmax0(r_hi * r_hi - r_lo * r_lo),
                   2.0 * kPi * r_lo * g.dz, 2.0 * kPi * r_hi * g.dz};
 }
 
@@ -716,8 +729,8 @@ __device__ __forceinline__ double outgoing(const double* fr, const double* fz, i
     double const f_rhi = fr[s * nfr + i + 1 + static_cast<int64_t>(nr + 1) * j];
     double const f_zlo = fz[s * nfz + i + static_cast<int64_t>(nr) * j];
     double const f_zhi = fz[s * nfz + i + static_cast<int64_t>(nr) * (j + 1)];
-    double o = dmax(f_rhi, 0.0) * m.a_hi + dmax(-f_rlo, 0.0) * m.a_lo;
-    o += (dmax(f_zhi, 0.0) + dmax(-f_zlo, 0.0)) * m.shell;
+    double o = dmax0(f_rhi) * m.a_hi + dmax0(-f_rlo) * m.a_lo;
+    o += (dmax0(f_zhi) + dmax0(-f_zlo)) * m.shell;
     return o;
 }
 
@@ -744,20 +757,20 @@ __global__ void limiter_kernel(TransportParams p, const double* __restrict__ old
                 scale3[s * nc + k] = 1.0;
                 continue;
             }
-            double const density = dmax(old3[s * nc + k], 0.0);
+            double const density = dmax0(old3[s * nc + k]);
             double const out = outgoing(fr, fz, nfr, nfz, g.nr, s, i, j, m);
             // divided out only where it can exceed the largest so far
             double const held = density * dmax(m.volume, 1.0e-300);
-            if (!(density > 0.0 && out < __longlong_as_double(static_cast<long long>(unlimited)) * held * kBelowOne)) {
-                double const rate = density > 0.0 ? out / held : (out > 0.0 ? 1.0e300 : 0.0);
+            if (!(gt0(density) && out < __longlong_as_double(static_cast<long long>(unlimited)) * held * kBelowOne)) {
+                double const rate = gt0(density) ? out / held : (gt0(out) ? 1.0e300 : 0.0);
                 unlimited = bits(rate) > unlimited ? bits(rate) : unlimited;
             }
             double limiter = 1.0;
-            if (out > 0.0) {
+            if (gt0(out)) {
                 // the quotient is at least 1 where its numerator is at least
                 // its denominator
                 double const keep = p.limiter_cfl * density * m.volume, leave = p.dt * out;
-                limiter = density > 0.0 ? (keep >= leave ? 1.0 : dmin(1.0, keep / leave)) : 0.0;
+                limiter = gt0(density) ? (keep >= leave ? 1.0 : dmin(1.0, keep / leave)) : 0.0;
             }
             scale3[s * nc + k] = limiter;
             min_scale = bits(limiter) < min_scale ? bits(limiter) : min_scale;
@@ -801,7 +814,7 @@ __global__ void scale_faces_kernel(TransportParams p, const double* __restrict__
             for (int s = 0; s < 3; ++s) {
                 double x = fr[s * nfr + t];
                 if (x != 0.0) {
-                    int const di = x > 0.0 ? i - 1 : i;
+                    int const di = gt0(x) ? i - 1 : i;
                     x = (di >= 0 && di <= nr - 1) ? x * scale3[s * nc + g.cell(di, j)] : 0.0;
                     fr[s * nfr + t] = x;
                 }
@@ -821,7 +834,7 @@ __global__ void scale_faces_kernel(TransportParams p, const double* __restrict__
             for (int s = 0; s < 3; ++s) {
                 double x = fz[s * nfz + f];
                 if (x != 0.0) {
-                    int const dj = x > 0.0 ? j - 1 : j;
+                    int const dj = gt0(x) ? j - 1 : j;
                     bool const inside = per || (dj >= 0 && dj <= nz - 1);
                     x = inside ? x * scale3[s * nc + g.cell(i, dj)] : 0.0;
                     fz[s * nfz + f] = x;
@@ -874,10 +887,10 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
             double const o = old3[s * nc + k];
             double v = o;
             if (p.enabled[s]) {
-                double const density = dmax(o, 0.0);
-                double out = dmax(fh_r[s], 0.0) * m.a_hi + dmax(-fl_r[s], 0.0) * m.a_lo;
-                out += (dmax(fh_z[s], 0.0) + dmax(-fl_z[s], 0.0)) * m.shell;
-                if (density > 0.0) {
+                double const density = dmax0(o);
+                double out = dmax0(fh_r[s]) * m.a_hi + dmax0(-fl_r[s]) * m.a_lo;
+                out += (dmax0(fh_z[s]) + dmax0(-fl_z[s])) * m.shell;
+                if (gt0(density)) {
                     // divided out only where they can exceed the largest so
                     // far; the fastest face is the one of the largest flux
                     double const held = density * volume.b;
@@ -885,7 +898,7 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
                         double const r = out / held;
                         rate_max = bits(r) > rate_max ? bits(r) : rate_max;
                     }
-                    double const x = dmax(dmax(dmax(-fl_r[s], fh_r[s]), dmax(-fl_z[s], fh_z[s])), 0.0);
+                    double const x = dmax0(dmax(dmax(-fl_r[s], fh_r[s]), dmax(-fl_z[s], fh_z[s])));
                     if (!(x < __longlong_as_double(static_cast<long long>(speed_max)) * density * kBelowOne)) {
                         double const sv = x / density;
                         speed_max = bits(sv) > speed_max ? bits(sv) : speed_max;
@@ -899,7 +912,7 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
                 }
             }
             new3[s * nc + k] = v;
-            if (!isfinite(v)) nonfinite = 1;
+            if (!finite(v)) nonfinite = 1;
             else if (ordered(v) < min_density) min_density = ordered(v);
         }
         double const cr_lo = kQe * (fl_r[0] - fl_r[1] - fl_r[2]);
@@ -910,8 +923,8 @@ __global__ void update_kernel(TransportParams p, const double* __restrict__ old3
         delta += (cz_hi - cz_lo) * m.shell;
         rho[k] -= exact_quot(p.dt * delta, volume);
         // carrier centres of the new state
-        double const pc = dmax(new3[k], 0.0) * m.volume;
-        double const qc = dmax(new3[nc + k], 0.0) * m.volume;
+        double const pc = dmax0(new3[k]) * m.volume;
+        double const qc = dmax0(new3[nc + k]) * m.volume;
         double const rc = g.r_lo + (static_cast<double>(i) + 0.5) * g.dr;
         double const zc = g.z_lo + (static_cast<double>(j) + 0.5) * g.dz;
         double const d = chi ? dmax(chi[k], 1.0e-300) : p.scalar_chi;
