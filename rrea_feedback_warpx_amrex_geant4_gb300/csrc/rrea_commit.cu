@@ -158,7 +158,7 @@ __global__ void cost_hist_kernel(const double* __restrict__ ux, const double* __
 // hist[0, kCostBins) counts, cursor[kCostBins, 2 kCostBins) zeroed slots.
 // A block ranks kCostTile particles in shared memory and takes each bin's
 // slots for all of them with one global atomic: one per particle, on a few
-// dozen addresses, was what bound it (2^21 electrons 0.30 ms; 2^19 now 0.016 ms).
+// dozen addresses, was what bound it (2^21 electrons 0.30 ms, 0.03 now).
 constexpr int kCostThreads = 256, kCostRun = 8, kCostTile = kCostThreads * kCostRun;
 
 __global__ void __launch_bounds__(kCostThreads)
