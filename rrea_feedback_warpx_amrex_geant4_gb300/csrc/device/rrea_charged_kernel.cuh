@@ -23,8 +23,8 @@ __device__ __forceinline__ void charged_step_body(ElectronArgs const& A)
     __shared__ IonPairSlot ion_slots[128];
     IonPairSlot* const my_slot = ion_slots + threadIdx.x;
     unsigned int moved = 0;
-    // the electrons' common-history loop has handled (and counted) the rest
-    bool const resumed = !POS && A.resumed != 0;
+    // the common-history loop has handled (and counted) the rest
+    bool const resumed = A.resumed != 0;
     int64_t const n = resumed ? static_cast<int64_t>(*A.resume_count) : A.n;
     for_each_particle(n, A.work, [&](int64_t i) {
         ResumeRec const* const from = resumed ? A.resume + i : nullptr;

@@ -11,7 +11,8 @@
 // leaves the particle to the full kernel, launched over the records, which
 // repeats the substep from the same state with the same counter-RNG draws.
 // Measured, one resident phase of 2^21 scale-up electrons: 16.7 ms in the
-// full loop, 11.0 ms here (10.1) and in the full loop over the recorded ones;
+// full loop, 11.0 ms here (10.1) and in the full loop over the recorded ones
+// (1.3e5 positrons 1.37 ms, 1.14);
 // the instruction-fetch stalls fall from 63 to 12 % of the issue interval and
 // the FP64 pipe, the bound, is 85 % busy.
 #pragma once
@@ -20,12 +21,16 @@
 
 namespace rrea_dev {
 
-// One electron through the outer step.  True when it is done (survived and
-// written back); false with `rec` filled when the full loop must take over.
+// One electron (POS: positron) through the outer step.  True when it is done
+// (survived and written back); false with `rec` filled when the full loop must
+// take over.
+template <bool POS>
 __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronArgs const& A, int64_t ip,
                                                uint64_t& subcycles_out, IonPairCache& ion_pairs, ResumeRec& rec)
 {
-    constexpr double q = -1.0;
+    constexpr double q = POS ? 1.0 : -1.0;
+    constexpr int species = POS ? 1 : 0;
+    constexpr int base = POS ? RREA_T_P_COLLISION : RREA_T_E_COLLISION;
     const double* __restrict__ arena = A.arena;
     rrea_gpu_config const& cfg = C.cfg;
     Geom const g = make_geom(C);
@@ -57,11 +62,12 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
     Err err;
     double const rho = C.density_ratio;
     constexpr uint32_t kRates = 1u << RREA_RATE_COLLISION | 1u << RREA_RATE_SOFT | 1u << RREA_RATE_HARD
-        | 1u << RREA_RATE_BREMS;
+        | 1u << RREA_RATE_BREMS | (POS ? 1u << RREA_RATE_ANNIHILATION : 0u);
     // every later chord starts where one that lay inside ended
     if (!strictly_inside(g, fma(run_x, run_x, run_y * run_y), run_z)) return false;
 
-    // ---- substep count, O/RreaElectronTransport.cpp:187-279, of a chord
+    // ---- substep count, O/RreaElectronTransport.cpp:187-279 and
+    // O/RreaPositronTransport.cpp:168-230, of a chord
     // that lies inside: its uniform slices never exceed the target by more
     // than the reference's tolerance while the count is below a thousand
     uint32_t subcycles;
@@ -71,16 +77,17 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
         double const sc = charged_speed(k, gb) * dt_s;
         double const ex = fma(sc, dx, run_x), ey = fma(sc, dy, run_y), ez = fma(sc, dz, run_z);
         if (!clip_inside<1, true>(run_x, run_y, run_z, 0.0, ex, ey, ez, fma(ex, ex, ey * ey), g, path)) return false;
-        if (!rate_bracket(C, arena, rc, k, err) || row_flags(rc.hit) & (kRates | 1u << RREA_RATE_ELASTIC)) return false;
+        if (!rate_bracket(C, arena, rc, k, err, base) || row_flags(rc.hit) & (kRates | 1u << RREA_RATE_ELASTIC)) return false;
         double const dpath = path.full
             * (A.prof.n == 0 ? rho : common_density(A.prof, rho, fma(0.5, path.dz, path.sz)));
         FieldRange const dfw = path_field_work(fv, g, path, q, 0.0, 1.0, err);
         double s0, s1, s2;
-        common_rates<false>(C, rc, k, s0, s1, s2);
+        common_rates<POS>(C, rc, k, s0, s1, s2);
         double const target = cfg.max_optical_depth_per_substep;
-        double const by_tau = ceil(((s0 * dpath) + (s1 * dpath)) / target);
+        double const by_tau = ceil((POS ? ((s0 + s1) + s2) * dpath : (s0 * dpath) + (s1 * dpath)) / target);
         double const gs_n = row_value(rc.hit, RREA_RATE_ELASTIC) * dpath;
-        double const drag = (max0(row_value(rc.hit, RREA_RATE_COLLISION)) + max0(row_value(rc.hit, RREA_RATE_SOFT))) * dpath;
+        double const col = max0(row_value(rc.hit, RREA_RATE_COLLISION));
+        double const drag = (POS ? col : col + max0(row_value(rc.hit, RREA_RATE_SOFT))) * dpath;
         double const impulse = fmax(cfg.max_field_impulse_fraction * k, fmax(cfg.field_impulse_floor_eV, 1.0));
         double const by_gs =
             ceil(fmin(gs_n, cfg.gs_total_collision_cap) / fmax(cfg.max_gs_collisions_per_substep, 1.0));
@@ -101,18 +108,19 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
         uint64_t hazard;
         Path<1> path;
         double dpath;
-        if (!live_hazard_index(0, sub, 0, hazard)) break;
-        if (!common_substep<false>(C, A, g, fv, rng,
-                                   SubstepDraws{hazard, static_cast<uint64_t>(sub) << 8, kChElectronCompetingOpticalDepth,
-                                                kChElectronGsAngle, kChElectronGsAzimuth},
-                                   sub_dt, pairs_per_eV, ion_pairs, rc, p, path, dpath)) {
+        if (!live_hazard_index(species, sub, 0, hazard)) break;
+        SubstepDraws const draws{hazard, static_cast<uint64_t>(sub) << 8,
+                                 POS ? kChPositronCompetingOpticalDepth : kChElectronCompetingOpticalDepth,
+                                 POS ? kChPositronGsAngle : kChElectronGsAngle,
+                                 POS ? kChPositronGsAzimuth : kChElectronGsAzimuth};
+        if (!common_substep<POS>(C, A, g, fv, rng, draws, sub_dt, pairs_per_eV, ion_pairs, rc, p, path, dpath)) {
             break;
         }
         dpath_sum += dpath;
         length_sum += path.full;
     }
-    // a low-energy survivor's gate needs the field and the mean drag
-    if (sub == subcycles && p.k > hm_thr && gt0(hm_thr) && p.k <= C.tix.charged_max_eV) {
+    // a low-energy electron's gate needs the field and the mean drag
+    if (sub == subcycles && (POS || (p.k > hm_thr && gt0(hm_thr) && p.k <= C.tix.charged_max_eV))) {
         // CommitSurvivorChargedWriteback, O/RreaTransportStep.H:874-905
         double const um = proper_velocity_from_kinetic(p.k);
         double const r = rz_radius(p.x, p.y);
@@ -147,10 +155,10 @@ __device__ __forceinline__ bool transport_lean(StepConstants const& C, ElectronA
     return false;
 }
 
-// The common-history kernel: every valid electron is either finished or
-// recorded in A.resume, in warp-aggregated order.
-template <int MinBlocks>
-__global__ void __launch_bounds__(128, MinBlocks) electron_lean_kernel(const __grid_constant__ ElectronArgs A)
+// The common-history kernels: every valid particle is either finished or
+// recorded in A.resume.
+template <bool POS>
+__device__ __forceinline__ void lean_step_body(ElectronArgs const& A)
 {
     StepConstants const& C = c_step;
     __shared__ IonPairSlot ion_slots[128];
@@ -168,10 +176,10 @@ __global__ void __launch_bounds__(128, MinBlocks) electron_lean_kernel(const __g
         }
         ++moved;
         IonPairCache ion_pairs;
-        ion_pairs.init(my_slot, 0.5 * C.cfg.low_energy_cutoff_eV, C.tix.w_air_eV_per_pair);
+        ion_pairs.init(my_slot, POS ? 0.0 : 0.5 * C.cfg.low_energy_cutoff_eV, C.tix.w_air_eV_per_pair);
         uint64_t sub = 0;
         ResumeRec rec;
-        bool const done = transport_lean(C, A, ip, sub, ion_pairs, rec);
+        bool const done = transport_lean<POS>(C, A, ip, sub, ion_pairs, rec);
         ion_pairs.flush(C, A.cells);
         if (!done) {
             rec.ip = ip;
@@ -184,6 +192,18 @@ __global__ void __launch_bounds__(128, MinBlocks) electron_lean_kernel(const __g
     }, A.order);
     unsigned int const warp_total = __reduce_add_sync(0xffffffffu, moved);
     if ((threadIdx.x & 31) == 0 && warp_total) atomicAdd(A.transported, static_cast<unsigned long long>(warp_total));
+}
+
+template <int MinBlocks>
+__global__ void __launch_bounds__(128, MinBlocks) electron_lean_kernel(const __grid_constant__ ElectronArgs A)
+{
+    lean_step_body<false>(A);
+}
+
+// (1.3e5 positrons: 1.14 ms with 16 resident blocks, 1.15 with 8)
+static __global__ void __launch_bounds__(128, 16) positron_lean_kernel(const __grid_constant__ ElectronArgs A)
+{
+    lean_step_body<true>(A);
 }
 
 }  // namespace rrea_dev

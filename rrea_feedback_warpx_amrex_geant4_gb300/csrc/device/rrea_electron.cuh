@@ -1017,7 +1017,7 @@ __device__ __forceinline__ int transport_charged(StepConstants const& C, Electro
     // ---- substep count, O/RreaElectronTransport.cpp:187-279
     uint64_t subcycles;
     RateCache rc;
-    bool const resume = !POS && from && from->sub != kResumeFromStart;
+    bool const resume = from && from->sub != kResumeFromStart;
     if (resume) {
         subcycles = from->subcycles;
     } else {

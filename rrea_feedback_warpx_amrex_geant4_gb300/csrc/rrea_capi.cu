@@ -33,12 +33,13 @@ constexpr int kSpecies = 3;
 // Chunks of a drop-in phase call whose upload overlaps the compute of the
 // chunks before it, and the tile size from which that pays.
 constexpr int kPhaseChunks = 4;
-// Electron tiles from here on run the common-history loop first.  Its
+// Charged tiles from here on run the common-history loop first.  Its
 // records' launch adds the latency of a full loop at low occupancy, which a
 // small tile does not earn back.  Measured (full loop alone / with the common
 // loop): scale-up electrons 3e4 0.43 / 0.54 ms, 6e4 0.74 / 0.71, 1e5 1.09 /
 // 0.96, 3e5 2.64 / 1.88; the plain case's slower ones 6e4 1.06 / 1.16, 1e5
-// 1.27 / 1.30, 1.5e5 1.63 / 1.58, 3e5 2.78 / 2.33.
+// 1.27 / 1.30, 1.5e5 1.63 / 1.58, 3e5 2.78 / 2.33.  Scale-up positrons 6e4
+// 0.74 / 0.79, 98,304 1.11 / 0.98, 1.3e5 1.37 / 1.14, 6e5 4.67 / 3.39.
 #ifndef RREA_LEAN_MIN_PARTICLES
 #define RREA_LEAN_MIN_PARTICLES (3 << 15)
 #endif
@@ -967,7 +968,8 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         int const fit = warps_per_sm <= 8 ? 2 : warps_per_sm <= 16 ? 4 : warps_per_sm <= 32 ? 8 : 16;
         if (fit < min_blocks) min_blocks = fit;
     }
-    bool const lean = species == RREA_SPECIES_ELECTRON && c.periodic_z == 0 && a.n_planes == 0 && a.n >= kLeanMinParticles;
+    bool const lean = species != RREA_SPECIES_PHOTON && c.periodic_z == 0 && a.n >= kLeanMinParticles
+        && (species == RREA_SPECIES_POSITRON || a.n_planes == 0);   // planes are the electrons'
     RREA_CUDA(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
     if (host && chunks == 1) {
         if (ctx->prefetched[species]) {
@@ -1032,19 +1034,26 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         if (species == RREA_SPECIES_PHOTON) {
             RREA_CUDA(ctx, rrea_launch::photon_step(b, blocks > 0 ? blocks : 1, ctx->launch_threads, c.periodic_z != 0,
                                                     cs));
-        } else if (species == RREA_SPECIES_POSITRON) {
-            RREA_CUDA(ctx, rrea_launch::positron_step(b, blocks > 0 ? blocks : 1, ctx->launch_threads, min_blocks,
-                                                      c.periodic_z != 0, cs));
         } else if (lean) {
             b.resume = ctx->d_resume + off;
             b.resume_count = ctx->d_words->work + 2 * kPhaseChunks + k;
-            RREA_CUDA(ctx, rrea_launch::electron_lean(b, blocks > 0 ? blocks : 1, ctx->launch_threads, ctx->launch_min_blocks, cs));
-            // the rest: about one electron in twenty, so the variant with
-            // registers for a quarter of the SM's threads
-            b.resumed = 1;
-            b.order = nullptr;
-            b.work = ctx->d_words->work + kPhaseChunks + k;
-            RREA_CUDA(ctx, rrea_launch::electron_step(b, ctx->num_sms * 8, 128, 8, false, cs));
+            rrea_dev::ElectronArgs rest = b;
+            rest.resumed = 1;
+            rest.order = nullptr;
+            rest.work = ctx->d_words->work + kPhaseChunks + k;
+            // the rest: about one particle in twenty, so the variant with
+            // registers for a quarter (electrons) or an eighth of the SM's threads
+            if (species == RREA_SPECIES_POSITRON) {
+                RREA_CUDA(ctx, rrea_launch::positron_lean(b, blocks > 0 ? blocks : 1, ctx->launch_threads, cs));
+                RREA_CUDA(ctx, rrea_launch::positron_step(rest, ctx->num_sms * 4, 128, 4, false, cs));
+            } else {
+                RREA_CUDA(ctx, rrea_launch::electron_lean(b, blocks > 0 ? blocks : 1, ctx->launch_threads,
+                                                          ctx->launch_min_blocks, cs));
+                RREA_CUDA(ctx, rrea_launch::electron_step(rest, ctx->num_sms * 8, 128, 8, false, cs));
+            }
+        } else if (species == RREA_SPECIES_POSITRON) {
+            RREA_CUDA(ctx, rrea_launch::positron_step(b, blocks > 0 ? blocks : 1, ctx->launch_threads, min_blocks,
+                                                      c.periodic_z != 0, cs));
         } else {
             RREA_CUDA(ctx, rrea_launch::electron_step(b, blocks > 0 ? blocks : 1, ctx->launch_threads, min_blocks,
                                                       c.periodic_z != 0, cs));

@@ -41,6 +41,7 @@ cudaError_t electron_step(rrea_dev::ElectronArgs const& args, int blocks, int th
 // with args.resumed then runs over the records.
 cudaError_t electron_lean(rrea_dev::ElectronArgs const& args, int blocks, int threads, int min_blocks,
                           cudaStream_t stream);
+cudaError_t positron_lean(rrea_dev::ElectronArgs const& args, int blocks, int threads, cudaStream_t stream);
 // Positron phase (rrea_positron_kernels.cu): its own constant bank, set
 // once per phase before its launches; min_blocks picks the register variant
 // as for electrons (2, 4, 8 or 16 resident 128-thread blocks per SM).

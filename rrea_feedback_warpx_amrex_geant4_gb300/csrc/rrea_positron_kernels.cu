@@ -6,6 +6,7 @@
 #include "rrea_kernels.h"
 
 #include "device/rrea_charged_kernel.cuh"
+#include "device/rrea_charged_lean.cuh"
 
 #include <cuda_runtime.h>
 
@@ -30,6 +31,13 @@ cudaError_t positron_step(rrea_dev::ElectronArgs const& args, int blocks, int th
     case 8: rrea_dev::positron_step_kernel<8, 1><<<blocks, threads, 0, stream>>>(args); break;
     default: rrea_dev::positron_step_kernel<16, 1><<<blocks, threads, 0, stream>>>(args); break;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t positron_lean(rrea_dev::ElectronArgs const& args, int blocks, int threads, cudaStream_t stream)
+{
+    note_launch();
+    rrea_dev::positron_lean_kernel<<<blocks, threads, 0, stream>>>(args);
     return cudaGetLastError();
 }
 
