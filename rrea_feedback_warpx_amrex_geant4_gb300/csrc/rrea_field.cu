@@ -109,11 +109,14 @@ __global__ void __launch_bounds__(256) advance_e_kernel(int nr, int nz, double d
 
 // Rows per thread: up to eight, while the grid still gives every SM its
 // resident threads (below that the rows' serial chain costs more than the
-// reciprocal it saves).
+// reciprocal it saves), and as many as a launch's second dimension needs to
+// reach the last row (65,535 blocks of 8 threads).
 int rows_for(int nr, int nz, int num_threads)
 {
     int64_t const rows = static_cast<int64_t>(nr + 1) * (nz + 1) / num_threads;
-    return static_cast<int>(rows < 1 ? 1 : (rows > 8 ? 8 : rows));
+    int64_t const least = (static_cast<int64_t>(nz) + 65535 * 8) / (65535 * 8);
+    int64_t const good = rows < 1 ? 1 : (rows > 8 ? 8 : rows);
+    return static_cast<int>(good > least ? good : least);
 }
 
 dim3 grid_for(int nr, int nz, int rows)

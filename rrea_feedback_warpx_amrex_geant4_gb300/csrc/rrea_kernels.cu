@@ -196,9 +196,13 @@ cudaError_t set_step_constants(rrea_dev::StepConstants const& c, cudaStream_t st
 cudaError_t field_prep(int nr, int nz, const double* er, const double* ez, const double* amb_er, const double* amb_ez,
                        double* cell_er, double* cell_ez, cudaStream_t stream)
 {
-    // up to four rows per thread while every SM keeps its resident threads
+    // up to four rows per thread while every SM keeps its resident threads,
+    // and as many as a launch's second dimension (65,535 blocks of 8 threads)
+    // needs to reach the last row
     int64_t const fit = static_cast<int64_t>(nr) * nz / (152 * 1024);
-    int const rows = static_cast<int>(fit < 1 ? 1 : (fit > 4 ? 4 : fit));
+    int64_t const least = (static_cast<int64_t>(nz) + 65535 * 8 - 1) / (65535 * 8);
+    int64_t const good = fit < 1 ? 1 : (fit > 4 ? 4 : fit);
+    int const rows = static_cast<int>(good > least ? good : least);
     dim3 const grid(static_cast<unsigned>((nr + 31) / 32), static_cast<unsigned>((nz + 8 * rows - 1) / (8 * rows)));
     note_launch();
     rrea_dev::field_prep_kernel<<<grid, dim3(32, 8), 0, stream>>>(nr, nz, rows, er, ez, amb_er, amb_ez, cell_er,
