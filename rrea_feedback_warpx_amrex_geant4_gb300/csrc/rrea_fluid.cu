@@ -419,6 +419,19 @@ __device__ __forceinline__ void closure_eval(Closure const& t, double en, int& s
     closure_between(t, en, out);
 }
 
+// The square of a magnitude in [2^-511, 2^511), where it neither overflows nor
+// loses its low bits.
+__device__ __forceinline__ bool square_in_range(double v2)
+{
+    return static_cast<uint32_t>(__double2hiint(v2)) - 0x20000000u < 0x3fe00000u;
+}
+// (h, a/h, b/h), h = hypot(a, b), where the square is not.
+__device__ __noinline__ double3 magnitude_any(double a, double b)
+{
+    double const h = hypot(a, b);
+    return h > 0.0 ? make_double3(h, a / h, b / h) : make_double3(h, 0.0, 0.0);
+}
+
 // BuildElectronClosureCellFields (S/LowEnergyFluidFaceTransport.cpp:1034-1243)
 __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const double* __restrict__ chi,
                                const double* __restrict__ er, const double* __restrict__ ez,
@@ -449,12 +462,22 @@ __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const doubl
             by_xn = exact_divisor(x * kNL);
         }
         // |E| and 1/|E| from one inverse root, |E| corrected by its residual
-        // (to half an ulp as hypot is; |E|^2 is far from overflow)
+        // (to half an ulp as hypot is)
         double const e_r = er[k], e_z = ez[k];
         double const e2 = fma(e_r, e_r, e_z * e_z);
-        double const inv_e = e2 > 0.0 ? frsqrt(e2) : 0.0;
-        double e_mag = e2 * inv_e;
-        e_mag = fma(0.5 * inv_e, fma(-e_mag, e_mag, e2), e_mag);
+        double e_mag = 0.0, br = 0.0, bz = 0.0;
+        if (square_in_range(e2)) {
+            double const inv_e = frsqrt(e2);
+            e_mag = e2 * inv_e;
+            e_mag = fma(0.5 * inv_e, fma(-e_mag, e_mag, e2), e_mag);
+            br = e_r * inv_e;
+            bz = e_z * inv_e;
+        } else if (e_r != 0.0 || e_z != 0.0) {
+            double3 const m = magnitude_any(e_r, e_z);
+            e_mag = m.x;
+            br = m.y;
+            bz = m.z;
+        }
         double const ev = ne ? ne[k] : 0.0;
         double const sv = src ? src[k] : 0.0;
         if (!finite(x) || !(x > 0.0) || !finite(e_mag) || !finite(ev) || !finite(sv)) {
@@ -481,7 +504,6 @@ __global__ void closure_kernel(Closure t, Grid g, double scalar_chi, const doubl
         if (nu) nu[k] = co[1] * x + co[2] * x * x;
         if (d3) {
             double const dl = exact_quot(co[3], by_x), dt = exact_quot(co[4], by_x);
-            double const br = e_r * inv_e, bz = e_z * inv_e;
             double const an = dl - dt;
             d3[k] = dt + an * br * br;
             d3[n + k] = an * br * bz;
@@ -522,7 +544,11 @@ __global__ void tensor_check_kernel(int64_t n, const double* __restrict__ d3, u6
             continue;
         }
         double const a = rr - zz, b = 2.0 * rz;
-        double const e = 0.5 * (rr + zz + fsqrt(fma(a, a, b * b)));
+        double const h2 = fma(a, a, b * b);
+        double h = 0.0;
+        if (square_in_range(h2)) h = fsqrt(h2);
+        else if (a != 0.0 || b != 0.0) h = magnitude_any(a, b).x;
+        double const e = 0.5 * (rr + zz + h);
         eig = bits(e) > eig ? bits(e) : eig;
     }
     post_max(words + w_eig, eig);
