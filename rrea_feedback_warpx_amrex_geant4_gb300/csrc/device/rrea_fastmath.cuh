@@ -115,10 +115,13 @@ __device__ __forceinline__ double frsqrt(double x)
     double const e = fma(-(x * y), y, 1.0);
     return fma(y * e, fma(e, 0.375, 0.5), y);
 }
-// sqrt(x) = x / sqrt(x), within two ulps; 0 for 0 (and for anything not positive)
+// sqrt(x) = x / sqrt(x), within two ulps; zeros and arguments outside
+// [2^-100, 2^100] go to CUDA's.
+static __device__ __noinline__ double sqrt_any(double x) { return sqrt(x); }
+
 __device__ __forceinline__ double fsqrt(double x)
 {
-    return __double2hiint(x) > 0 ? x * frsqrt(x) : 0.0;
+    return static_cast<uint32_t>(__double2hiint(x)) - 0x39b00000u > 0x0c800000u ? sqrt_any(x) : x * frsqrt(x);
 }
 
 // sin and cos of the table angle 2 pi j/256 plus r, |r| <= pi/256: sin r and
