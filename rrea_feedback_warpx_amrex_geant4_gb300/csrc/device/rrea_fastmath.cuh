@@ -98,30 +98,44 @@ __device__ __forceinline__ double fexp(const double* __restrict__ arena, double 
 
 // 1/sqrt(x) for the normalisations of the loop: an FP32 seed (relative error
 // below 2^-21) and one third-order Householder step, y (1 + e/2 + 3 e^2/8)
-// with e = 1 - x y^2 (the remainder 5 e^3/16 is below 2^-62), five FP64
-// slots; within an ulp.  Arguments outside [2^-100, 2^100] go to CUDA's.
-static __device__ __noinline__ double rsqrt_any(double x) { return rsqrt(x); }
-
-__device__ __forceinline__ double frsqrt(double x)
+// with e = 1 - x y^2 (the remainder 5 e^3/16 is below 2^-61), five FP64
+// slots.  The square of the seed's 24 bits is exact, so e rounds once and the
+// result is within 0.51 ulp (CUDA's 0.51; 0.98 with x y formed first).
+// Arguments outside [2^-100, 2^100] go to CUDA's.
+__device__ __forceinline__ bool root_in_range(double x)
 {
-    uint32_t const hi = static_cast<uint32_t>(__double2hiint(x));
-    if (hi - 0x39b00000u > 0x0c800000u) return rsqrt_any(x);
-    uint32_t const lo = static_cast<uint32_t>(__double2loint(x));
+    return static_cast<uint32_t>(__double2hiint(x)) - 0x39b00000u <= 0x0c800000u;
+}
+__device__ __forceinline__ double rsqrt_seed(double x)
+{
+    uint32_t const hi = static_cast<uint32_t>(__double2hiint(x)), lo = static_cast<uint32_t>(__double2loint(x));
     float const x32 = __uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29));
     float y32;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y32) : "f"(x32));
     uint32_t const u = __float_as_uint(y32);
-    double const y = __hiloint2double(static_cast<int>((u >> 3) + 0x38000000u), static_cast<int>(u << 29));
-    double const e = fma(-(x * y), y, 1.0);
+    return __hiloint2double(static_cast<int>((u >> 3) + 0x38000000u), static_cast<int>(u << 29));
+}
+static __device__ __noinline__ double rsqrt_any(double x) { return rsqrt(x); }
+
+__device__ __forceinline__ double frsqrt(double x)
+{
+    if (!root_in_range(x)) return rsqrt_any(x);
+    double const y = rsqrt_seed(x);
+    double const e = fma(-x, y * y, 1.0);
     return fma(y * e, fma(e, 0.375, 0.5), y);
 }
-// sqrt(x) = x / sqrt(x), within two ulps; zeros and arguments outside
-// [2^-100, 2^100] go to CUDA's.
+// sqrt(x) as x y (1 + e/2 + 3 e^2/8) with the rounding of x y recovered:
+// within 0.51 ulp, eight FP64 slots (x times frsqrt: six, 1.32 ulps).  Zeros
+// and arguments outside the range go to CUDA's.
 static __device__ __noinline__ double sqrt_any(double x) { return sqrt(x); }
 
 __device__ __forceinline__ double fsqrt(double x)
 {
-    return static_cast<uint32_t>(__double2hiint(x)) - 0x39b00000u > 0x0c800000u ? sqrt_any(x) : x * frsqrt(x);
+    if (!root_in_range(x)) return sqrt_any(x);
+    double const y = rsqrt_seed(x);
+    double const e = fma(-x, y * y, 1.0);
+    double const s = x * y;
+    return s + fma(s * e, fma(e, 0.375, 0.5), fma(x, y, -s));
 }
 
 // sin and cos of the table angle 2 pi j/256 plus r, |r| <= pi/256: sin r and

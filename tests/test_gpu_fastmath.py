@@ -73,10 +73,10 @@ def test_roots(evaluate):
                         _neighbours(2.0 ** np.arange(-99, 100))])
     inv, _ = evaluate(0, x)
     ref = 1.0 / np.sqrt(L(x))
-    assert (np.abs(inv - ref) <= np.spacing(ref.astype(np.float64))).all()
+    assert (np.abs(inv - ref) <= 0.51 * np.spacing(ref.astype(np.float64))).all()
     root, _ = evaluate(1, x)
     ref = np.sqrt(L(x))
-    assert (np.abs(root - ref) <= 2.0 * np.spacing(ref.astype(np.float64))).all()
+    assert (np.abs(root - ref) <= 0.51 * np.spacing(ref.astype(np.float64))).all()
     y = np.concatenate([SPECIAL, _logspace(rng, -1022, -101, 1000), _logspace(rng, 101, 1023, 1000)])
     inv, cuda = evaluate(0, y)
     np.testing.assert_array_equal(inv, cuda)
