@@ -139,8 +139,10 @@ __device__ __forceinline__ double fsqrt(double x)
 }
 
 // sin and cos of the table angle 2 pi j/256 plus r, |r| <= pi/256: sin r and
-// cos r - 1 are r - r^3/6 + r^5/120 and -r^2/2 + r^4/24 - r^6/720, the terms
-// from r^4 on in FP32; within 2^-52 absolutely.
+// cos r - 1 are r - r^3/6 + r^5/120 and -r^2/2 + r^4/24 - r^6/720, the last
+// terms in FP32, and the table's value is added last: within 1.1 x 2^-53
+// absolutely (CUDA's 1.15; 2.0 with the r^4 term in FP32 and the table's value
+// added to each part).
 constexpr double kTurnStep = 2.45436926061702587187e-02;     // RN(2 pi / 256)
 constexpr double kTurnStepLo = 9.56755311833869693105e-19;   // RN(2 pi / 256 - kTurnStep)
 constexpr double kInvTurnStep = 4.07436654315252084757e+01;  // RN(256 / (2 pi))
@@ -149,13 +151,13 @@ __device__ __forceinline__ void sincos_step(const double* __restrict__ arena, in
     double2 const tab = __ldg(reinterpret_cast<const double2*>(arena + RREA_ARENA_TURN_TABLE) + (j & 255));
     double const r2 = r * r;
     float const q = narrow_f32(r2);
-    double const cm = r2 * (widen_f32(q * (1.0f / 24.0f - q * (1.0f / 720.0f))) - 0.5);
+    double const cm = r2 * fma(r2, 1.0 / 24.0 - widen_f32(q * (1.0f / 720.0f)), -0.5);
     double const sr = fma(r * r2, widen_f32(q * (1.0f / 120.0f)) - 1.0 / 6.0, r);
-    s = fma(tab.y, sr, fma(tab.x, cm, tab.x));
-    c = fma(-tab.x, sr, fma(tab.y, cm, tab.y));
+    s = tab.x + fma(tab.y, sr, tab.x * cm);
+    c = tab.y + fma(-tab.x, sr, tab.y * cm);
 }
 // sin and cos of 2 pi u for u in [0, 1): the nearest of 256 table angles and
-// the remainder (exact up to the product by 2 pi/256), 14 FP64 slots against
+// the remainder (exact up to the product by 2 pi/256), 17 FP64 slots against
 // 31 of a reduction of 2 pi u.  It takes the angle itself, where the
 // reference rounds 2 pi u (to 4e-16) first.
 __device__ __forceinline__ void sincos_turn(const double* __restrict__ arena, double u, double& s, double& c)

@@ -1,9 +1,10 @@
-"""The inverse root, root and quotient that the kernels use in place of CUDA's
-(device/rrea_fastmath.cuh, rrea_exact_quot.cuh), each against extended
-precision within the bound its comment states, over the range it covers and at both sides of every hand-over
-to CUDA's function; at zeros of both signs, subnormals, infinities and NaN the
-result is CUDA's (the sign of a zero quotient aside, which nothing reads).
-tests/cpp/fastmath.cu evaluates them."""
+"""The inverse root, root, sine, cosine and quotient that the kernels use in
+place of CUDA's (device/rrea_fastmath.cuh, rrea_exact_quot.cuh), each against
+extended precision within the bound its comment states, over the range it
+covers and at both sides of every hand-over to CUDA's function; at zeros of
+both signs, subnormals, infinities and NaN the result is CUDA's (the sign of a
+zero sine or quotient aside, which nothing reads).  tests/cpp/fastmath.cu
+evaluates them."""
 import ctypes
 import os
 import subprocess
@@ -86,6 +87,24 @@ def test_roots(evaluate):
     np.testing.assert_allclose(edge, np.sqrt(ROOT_EDGES), rtol=2.0 ** -51, atol=0)
     edge, _ = evaluate(0, ROOT_EDGES)
     np.testing.assert_allclose(edge, 1.0 / np.sqrt(ROOT_EDGES), rtol=2.0 ** -51, atol=0)
+
+
+def test_sine_and_cosine(evaluate):
+    rng = np.random.default_rng(2)
+    step = 2.0 * np.pi / TURNS
+    k = np.arange(-1024, 1025)
+    x = np.concatenate([rng.uniform(-np.pi, np.pi, 300_000), rng.uniform(-1024.0, 1024.0, 100_000),
+                        _neighbours(k * step), _neighbours((k + 0.5) * step), _logspace(rng, -1060, 0, 2000),
+                        -_logspace(rng, -1060, 0, 2000), [0.0, -0.0, np.nextafter(1024.0, 0.0)]])
+    s, c = evaluate(2, x)
+    assert np.abs(s - np.sin(L(x))).max() <= 1.1 * 2.0 ** -53
+    assert np.abs(c - np.cos(L(x))).max() <= 1.1 * 2.0 ** -53
+    far = np.concatenate([[1024.0, -1024.0, 1e6, 1e22, -1e300, INF, -INF, NAN, NEG_NAN], _logspace(rng, 10, 1023, 1000)])
+    np.testing.assert_array_equal(evaluate(2, far), evaluate(3, far))
+    u = np.concatenate([rng.uniform(0.0, 1.0, 200_000), np.clip(_neighbours(np.arange(512) / 512.0), 0.0, 1.0)])
+    s, c = evaluate(4, u)
+    assert np.abs(s - np.sin(2.0 * PI * L(u))).max() <= 1.1 * 2.0 ** -53
+    assert np.abs(c - np.cos(2.0 * PI * L(u))).max() <= 1.1 * 2.0 ** -53
 
 
 def test_quotient(evaluate):
