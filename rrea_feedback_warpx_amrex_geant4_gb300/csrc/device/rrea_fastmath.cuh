@@ -188,22 +188,27 @@ __device__ __forceinline__ void fsincos(const double* __restrict__ arena, double
     sincos_step(arena, __double2loint(t), fma(-k, kTurnStepLo, fma(-k, kTurnStep, a)), s, c);
 }
 
-// atan2(y, x): the FP32 angle names the nearest of 256 table angles a, the
-// point is turned by -a to (u, v) (v with the rounding of its second product
-// recovered, so that it keeps its relative accuracy), and with t = v/u,
-// |t| < tan(pi/250), the angle is a + t - t^3/3 + t^5/5 - t^7/7 + t^9/9 (the
-// last two terms in FP32; the next is below 2^-67): within two ulps, for 20
-// FP64 slots against 46.  Points nearer than 2^-100 to the axis or farther
-// than 2^100 go to CUDA's.
+// atan2(y, x): the FP32 angle names the nearest of 256 table angles a (0 up to
+// 0.02, where the first table angle's rounding would weigh more than the
+// result's), the point is turned by -a to (u, v) (v with the rounding of its
+// second product recovered, so that it keeps its relative accuracy), and with
+// t = v/u, |t| < 0.0201, the angle is a + t - t^3/3 + t^5/5 - t^7/7 + t^9/9
+// (the last two terms in FP32; the next is below 2^-59): within two ulps (1.5
+// measured, CUDA's 1.7), for 20 FP64 slots against 46.  Points nearer than
+// 2^-100 to the origin or farther than 2^100 go to CUDA's.
 static __device__ __noinline__ double atan2_any(double y, double x) { return atan2(y, x); }
 
 __device__ __forceinline__ double fatan2(const double* __restrict__ arena, double y, double x)
 {
-    int const j = __float2int_rn(atan2f(narrow_f32(y), narrow_f32(x)) * static_cast<float>(kInvTurnStep));
+    // the larger coordinate decides: past the FP32 range the seed would name
+    // any angle
+    uint32_t const hi = max(static_cast<uint32_t>(__double2hiint(x)) & 0x7fffffffu,
+                            static_cast<uint32_t>(__double2hiint(y)) & 0x7fffffffu);
+    if (hi - 0x39b00000u > 0x0c800000u) return atan2_any(y, x);
+    float const a32 = atan2f(narrow_f32(y), narrow_f32(x));
+    int const j = fabsf(a32) < 0.02f ? 0 : __float2int_rn(a32 * static_cast<float>(kInvTurnStep));
     double2 const tab = __ldg(reinterpret_cast<const double2*>(arena + RREA_ARENA_TURN_TABLE) + (j & 255));
     double const u = fma(x, tab.y, y * tab.x);
-    uint32_t const hi = static_cast<uint32_t>(__double2hiint(u));
-    if (hi - 0x39b00000u > 0x0c800000u) return atan2_any(y, x);
     double const p = x * tab.x;
     double const v = fma(y, tab.y, -p) - fma(x, tab.x, -p);
     // v / u: an FP32 reciprocal, one Newton step, the quotient's residual
@@ -216,8 +221,10 @@ __device__ __forceinline__ double fatan2(const double* __restrict__ arena, doubl
     double const t2 = t * t;
     float const q = narrow_f32(t2);
     double const s = fma(t2, 0.2 - widen_f32(q * (1.0f / 7.0f - q * (1.0f / 9.0f))), -1.0 / 3.0);
+    double const angle = fma(t * t2, s, t);
+    if (j == 0) return copysign(angle, y);   // (-0 keeps its sign)
     double const k = __longlong_as_double(0x4338000000000000LL + j) - 6755399441055744.0;   // j as a double
-    return fma(k, kTurnStep, fma(k, kTurnStepLo, fma(t * t2, s, t)));
+    return fma(k, kTurnStep, fma(k, kTurnStepLo, angle));
 }
 
 }  // namespace rrea_dev

@@ -74,8 +74,10 @@ RREA_HD uint32_t row_float_bits(float f)
 }
 
 // FP64 <-> FP32 on the integer pipe (a conversion instruction takes as long
-// as an FP64 multiply-add).  Narrowing truncates; both flush magnitudes below
-// 2^-126 to zero.  They are for the small terms of a sum.
+// as an FP64 multiply-add).  Narrowing truncates, and both flush magnitudes
+// below 2^-126 to zero (narrowing keeps the sign, which the quadrant of an
+// angle needs); magnitudes from 2^128 on are the caller's to keep out.  They
+// are for the small terms of a sum.
 RREA_HD float narrow_f32(double x)
 {
     long long const b = row_bits(x);
@@ -83,7 +85,7 @@ RREA_HD float narrow_f32(double x)
     uint32_t const lo = static_cast<uint32_t>(b);
     uint32_t const mag = hi & 0x7fffffffu;
     uint32_t const u = ((mag - 0x38000000u) << 3) | (lo >> 29);
-    return mag < 0x38100000u ? 0.0f : row_float(u | (hi & 0x80000000u));
+    return row_float((mag < 0x38100000u ? 0u : u) | (hi & 0x80000000u));
 }
 RREA_HD double widen_f32(float f)
 {

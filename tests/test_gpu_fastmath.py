@@ -1,10 +1,10 @@
-"""The inverse root, root, sine, cosine and quotient that the kernels use in
-place of CUDA's (device/rrea_fastmath.cuh, rrea_exact_quot.cuh), each against
-extended precision within the bound its comment states, over the range it
-covers and at both sides of every hand-over to CUDA's function; at zeros of
-both signs, subnormals, infinities and NaN the result is CUDA's (the sign of a
-zero sine or quotient aside, which nothing reads).  tests/cpp/fastmath.cu
-evaluates them."""
+"""The inverse root, root, sine, cosine, arc tangent and quotient that the
+kernels use in place of CUDA's (device/rrea_fastmath.cuh,
+rrea_exact_quot.cuh), each against extended precision within the bound its
+comment states, over the range it covers and at both sides of every hand-over
+to CUDA's function; at zeros of both signs, subnormals, infinities and NaN the
+result is CUDA's (the sign of a zero sine or quotient aside, which nothing
+reads).  tests/cpp/fastmath.cu evaluates them."""
 import ctypes
 import os
 import subprocess
@@ -105,6 +105,44 @@ def test_sine_and_cosine(evaluate):
     s, c = evaluate(4, u)
     assert np.abs(s - np.sin(2.0 * PI * L(u))).max() <= 1.1 * 2.0 ** -53
     assert np.abs(c - np.cos(2.0 * PI * L(u))).max() <= 1.1 * 2.0 ** -53
+
+
+def _check_angle(evaluate, x, y):
+    """CUDA's angle where the larger coordinate is outside [2^-100, 2^100], else
+    within two ulps of the exact one; the sign (of a zero too) always."""
+    a, cuda = evaluate(5, x, y)
+    m = np.maximum(np.abs(x), np.abs(y))   # NaN if either is
+    near = (m >= 2.0 ** -100) & (m <= 2.0 ** 100)
+    np.testing.assert_array_equal(a[~near], cuda[~near])
+    ref = np.arctan2(L(y[near]), L(x[near]))
+    ulp = np.spacing(np.maximum(np.abs(ref), 2.3e-308).astype(np.float64))
+    assert (np.abs(a[near] - ref) <= 2.0 * ulp).all()
+    number = ~np.isnan(cuda)
+    np.testing.assert_array_equal(np.signbit(a[number]), np.signbit(cuda[number]))
+
+
+def test_arc_tangent(evaluate):
+    rng = np.random.default_rng(3)
+    step = 2.0 * np.pi / TURNS
+    k = np.arange(-TURNS // 2, TURNS // 2 + 1)
+    th = np.concatenate([rng.uniform(-np.pi, np.pi, 200_000), rng.uniform(-0.05, 0.05, 100_000),
+                         _neighbours(k * step), _neighbours((k + 0.5) * step)])
+    r = _logspace(rng, -98, 98, th.size)
+    x, y = r * np.cos(th), r * np.sin(th)
+    # beside the axes, down to coordinates past the seed's range
+    big, small = _logspace(rng, -90, 99, 4000), _logspace(rng, -1000, -91, 4000)
+    sx, sy = rng.choice([-1.0, 1.0], (2, 4000))
+    x = np.concatenate([x, sx * big, sx * small, sx * big, sx * 0.0, sx * big])
+    y = np.concatenate([y, sy * small, sy * big, sy * 0.0, sy * big, sy * big])
+    _check_angle(evaluate, x, y)
+    v = np.concatenate([SPECIAL, -SPECIAL, [2.0 ** -101, 2.0 ** 101, 2.0 ** 127, 2.0 ** 128, 2.0 ** 130, 2.0 ** 200,
+                                            -2.0 ** 130]])
+    _check_angle(evaluate, *(g.ravel() for g in np.meshgrid(v, v)))
+    # one coordinate far beyond the other's, in and out of range
+    one = rng.choice([-1.0, 1.0], 2000) * rng.uniform(0.5, 2.0, 2000)
+    huge = rng.choice([-1.0, 1.0], 2000) * _logspace(rng, 101, 1023, 2000)
+    for x, y in ((huge, one), (one, huge), (huge, 2.0 ** 60 * one), (huge, huge[::-1].copy())):
+        _check_angle(evaluate, x, y)
 
 
 def test_quotient(evaluate):
