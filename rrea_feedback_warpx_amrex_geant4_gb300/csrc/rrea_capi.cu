@@ -209,7 +209,9 @@ struct rrea_gpu_ctx {
     uint64_t* d_diag_sub = nullptr;
     uint64_t* d_diag_ev = nullptr;
     int32_t* d_diag_disp = nullptr;
-    rrea_dev::ResumeRec* d_resume = nullptr;  // the common-history loop's records, one slot per tile slot
+    // the common-history loop's records, one slot per tile slot (null where it
+    // never runs: periodic z, a capacity below the switch, no memory left)
+    rrea_dev::ResumeRec* d_resume = nullptr;
     // a drop-in phase call uploads its host tile in chunks on side[0] while
     // the kernels of earlier chunks run on `stream` and side[1]
     cudaEvent_t chunk_up[kPhaseChunks] = {};
@@ -452,9 +454,14 @@ rrea_gpu_status rrea_gpu_create(const rrea_gpu_config* cfg, int64_t capacity, rr
         && dalloc(&ctx->d_alive, n) == cudaSuccess && dalloc(&ctx->d_child_lineage, nsec) == cudaSuccess
         && dalloc(&ctx->d_cost_scratch,
                   static_cast<size_t>(kPhaseChunks) * rrea_launch::cost_order_scratch_elems()) == cudaSuccess
-        && dalloc(&ctx->d_resume, n) == cudaSuccess
         && cudaEventCreate(&ctx->ev_start) == cudaSuccess && cudaEventCreate(&ctx->ev_stop) == cudaSuccess;
     if (!ok) return bail(RREA_GPU_ERR_CUDA);
+    // last, so that it takes memory from nothing the context cannot do without;
+    // without it every tile takes the full loop
+    if (cfg->periodic_z == 0 && capacity >= kLeanMinParticles && dalloc(&ctx->d_resume, n) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->d_resume = nullptr;
+    }
     if (cudaMemsetAsync(ctx->d_cells, 0, 5 * ncell * sizeof(double), ctx->stream) != cudaSuccess) {
         return bail(RREA_GPU_ERR_CUDA);
     }
@@ -968,7 +975,7 @@ rrea_gpu_status launch_phase(rrea_gpu_ctx* ctx, int species, int32_t step, doubl
         int const fit = warps_per_sm <= 8 ? 2 : warps_per_sm <= 16 ? 4 : warps_per_sm <= 32 ? 8 : 16;
         if (fit < min_blocks) min_blocks = fit;
     }
-    bool const lean = species != RREA_SPECIES_PHOTON && c.periodic_z == 0 && a.n >= kLeanMinParticles
+    bool const lean = ctx->d_resume && species != RREA_SPECIES_PHOTON && a.n >= kLeanMinParticles
         && (species == RREA_SPECIES_POSITRON || a.n_planes == 0);   // planes are the electrons'
     RREA_CUDA(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
     if (host && chunks == 1) {
