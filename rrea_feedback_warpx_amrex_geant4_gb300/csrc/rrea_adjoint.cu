@@ -48,6 +48,7 @@
 // 38.6 ms.
 #include "rrea_kernels.h"
 #include "device/rrea_device_path.cuh"
+#include "host/adjoint_tape.hpp"
 
 #include <cuda_runtime.h>
 
@@ -680,16 +681,24 @@ cudaError_t adjoint_stage(AdjointSetup const& in, const double* seeds6, const do
     alloc(&s->id, n);
     alloc(&s->ckpt, n_ckpt * 6 * n);
     alloc(&s->final_state, 6 * n);
-    // The forward pass leaves the tape of the last segments, as many as fit
-    // in kTapeBytes (at least one, which the reverse pass needs for any
+    alloc(&s->nodes, in.n_nodes);
+    alloc(&s->tape_state, 2);
+    alloc(&s->adj, 5 * n);
+    alloc(&s->loss, 1);
+    alloc(&s->partials, s->blocks);
+    alloc(&s->ends, n);
+    // The forward pass leaves the tape of the last segments, as many as
+    // kept_segments allows (at least one, which the reverse pass needs for any
     // other), so that those are not computed a second time: 1e5 electrons
     // over 96 steps in three segments, forward and reverse
     // 48.8 to 32.7 ms (an entry is written and read once, 4 GB in all, where
-    // computing it again took a third of the reverse pass).
+    // computing it again took a third of the reverse pass).  It comes last,
+    // and gives way to one segment where it does not fit.
     int64_t const entries = static_cast<int64_t>(in.ckpt_every) * in.substeps;
-    int64_t const entry_bytes = (6 + rrea_dev::adj::kAux) * static_cast<int64_t>(sizeof(double)) * (n > 0 ? n : 1);
-    int64_t const fit = kTapeBytes / entry_bytes / entries;
-    s->kept = static_cast<int>(fit < 1 ? 1 : fit < n_ckpt ? fit : n_ckpt);
+    int64_t const segment_bytes = (6 + rrea_dev::adj::kAux) * static_cast<int64_t>(sizeof(double)) * entries * n;
+    size_t free_bytes = 0, total_bytes = 0;
+    if (e == cudaSuccess) e = cudaMemGetInfo(&free_bytes, &total_bytes);
+    s->kept = rrea_host::kept_segments(n_ckpt, segment_bytes, kTapeBytes, static_cast<int64_t>(free_bytes));
     alloc(&s->tape, s->kept * entries * 6 * n);
     alloc(&s->aux, s->kept * entries * rrea_dev::adj::kAux * n);
     if (e == cudaErrorMemoryAllocation && s->kept > 1) {
@@ -701,12 +710,6 @@ cudaError_t adjoint_stage(AdjointSetup const& in, const double* seeds6, const do
         alloc(&s->tape, entries * 6 * n);
         alloc(&s->aux, entries * rrea_dev::adj::kAux * n);
     }
-    alloc(&s->nodes, in.n_nodes);
-    alloc(&s->tape_state, 2);
-    alloc(&s->adj, 5 * n);
-    alloc(&s->loss, 1);
-    alloc(&s->partials, s->blocks);
-    alloc(&s->ends, n);
     p.ends = s->ends;
     p.replay = 0;
     if (e == cudaSuccess && n > 0) {
