@@ -357,6 +357,8 @@ __device__ int advance_charged_newborn(StepConstants const& C, ElectronArgs cons
                     dy = now.dy;
                     dz = now.dz;
                     k = now.k;
+                    require_certified();
+                    if (err.code) break;
                     path = chord_path;
                     final_fraction = 1.0;
                     completed = sub + 1U;
