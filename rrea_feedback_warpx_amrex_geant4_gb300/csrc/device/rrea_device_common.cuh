@@ -301,20 +301,11 @@ __device__ __forceinline__ double semilogx(const double* __restrict__ x, const d
     return __ldg(y + lo) + t * (__ldg(y + hi) - __ldg(y + lo));
 }
 
-// S/RreaInteractionTables.cpp:110-119
-__device__ __forceinline__ double mfp_from_inverse(double inv, Err& err)
-{
-    if (!finite_bits(inv) || lt0(inv)) {
-        err.set(RREA_GPU_ERR_INVALID_STATE);
-        return 1.0e99;
-    }
-    return gt0(inv) ? 1.0 / inv : 1.0e99;
-}
-
-// The rate 1/MFP of an inverse-MFP table value as the reference forms it,
-// 1 / mfp_from_inverse(inv): 1e-99 for a zero value (the 1e99 m MFP), and
-// for a normal positive value 1 / (1 / inv), which is inv to within an ulp;
-// returning inv saves two FP64 division sequences per rate.
+// The rate 1/MFP of an inverse-MFP table value as the reference forms it
+// (S/RreaInteractionTables.cpp:110-119), 1 / (inv > 0 ? 1 / inv : 1e99 m):
+// 1e-99 for a zero value, and for a normal positive value 1 / (1 / inv), which
+// is inv to within an ulp; returning inv saves two FP64 division sequences per
+// rate.
 __device__ __forceinline__ double rate_from_inverse(double inv, Err& err)
 {
     if (!finite_bits(inv) || lt0(inv)) {
