@@ -912,8 +912,9 @@ rrea_gpu_status rrea_gpu_ensemble_population_thin_all(rrea_gpu_ctx* ctx, int32_t
  *          - plane_weight (sig((z_i(T) - z_plane) / z_width) - sig((z_i(0) - z_plane) / z_width)) ]
  * The forward pass checkpoints every `checkpoint_every` steps; the reverse
  * pass recomputes each segment from its checkpoint, unless the forward pass
- * left its steps' values (the last segments, up to 8 GiB) and the nodes are
- * the same, and runs the hand-written adjoint back through it.
+ * left its steps' values (the last segments, up to 8 GiB and half of the
+ * memory left) and the nodes are the same, and runs the hand-written adjoint
+ * back through it.
  *
  * stage: the seeds (host arrays: z, direction xyz (3n, normalised here),
  *   kinetic energy, weight, id); needs the tables loaded.

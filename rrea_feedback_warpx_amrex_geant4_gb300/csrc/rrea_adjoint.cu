@@ -44,8 +44,8 @@
 // and one each for gamma beta and 1/gamma), the stopping power and its
 // derivative come from interval polynomials (device/rrea_rate_rows.cuh), and
 // the rotation's sines from a table or a series.  Measured, 100,003
-// electrons, 96 steps of 4 substeps: forward 35.9 -> 12.0 ms, reverse 71.9 ->
-// 38.6 ms.
+// electrons, 96 steps of 4 substeps in three segments: forward 36.2 -> 17.9 ms
+// (16.8 without the tape it leaves), reverse 71.9 -> 15.4 ms.
 #include "rrea_kernels.h"
 #include "device/rrea_device_path.cuh"
 #include "host/adjoint_tape.hpp"
@@ -690,9 +690,9 @@ cudaError_t adjoint_stage(AdjointSetup const& in, const double* seeds6, const do
     // The forward pass leaves the tape of the last segments, as many as
     // kept_segments allows (at least one, which the reverse pass needs for any
     // other), so that those are not computed a second time: 1e5 electrons
-    // over 96 steps in three segments, forward and reverse
-    // 48.8 to 32.7 ms (an entry is written and read once, 4 GB in all, where
-    // computing it again took a third of the reverse pass).  It comes last,
+    // over 96 steps in three segments, forward 16.1 to 17.0 and reverse 32.4
+    // to 15.4 ms (an entry is written and read once, 4 GB in all, where
+    // computing it again took half of the reverse pass).  It comes last,
     // and gives way to one segment where it does not fit.
     int64_t const entries = static_cast<int64_t>(in.ckpt_every) * in.substeps;
     int64_t const segment_bytes = (6 + rrea_dev::adj::kAux) * static_cast<int64_t>(sizeof(double)) * entries * n;

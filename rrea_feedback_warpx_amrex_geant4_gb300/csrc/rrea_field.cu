@@ -124,7 +124,7 @@ dim3 grid_for(int nr, int nz, int rows)
     return dim3(static_cast<unsigned>(nr / 32 + 1), static_cast<unsigned>((nz + 1 + 8 * rows - 1) / (8 * rows)));
 }
 
-constexpr int kFieldThreads = 152 * 1024;
+constexpr int kFieldThreads = 152 * 1024;   // a GB300's SMs by half of an SM's threads
 
 }  // namespace
 }  // namespace rrea_dev

@@ -4,13 +4,16 @@
 // the Maxwell substeps of RreaAmrexAdvance::AdvanceOneStep
 // (S/RreaAmrexAdvance.cpp:593-838).
 //
-// Every kernel is a coalesced sweep over cells or faces (i fastest); the
-// whole state of a 512 x 4096 grid is ~0.5 GB, so each sweep is bound by HBM
-// bandwidth.  Reductions (maxima, minima, flags, sums) pre-reduce across the
+// Every kernel is a coalesced sweep over cells or faces (i fastest), bound by
+// the FP64 pipe (figures at the column launches below).  Reductions (maxima, minima, flags, sums) pre-reduce across the
 // warp and post one atomic per warp into a small word/sum block that the
 // host reads once per call (once per coupled step, plus the stiffness probe
-// that sizes the substeps).  This file is compiled without FMA contraction
-// so that every product and sum rounds as in the reference's host build.
+// that sizes the substeps).  This file is compiled without FMA contraction, so
+// the flux, limiter, update and charge arithmetic rounds as in the reference's
+// host build (quotients included, device/rrea_exact_quot.cuh).  What does not:
+// the closure's values between nodes (interval polynomials), |E| and the
+// tensor's eigenvalue (inverse roots), and the attachment decay below 1/16 (a
+// series), each within an ulp or two of the reference's.
 #include "rrea_kernels.h"
 #include "device/rrea_exact_quot.cuh"
 #include "device/rrea_fastmath.cuh"
